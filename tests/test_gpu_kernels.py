@@ -231,6 +231,20 @@ def test_gemv_gate_up(M, I, K, blk):
         close(got, ref, torch.bfloat16, "gemv gate/up with SiLU-mul", extra=2.0 ** -7 * ref.abs().max().item())
 
 
+@pytest.mark.parametrize("M,N,K,bias", [(1, 1, 4, False), (1, 4800, 68, True), (4, 33, 60, False), (5, 15, 64, True), (16, 4737, 132, False),
+                                        (17, 31, 2048, False), (32, 130, 196, True), (33, 1, 4, False), (33, 65, 20, True),
+                                        (64, 127, 2052, False), (65, 16384, 36, False), (200, 2048, 52, True), (333, 130, 16, False)])
+def test_gemm_simple_32bit_kernels_sum_in_one_order(M, N, K, bias):
+    """32-bit operands in 16-byte rows take kernels of their own (by rows of x, features and SMs); rows that start elsewhere take
+    the general one.  All sum an output's products one after the other: the results are equal, and right."""
+    x, w = torch.randn(M, K), torch.randn(N, K)
+    b = torch.randn(N).to(DEV) if bias else None
+    odd = lambda t: torch.cat([t, t[:, :1]], 1).to(DEV)[:, :K]             # rows of K + 1 floats: no 16-byte rows
+    got = k().gemm_simple(x.to(DEV), w.to(DEV), b, torch.float32)
+    assert torch.equal(got, k().gemm_simple(odd(x), odd(w), b, torch.float32))
+    close(got, plain_ops.linear(x, w, None if b is None else b.cpu(), torch.float64), torch.float32, "gemm_simple", scale=None)
+
+
 @pytest.mark.parametrize("ta,tw,tc", [(torch.bfloat16, torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32, torch.float32),
                                       (torch.bfloat16, torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16, torch.bfloat16)])
 def test_gemm_simple_mixed_types(ta, tw, tc):
