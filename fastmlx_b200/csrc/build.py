@@ -34,6 +34,8 @@ GROUPS = {
     "chan": "chan",
     # the matrix memory with exponential gates
     "mlstm": "mlstm",
+    # recurrences with a decay per head over portions, in runs of tokens as matrix products
+    "chunks": "chunks",
     # host code: the native step executor (no kernel of its own)
     "host": "host",
     # the tensor-core product built for one test: a wait limit of 100,000 clocks and a producer that

@@ -1,0 +1,483 @@
+// Linear recurrences with a matrix of 32-bit state per head, over portions, in runs of 32 tokens as matrix products.
+//
+//     S <- a_t S + k_t u_t^T;   o_t = S^T q_t;   u_t = v_t (weighed by a number per token), or the delta rule's
+//     u_t = beta_t (v_t - (a_t S)^T k_t)
+//
+// with one decay a_t per head.  Within a run that starts from S, with A_t = a_1 ... a_t,
+//
+//     o_t = A_t S^T q_t + sum_{s <= t} (q_t . k_s) (A_t / A_s) u_s
+//     u   = T diag(beta) (v - A (k S)),   T = (1 + strictly lower part of beta_t (k_t . k_s) (A_t / A_s))^-1
+//     S  <- A_32 S + sum_s (A_32 / A_s) k_s u_s^T
+//
+// Ratios A_t / A_s are running products of decays (at most one, no logarithm, no division).  Every product that meets the
+// state runs on the tensor cores with three bfloat16 terms an operand (split_mma.cuh), so that it is as exact as the walk
+// token by token in 32-bit multiply-adds (the kernels of delta_rule.cu and ssm.cu; 2,048 tokens against 64-bit, decays near one:
+// 1.8e-7 of the result's norm here, 2.4e-7 there; decays of 0.8: 1.2e-7 and 1.1e-7).  That walk is one chain of dependent
+// steps of some 250 ns a token; a run of 32 tokens here takes 1.4 us at 64 rows of state, 3.3 us at 128.  One request of 2,048
+// tokens, 32 heads on 8 key heads, both kernels: delta rule 64 x 64 521 -> 115 us, 128 x 128 (two requests) 1,010 -> 234 us;
+// plain write 346 -> 98 and 660 -> 198 us; 1,777 tokens of five requests, 64 heads of 64 values over 128 rows 561 -> 188 us.
+//
+//   chunk_prepare  per (run, key group): k and q as three terms; k . k^T and q . k^T in 32-bit, and per head of the group
+//                  the decayed q . k^T and T, as three terms.  All runs at once.
+//   chunk_scan     per (request, head, 16 or 32 columns of S): the runs in order.
+//
+// A token that holds an infinity or a NaN makes the outputs of its own request's run of 32 tokens NaN, also those in front of it
+// in the run; other requests are not touched.
+#include <math.h>
+#include "split_mma.cuh"
+
+namespace {
+constexpr int RUN = 32;                         // tokens of a run
+// Rows of the workspaces are as far apart as chunk_scan wants them in shared memory (eight 16-byte pieces of eight rows meet no
+// bank twice), so that a run's operands are two runs of bytes to copy: k and q of a group, and P, T and numbers of a head.
+constexpr int PT_LD = RUN + 8;
+constexpr int GRAM_LD = RUN + 4;
+template <int D> constexpr int QK_LD = D + 8;
+template <int D> constexpr int QK_SIZE = 2 * 3 * RUN * QK_LD<D>;              // bf16 of q and k of a run and group
+constexpr int PLANE = 3 * RUN * PT_LD;                                        // bf16 of one 32 x 32 matrix in three terms
+template <bool DELTA> constexpr int PT_SIZE = (DELTA ? 2 : 1) * PLANE + 4 * RUN;   // P, T and, as floats, A_t and E_s
+
+// The place of a row's first run in the workspaces: rows do not overlap, whatever their lengths.
+__device__ __forceinline__ int first_run(int row_start, int r) { return row_start / RUN + r; }
+
+// x [T, C]: q of group g at qoff + g D, k at koff + g D.  decay, weight: per token and head, rows of gstride.
+// qk [run][G][q, k][3][32][D], pt [run][H][P, T (delta rule)][3][32][32] and floats [A_t: 32, E_s: 32].
+template <int D, bool DELTA>
+__global__ void __launch_bounds__(128)
+chunk_prepare_kernel(const float* x, long long C, int qoff, int koff, const float* decay, const float* weight, int gstride,
+                     const int* row_start, int min_tokens, int H, int G, bf16* qk, bf16* pt) {
+  constexpr int LD = D + 4;
+  extern __shared__ __align__(16) float psm[];
+  float* qs = psm;                              // [32][LD]
+  float* ks = qs + RUN * LD;
+  float* qkm = ks + RUN * LD;                   // q . k^T, [32][GRAM_LD]
+  float* kkm = qkm + RUN * GRAM_LD;             // k . k^T
+  const int c = blockIdx.x, g = blockIdx.y, r = blockIdx.z;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  float* mine = kkm + RUN * GRAM_LD + warp * RUN * GRAM_LD;      // a warp's matrix
+  pdl_wait();      // no early trigger: blocks of chunk_scan would sit on the shared memory that this kernel's blocks want
+  const int first = row_start[r], n = row_start[r + 1] - first;
+  if (c * RUN >= n || n < min_tokens) return;
+  const int t0 = first + c * RUN, cnt = min(RUN, n - c * RUN);
+  const long long run = first_run(first, r) + c;
+  bf16* planes = qk + (run * G + g) * QK_SIZE<D>;
+  for (int e = tid; e < 2 * RUN * (D / 4); e += 128) {
+    const int which = e / (RUN * (D / 4)), row = e / (D / 4) % RUN, d = e % (D / 4) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row < cnt) v = load4(x + (long long)(t0 + row) * C + (which ? koff : qoff) + g * D + d);
+    store4((which ? ks : qs) + row * LD + d, v);
+    unsigned a[3], b[3];
+    three_terms(v.x, v.y, a[0], a[1], a[2]);
+    three_terms(v.z, v.w, b[0], b[1], b[2]);
+#pragma unroll
+    for (int term = 0; term < 3; ++term)
+      *reinterpret_cast<uint2*>(planes + ((which * 3 + term) * RUN + row) * QK_LD<D> + d) = make_uint2(a[term], b[term]);
+  }
+  __syncthreads();
+  {
+    const int t = tid >> 2, s0 = tid & 3;       // a thread's eight columns s0, s0 + 4, ...: neighbours read neighbouring rows
+    float tq[RUN / 4], tk[RUN / 4];
+#pragma unroll
+    for (int j = 0; j < RUN / 4; ++j) tq[j] = tk[j] = 0.f;
+    auto fma4 = [](float4& c, float4 u, float4 v) {
+      c.x = fmaf(u.x, v.x, c.x); c.y = fmaf(u.y, v.y, c.y); c.z = fmaf(u.z, v.z, c.z); c.w = fmaf(u.w, v.w, c.w);
+    };
+#pragma unroll 1
+    for (int d0 = 0; d0 < D; d0 += 16) {        // sums of 16 products in four chains, then of those: as short chains as the walk's
+      float4 aq[RUN / 4], ak[RUN / 4];
+#pragma unroll
+      for (int j = 0; j < RUN / 4; ++j) aq[j] = ak[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int d = d0; d < d0 + 16; d += 4) {
+        const float4 q4 = load4(qs + t * LD + d), k4 = load4(ks + t * LD + d);
+#pragma unroll
+        for (int j = 0; j < RUN / 4; ++j) {
+          const float4 s4 = load4(ks + (s0 + 4 * j) * LD + d);
+          fma4(aq[j], q4, s4);
+          if (DELTA) fma4(ak[j], k4, s4);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < RUN / 4; ++j) {
+        tq[j] += (aq[j].x + aq[j].y) + (aq[j].z + aq[j].w);
+        if (DELTA) tk[j] += (ak[j].x + ak[j].y) + (ak[j].z + ak[j].w);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < RUN / 4; ++j) {
+      qkm[t * GRAM_LD + s0 + 4 * j] = tq[j];
+      if (DELTA) kkm[t * GRAM_LD + s0 + 4 * j] = tk[j];
+    }
+  }
+  __syncthreads();
+  auto emit = [&](bf16* dst) {                  // a warp's 32 x 32 matrix as three terms
+#pragma unroll 2
+    for (int row = lane >> 3; row < RUN; row += 4) {
+      const int s = (lane & 7) * 4;
+      const float4 v = load4(mine + row * GRAM_LD + s);
+      unsigned a[3], b[3];
+      three_terms(v.x, v.y, a[0], a[1], a[2]);
+      three_terms(v.z, v.w, b[0], b[1], b[2]);
+#pragma unroll
+      for (int term = 0; term < 3; ++term)
+        *reinterpret_cast<uint2*>(dst + (term * RUN + row) * PT_LD + s) = make_uint2(a[term], b[term]);
+    }
+  };
+  const int per = H / G;
+  for (int hh = warp; hh < per; hh += 4) {
+    const int h = g * per + hh;
+    const bool live = lane < cnt;
+    const float a = live ? decay[(long long)(t0 + lane) * gstride + h] : 1.f;
+    const float w = live ? weight[(long long)(t0 + lane) * gstride + h] : 0.f;
+    bf16* out = pt + (run * H + h) * PT_SIZE<DELTA>;
+    float* sc = reinterpret_cast<float*>(out + (DELTA ? 2 : 1) * PLANE);
+    float ratio = 0.f, cum = 1.f, own = 1.f;    // lane s: A_t / A_s as t goes on; A_t; A_lane
+    float rows[RUN];
+#pragma unroll
+    for (int t = 0; t < RUN; ++t) {
+      const float at = __shfl_sync(0xffffffffu, a, t), wt = __shfl_sync(0xffffffffu, w, t);
+      cum *= at;
+      if (lane == t) own = cum;
+      ratio = lane < t ? ratio * at : lane == t ? 1.f : 0.f;
+      // the decayed q . k^T, the weights of a plain write folded in
+      mine[t * GRAM_LD + lane] = lane <= t ? qkm[t * GRAM_LD + lane] * ratio * (DELTA ? 1.f : w) : 0.f;
+      if (DELTA) rows[t] = lane < t ? wt * kkm[t * GRAM_LD + lane] * ratio : 0.f;
+    }
+    sc[lane] = own;
+    sc[RUN + lane] = DELTA ? ratio : ratio * w;
+    __syncwarp();
+    emit(out);
+    __syncwarp();
+    if (DELTA) {
+#pragma unroll
+      for (int t = 0; t < RUN; ++t) mine[t * GRAM_LD + lane] = rows[t];
+      __syncwarp();
+      // lane j solves for column j of T from the top down: T_ij = [i = j] - sum_{l < i} M_il T_lj
+      float T[RUN];
+#pragma unroll
+      for (int i = 0; i < RUN; ++i) {
+        float p[4] = {lane == i ? 1.f : 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int l = 0; l < i; l += 4) {
+          const float4 m = load4(mine + i * GRAM_LD + l);
+          p[0] = fmaf(-m.x, T[l], p[0]);
+          if (l + 1 < i) p[1] = fmaf(-m.y, T[l + 1], p[1]);
+          if (l + 2 < i) p[2] = fmaf(-m.z, T[l + 2], p[2]);
+          if (l + 3 < i) p[3] = fmaf(-m.w, T[l + 3], p[3]);
+        }
+        T[i] = (p[0] + p[1]) + (p[2] + p[3]);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < RUN; ++i) mine[i * GRAM_LD + lane] = T[i] * w;      // its columns take beta
+      __syncwarp();
+      emit(out + PLANE);
+      __syncwarp();
+    }
+  }
+}
+
+// Shared memory of chunk_scan: two stages of a run's operands, and what the four warps of 16 columns hand one another.
+template <int D, int MT, bool DELTA> struct ScanSmem {
+  static constexpr int V_LD = 16 * MT + 4;                                // floats
+  static constexpr size_t STAGE = (size_t)(QK_SIZE<D> + PT_SIZE<DELTA>) * 2 + (size_t)RUN * V_LD * 4;
+  static constexpr int S_WORDS = 3 * (D / 16) * 32 * 4;                   // 32-bit words of S^T's fragments, per 16 columns
+  static constexpr int U_WORDS = 3 * (RUN / 16) * 32 * 4;                 // of R's, U's and E's
+  static constexpr size_t BYTES = 2 * STAGE + (size_t)MT * (S_WORDS + (DELTA ? 3 : 2) * U_WORDS) * 4;
+};
+
+// grid (columns / (16 MT), H, R), 128 MT + 32 threads: four warps per 16 columns, and one that copies.  S^T is kept as
+// accumulator tiles of 16 columns by 8 rows of state, a quarter of the rows in each warp; a warp works out the run's
+// read-outs for 8 of its 32 tokens.  A product's left operand is always S^T or a 16 x 32 matrix of the columns' values:
+// accumulators turn into the next product's left operand where they lie, and cross to the other warps through shared
+// memory as finished fragments.  Bound by the latency of that chain (four exchanges a run), not by a unit: hence 32 tokens
+// a run (64 take 1.2 times the products and 1.3 times the operands' bytes per token), four warps to share a link's
+// products, and copies that no link waits for.
+template <int D, int MT, bool DELTA>
+__global__ void __launch_bounds__(128 * MT + 32)
+chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, int voff, const float* skip, const int* row_start,
+                  const int* row_slot, float* state, long long slot_stride, float* out, int min_tokens, int H, int G, int P, int max_slots) {
+  using Z = ScanSmem<D, MT, DELTA>;
+  constexpr int KT = D / 16, NS = D / 32;        // k-tiles of S; 8-row tiles of S^T per warp
+  extern __shared__ __align__(16) unsigned char csm[];
+  const int r = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * 16 * MT;
+  const int tid = threadIdx.x, lane = tid & 31, mt = tid >> 7, w = tid >> 5 & 3;
+  pdl_wait();
+  pdl_trigger();
+  const int slot = row_slot[r];
+  if (slot < 0 || slot >= max_slots) return;
+  const int first = row_start[r], n = row_start[r + 1] - first;
+  if (n < min_tokens) return;                    // walked token by token in a launch of its own
+  const int runs = (n + RUN - 1) / RUN, g = h / (H / G);
+  const long long run0 = first_run(first, r);
+  if (tid >= 128 * MT) {                         // the copying warp: a run's operands land while the run before it is walked
+    auto cp16 = [](void* dst, const void* src, bool there) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0));
+    };
+    for (int c = 0; c < runs; ++c) {
+      unsigned char* dst = csm + (c & 1) * Z::STAGE;
+      const unsigned char* src = reinterpret_cast<const unsigned char*>(qk + ((run0 + c) * G + g) * QK_SIZE<D>);
+#pragma unroll 8
+      for (int e = lane * 16; e < QK_SIZE<D> * 2; e += 512) cp16(dst + e, src + e, true);
+      dst += QK_SIZE<D> * 2;
+      src = reinterpret_cast<const unsigned char*>(pt + ((run0 + c) * H + h) * PT_SIZE<DELTA>);
+#pragma unroll 8
+      for (int e = lane * 16; e < PT_SIZE<DELTA> * 2; e += 512) cp16(dst + e, src + e, true);
+      float* dv = reinterpret_cast<float*>(dst + PT_SIZE<DELTA> * 2);
+#pragma unroll
+      for (int e = lane; e < RUN * 4 * MT; e += 32) {
+        const int t = e / (4 * MT), q = e % (4 * MT) * 4;
+        const bool there = c * RUN + t < n;
+        cp16(dv + t * Z::V_LD + q, x + (long long)(first + (there ? c * RUN + t : 0)) * C + voff + (long long)h * P + c0 + q, there);
+      }
+      asm volatile("cp.async.commit_group;\n" ::);
+      asm volatile("cp.async.wait_group 0;\n" ::);
+      __syncthreads();                           // run c is there; run c - 1 has been walked, and its stage is free
+    }
+    return;
+  }
+  unsigned* sfr = reinterpret_cast<unsigned*>(csm + 2 * Z::STAGE) + mt * Z::S_WORDS;
+  unsigned* ufr = reinterpret_cast<unsigned*>(csm + 2 * Z::STAGE) + MT * Z::S_WORDS + mt * (DELTA ? 3 : 2) * Z::U_WORDS;
+  unsigned* efr = ufr + Z::U_WORDS;
+  unsigned* rfr = efr + Z::U_WORDS;
+  const float sk = DELTA ? 0.f : skip[h];
+  auto meet = [&]() {                            // the four warps of these 16 columns
+    asm volatile("bar.sync %0, 128;\n" ::"r"(1 + mt) : "memory");
+  };
+  const int row = lane >> 2, two = (lane & 3) * 2;            // a thread's columns of S: row, row + 8; within a tile of 8: two, two + 1
+  float* sp = state + (long long)slot * slot_stride + ((long long)h * P + c0 + mt * 16) * D + w * (D / 4);
+  float S[NS][4];
+#pragma unroll
+  for (int j = 0; j < NS; ++j) {
+    const float2 a = *reinterpret_cast<const float2*>(sp + (long long)row * D + j * 8 + two);
+    const float2 b = *reinterpret_cast<const float2*>(sp + (long long)(row + 8) * D + j * 8 + two);
+    S[j][0] = a.x; S[j][1] = a.y; S[j][2] = b.x; S[j][3] = b.y;
+  }
+  auto share_state = [&]() {                     // this warp's rows of state as left fragments, three terms
+#pragma unroll
+    for (int j = 0; j < NS; j += 2) {
+      unsigned f[3][4];
+      three_terms(S[j][0], S[j][1], f[0][0], f[1][0], f[2][0]);
+      three_terms(S[j][2], S[j][3], f[0][1], f[1][1], f[2][1]);
+      three_terms(S[j + 1][0], S[j + 1][1], f[0][2], f[1][2], f[2][2]);
+      three_terms(S[j + 1][2], S[j + 1][3], f[0][3], f[1][3], f[2][3]);
+#pragma unroll
+      for (int t = 0; t < 3; ++t)
+        *reinterpret_cast<uint4*>(sfr + ((t * KT + w * (NS / 2) + j / 2) * 32 + lane) * 4) = make_uint4(f[t][0], f[t][1], f[t][2], f[t][3]);
+    }
+  };
+  auto share_tile = [&](unsigned* dst, const float (&v)[4]) {  // this warp's 8 tokens of a 16 x 32 matrix, likewise
+    unsigned f[3][2];
+    three_terms(v[0], v[1], f[0][0], f[1][0], f[2][0]);
+    three_terms(v[2], v[3], f[0][1], f[1][1], f[2][1]);
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+      *reinterpret_cast<uint2*>(dst + ((t * 2 + (w >> 1)) * 32 + lane) * 4 + (w & 1) * 2) = make_uint2(f[t][0], f[t][1]);
+  };
+  auto fragment = [&](unsigned (&f)[3][4], const unsigned* src, int tiles, int k) {
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      const uint4 u = *reinterpret_cast<const uint4*>(src + ((t * tiles + k) * 32 + lane) * 4);
+      f[t][0] = u.x; f[t][1] = u.y; f[t][2] = u.z; f[t][3] = u.w;
+    }
+  };
+  share_state();
+  const long long ostride = (long long)H * P;
+  float* op = out + (long long)first * ostride + (long long)h * P + c0 + mt * 16;
+  const int t0 = w * 8 + two;                    // this thread's tokens of a run: t0, t0 + 1
+  const int rows8 = w * 8 + (lane & 7), quarter = (lane >> 3) * 8;
+  for (int c = 0; c < runs; ++c) {
+    __syncthreads();                             // the run's operands and S's fragments are there
+    const bf16* dq = reinterpret_cast<const bf16*>(csm + (c & 1) * Z::STAGE);
+    const bf16* dk = dq + 3 * RUN * QK_LD<D>;
+    const bf16* dp = dq + QK_SIZE<D>;
+    const float* ds = reinterpret_cast<const float*>(dp + (DELTA ? 2 : 1) * PLANE);
+    const float* dv = ds + 2 * RUN + mt * 16;
+    const float A0 = ds[t0], A1 = ds[t0 + 1], E0 = ds[RUN + t0], E1 = ds[RUN + t0 + 1], last = ds[RUN - 1];
+    float v[4] = {dv[t0 * Z::V_LD + row], dv[(t0 + 1) * Z::V_LD + row], dv[t0 * Z::V_LD + row + 8], dv[(t0 + 1) * Z::V_LD + row + 8]};
+    const float x0 = v[0], x1 = v[1], x2 = v[2], x3 = v[3];
+    // what the state in front of the run gives these 8 tokens: S^T q, and S^T k for the delta rule; side by side, so that one's
+    // chains of products fill the other's waits
+    Sums o, kS;
+    o.zero();
+    kS.zero();
+    auto read_out = [&]() {
+#pragma unroll
+      for (int k2 = 0; k2 < KT / 2; ++k2) {
+        unsigned bq[3][4], bk[3][4];
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+          if (DELTA) ldmatrix4(bk[t], dk + (t * RUN + rows8) * QK_LD<D> + k2 * 32 + quarter);
+          ldmatrix4(bq[t], dq + (t * RUN + rows8) * QK_LD<D> + k2 * 32 + quarter);
+        }
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          unsigned a[3][4];
+          fragment(a, sfr, KT, k2 * 2 + kk);
+          if (DELTA) kS.add(a, bk, kk * 2);
+          o.add(a, bq, kk * 2);
+        }
+      }
+    };
+    if (DELTA) read_out();
+    if (DELTA) {                                  // u = T diag(beta) (v - A (S^T k))
+      unsigned bt[3][4];
+#pragma unroll
+      for (int t = 0; t < 3; ++t) ldmatrix4(bt[t], dp + PLANE + (t * RUN + rows8) * PT_LD + quarter);
+      v[0] = fmaf(-A0, kS.at(0), v[0]); v[1] = fmaf(-A1, kS.at(1), v[1]);
+      v[2] = fmaf(-A0, kS.at(2), v[2]); v[3] = fmaf(-A1, kS.at(3), v[3]);
+      share_tile(rfr, v);
+      meet();
+      Sums u;
+      u.zero();
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        if (k <= (w >> 1)) {                      // T is lower triangular
+          unsigned a[3][4];
+          fragment(a, rfr, 2, k);
+          u.add(a, bt, k * 2);
+        }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = u.at(i);
+    }
+    share_tile(ufr, v);
+    v[0] *= E0; v[1] *= E1; v[2] *= E0; v[3] *= E1;
+    share_tile(efr, v);
+    if (!DELTA) read_out();                       // behind the tiles that the others wait for
+    meet();
+    // S <- A_32 S + sum_s (E_s u_s) k_s^T for this warp's rows of state, and what the run's own tokens give: the decayed
+    // q . k^T times u
+    Sums y, d[NS];
+    y.zero();
+    {
+      unsigned bp[3][4];
+#pragma unroll
+      for (int t = 0; t < 3; ++t) ldmatrix4(bp[t], dp + (t * RUN + rows8) * PT_LD + quarter);
+#pragma unroll
+      for (int j = 0; j < NS; ++j) d[j].zero();
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        unsigned e[3][4], a[3][4];
+        fragment(e, efr, 2, k);
+        fragment(a, ufr, 2, k);
+#pragma unroll
+        for (int j = 0; j < NS; ++j) {
+          unsigned b[3][2];
+#pragma unroll
+          for (int t = 0; t < 3; ++t)
+            ldmatrix2_trans(b[t], dk + (t * RUN + k * 16 + (lane & 15)) * QK_LD<D> + w * (D / 4) + j * 8);
+          d[j].add(e, b, 0);
+        }
+        if (k <= (w >> 1)) y.add(a, bp, k * 2);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NS; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) S[j][i] = fmaf(S[j][i], last, d[j].at(i));
+    share_state();                                // the others' reads of these fragments lie in front of the last meeting
+    const int t = c * RUN + t0;
+    float res[4] = {fmaf(A0, o.at(0), y.at(0)), fmaf(A1, o.at(1), y.at(1)), fmaf(A0, o.at(2), y.at(2)), fmaf(A1, o.at(3), y.at(3))};
+    if (!DELTA) {
+      res[0] = fmaf(sk, x0, res[0]); res[1] = fmaf(sk, x1, res[1]);
+      res[2] = fmaf(sk, x2, res[2]); res[3] = fmaf(sk, x3, res[3]);
+    }
+    if (t < n) {
+      op[(long long)t * ostride + row] = res[0];
+      op[(long long)t * ostride + row + 8] = res[2];
+    }
+    if (t + 1 < n) {
+      op[(long long)(t + 1) * ostride + row] = res[1];
+      op[(long long)(t + 1) * ostride + row + 8] = res[3];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NS; ++j) {
+    *reinterpret_cast<float2*>(sp + (long long)row * D + j * 8 + two) = make_float2(S[j][0], S[j][1]);
+    *reinterpret_cast<float2*>(sp + (long long)(row + 8) * D + j * 8 + two) = make_float2(S[j][2], S[j][3]);
+  }
+}
+
+struct Args {
+  const float *x, *decay, *weight, *skip;
+  long long C;
+  int qoff, koff, voff;
+  const int *row_start, *row_slot;
+  float* state;
+  long long slot_stride;
+  float* out;
+  void* ws;
+  int T, R, H, G, P, max_slots, max_q, min_tokens;
+};
+
+long long runs_of(int T, int R) { return (long long)T / RUN + R; }       // places for runs: see first_run
+
+template <int D, bool DELTA> long long bytes_of(int T, int R, int H, int G) {
+  return runs_of(T, R) * 2 * ((long long)G * QK_SIZE<D> + (long long)H * PT_SIZE<DELTA>);
+}
+long long ws_bytes(int T, int R, int H, int G, int D, bool delta) {
+  return D == 64 ? (delta ? bytes_of<64, true>(T, R, H, G) : bytes_of<64, false>(T, R, H, G))
+                 : (delta ? bytes_of<128, true>(T, R, H, G) : bytes_of<128, false>(T, R, H, G));
+}
+
+template <int D, bool DELTA> int launch(const Args& a, cudaStream_t stream) {
+  bf16* qk = reinterpret_cast<bf16*>(a.ws);
+  bf16* pt = qk + runs_of(a.T, a.R) * a.G * QK_SIZE<D>;
+  constexpr int prep = (2 * RUN * (D + 4) + 6 * RUN * GRAM_LD) * 4;
+  if (prep > 48 * 1024)
+    cudaFuncSetAttribute(chunk_prepare_kernel<D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep);
+  fmx_launch(chunk_prepare_kernel<D, DELTA>, dim3((a.max_q + RUN - 1) / RUN, a.G, a.R), dim3(128), prep, stream, a.x, a.C, a.qoff, a.koff,
+             a.decay, a.weight, 2 * a.H, a.row_start, a.min_tokens, a.H, a.G, qk, pt);
+  // 32 columns a block where blocks of 16 would be more than two for each SM: half the operands' traffic
+  const bool pair = a.P % 32 == 0 && (long long)a.R * a.H * (a.P / 16) > (long long)(D > 64 ? 1 : 2) * fmx_num_sms();
+#define FMX_SCAN(MT)                                                                                                         \
+  do {                                                                                                                       \
+    constexpr size_t smem = ScanSmem<D, MT, DELTA>::BYTES;                                                                   \
+    cudaFuncSetAttribute(chunk_scan_kernel<D, MT, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
+    fmx_launch(chunk_scan_kernel<D, MT, DELTA>, dim3(a.P / (16 * MT), a.H, a.R), dim3(128 * MT + 32), smem, stream, (const bf16*)qk, \
+               (const bf16*)pt, a.x, a.C, a.voff, a.skip, a.row_start, a.row_slot, a.state, a.slot_stride, a.out, \
+               a.min_tokens, a.H, a.G, a.P, a.max_slots);                                                                                  \
+  } while (0)
+  if (pair) FMX_SCAN(2);
+  else FMX_SCAN(1);
+#undef FMX_SCAN
+  FMX_LAUNCH_CHECK();
+  return 0;
+}
+
+int check(const char* who, const Args& a, int D, bool delta, long long ws_size) {
+  if (a.T <= 0 || a.R <= 0 || a.H <= 0 || a.G <= 0 || a.H % a.G || a.P <= 0 || a.P % 16 || (D != 64 && D != 128) || a.max_q <= 0)
+    return fmx_fail("%s: bad sizes T=%d R=%d H=%d G=%d D=%d P=%d max_q=%d", who, a.T, a.R, a.H, a.G, D, a.P, a.max_q);
+  if (a.H > 65535 || a.R > 65535) return fmx_fail("%s: batch too large", who);
+  if (a.C % 4 || a.slot_stride % 4 || (uintptr_t)a.x % 16 || (uintptr_t)a.state % 16 || (uintptr_t)a.ws % 16)
+    return fmx_fail("%s: rows that do not start on 16 bytes", who);
+  if (ws_size < ws_bytes(a.T, a.R, a.H, a.G, D, delta)) return fmx_fail("%s: the workspace is too small", who);
+  return 0;
+}
+}  // namespace
+
+// Bytes of workspace that T tokens of R rows take.
+FMX_EXPORT long long fmx_chunk_scan_bytes(int T, int R, int H, int G, int D, int delta) { return ws_bytes(T, R, H, G, D, delta != 0); }
+
+// The gated delta rule (see fmx_delta_rule) over the rows of at least min_tokens tokens; max_q: the longest one.
+FMX_EXPORT int fmx_chunk_delta_rule(const float* qkv, const float* gb, const int* row_start, const int* row_slot, float* state,
+                                    long long slot_stride, float* out, void* ws, long long ws_size, int T, int R, int H, int G,
+                                    int D, int Dv, int max_slots, int max_q,
+                                    int min_tokens, cudaStream_t stream) {
+  const Args a = {qkv, gb, gb + H, nullptr, 2LL * G * D + (long long)H * Dv, 0, G * D, 2 * G * D, row_start, row_slot, state, slot_stride,
+                  out, ws, T, R, H, G, Dv, max_slots, max_q, min_tokens};
+  if (int bad = check("fmx_chunk_delta_rule", a, D, true, ws_size)) return bad;
+  return D == 64 ? launch<64, true>(a, stream) : launch<128, true>(a, stream);
+}
+
+// The state-space recurrence (see fmx_ssm_scan) over them.
+FMX_EXPORT int fmx_chunk_ssm_scan(const float* xbc, const float* dd, const float* d_skip, const int* row_start, const int* row_slot,
+                                  float* state, long long slot_stride, float* out, void* ws, long long ws_size, int T, int R, int H,
+                                  int G, int N, int P, int max_slots, int max_q,
+                                    int min_tokens, cudaStream_t stream) {
+  const int inner = H * P;
+  const Args a = {xbc, dd + H, dd, d_skip, (long long)inner + 2LL * G * N, inner + G * N, inner, 0, row_start, row_slot, state, slot_stride,
+                  out, ws, T, R, H, G, P, max_slots, max_q, min_tokens};
+  if (int bad = check("fmx_chunk_ssm_scan", a, N, false, ws_size)) return bad;
+  return N == 64 ? launch<64, false>(a, stream) : launch<128, false>(a, stream);
+}

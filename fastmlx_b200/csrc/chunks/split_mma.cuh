@@ -1,0 +1,58 @@
+// Products of 32-bit matrices on the tensor cores: every operand as three bfloat16 terms (8 + 8 + 8 bits of its 24),
+// six of the nine products of terms, summed in 32-bit.  What is left out lies 2^-24 below a product.
+#pragma once
+#include "packed.cuh"
+
+namespace {
+// (x, y) -> three pairs of bfloat16 whose sums are x and y (to 2^-27 of them)
+__device__ __forceinline__ void three_terms(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  const float2 hf = __bfloat1622float2(h);
+  const float rx = x - hf.x, ry = y - hf.y;
+  const __nv_bfloat162 m = __floats2bfloat162_rn(rx, ry);
+  const float2 mf = __bfloat1622float2(m);
+  const __nv_bfloat162 l = __floats2bfloat162_rn(rx - mf.x, ry - mf.y);
+  hi = *reinterpret_cast<const unsigned*>(&h);
+  mid = *reinterpret_cast<const unsigned*>(&m);
+  lo = *reinterpret_cast<const unsigned*>(&l);
+}
+
+__device__ __forceinline__ void mma16816(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ void ldmatrix4(unsigned (&r)[4], const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void ldmatrix2_trans(unsigned (&r)[2], const bf16* p) {        // lanes 0 to 15 name the rows
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+               : "=r"(r[0]), "=r"(r[1]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+}
+
+// A 16 x 8 tile of sums, kept apart by size of the terms: chains of dependent products that do not wait for one another.
+// Products of the leading terms are added up in rounded 32-bit sums: the tensor cores' own sums cut off, and of
+// these products that would be seen.
+struct Sums {
+  float big[4], middle[4], small[4];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) big[i] = middle[i] = small[i] = 0.f;
+  }
+  // += a (16 x 16, three terms) . b (16 x 8, three terms; the k-tile's two registers are b[term][j], b[term][j + 1])
+  template <int NB> __device__ __forceinline__ void add(const unsigned (&a)[3][4], const unsigned (&b)[3][NB], int j) {
+    float now[4] = {0.f, 0.f, 0.f, 0.f};
+    mma16816(now, a[0], b[0][j], b[0][j + 1]);
+    mma16816(middle, a[0], b[1][j], b[1][j + 1]);
+    mma16816(small, a[1], b[1][j], b[1][j + 1]);
+    mma16816(middle, a[1], b[0][j], b[0][j + 1]);
+    mma16816(small, a[0], b[2][j], b[2][j + 1]);
+    mma16816(small, a[2], b[0][j], b[0][j + 1]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) big[i] += now[i];
+  }
+  __device__ __forceinline__ float at(int i) const { return big[i] + (middle[i] + small[i]); }
+};
+}  // namespace

@@ -95,7 +95,7 @@ delta_prepare_kernel(const T* proj, long long stride, const float* ab, long long
 template <int NPL, int L, int TB>
 __global__ void __launch_bounds__(128)
 delta_rule_kernel(const float* qkv, const float* gb, const int* row_start, const int* row_slot, float* state,
-                  long long slot_stride, float* out, int H, int G, int D, int Dv, int max_slots) {
+                  long long slot_stride, float* out, int H, int G, int D, int Dv, int max_slots, int max_tokens) {
   constexpr int COLS = 128 / L, DP = NPL * L;
   constexpr int ROWF = (2 * DP + COLS + 2 + 3) / 4 * 4;       // floats of one token in a run: k | q | values | decay, beta
   extern __shared__ __align__(16) float runs[];                // two runs of TB tokens
@@ -112,6 +112,7 @@ delta_rule_kernel(const float* qkv, const float* gb, const int* row_start, const
   const int slot = row_slot[r];
   if (slot < 0 || slot >= max_slots) return;
   const int first = row_start[r], n = row_start[r + 1] - first;
+  if (n > max_tokens) return;                    // a row for the kernels that walk runs of tokens
   const int C = 2 * G * D + H * Dv;
   const int g = h / (H / G);
   const bool live = col < Dv;
@@ -284,7 +285,7 @@ FMX_EXPORT int fmx_delta_prepare(const void* proj, long long stride, const float
 
 FMX_EXPORT int fmx_delta_rule(const float* qkv, const float* gb, const int* row_start, const int* row_slot, float* state,
                               long long slot_stride, float* out, int R, int H, int G, int D, int Dv, int max_slots,
-                              int lanes, cudaStream_t stream) {
+                              int lanes, int max_tokens, cudaStream_t stream) {
   if (R == 0) return 0;
   if (R < 0 || H <= 0 || G <= 0 || H % G || D <= 0 || Dv <= 0 || D > 256)
     return fmx_fail("fmx_delta_rule: bad sizes R=%d H=%d G=%d D=%d Dv=%d", R, H, G, D, Dv);
@@ -297,7 +298,7 @@ FMX_EXPORT int fmx_delta_rule(const float* qkv, const float* gb, const int* row_
     if (smem > 48 * 1024)                                                                                              \
       cudaFuncSetAttribute(delta_rule_kernel<NPL, L, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
     fmx_launch(delta_rule_kernel<NPL, L, TB>, grid, dim3(128), smem, stream, qkv, gb, row_start, row_slot, state,      \
-               slot_stride, out, H, G, D, Dv, max_slots);                                                              \
+               slot_stride, out, H, G, D, Dv, max_slots, max_tokens);                                                              \
   } while (0)
   // Lanes per column: few lanes make a step's sums over lanes short, many lanes make its dots short and give the
   // grid more warps.  `lanes` = 0 leaves the choice here.

@@ -84,7 +84,7 @@ template <int NPL, int L, int TB>
 __global__ void __launch_bounds__(128)
 ssm_scan_kernel(const float* xbc, const float* dd, const float* __restrict__ d_skip, const int* row_start,
                 const int* row_slot, float* state, long long slot_stride, float* out, int H, int G, int N, int P,
-                int max_slots) {
+                int max_slots, int max_tokens) {
   constexpr int COLS = 128 / L, NP = NPL * L;
   constexpr int ROWF = (2 * NP + COLS + 2 + 3) / 4 * 4;       // floats of one token in a run: B | C | x values | dt, decay
   extern __shared__ __align__(16) float runs[];                // two runs of TB tokens
@@ -101,6 +101,7 @@ ssm_scan_kernel(const float* xbc, const float* dd, const float* __restrict__ d_s
   const int slot = row_slot[r];
   if (slot < 0 || slot >= max_slots) return;
   const int first = row_start[r], n = row_start[r + 1] - first;
+  if (n > max_tokens) return;                    // a row for the kernels that walk runs of tokens
   const int inner = H * P, C = inner + 2 * G * N;
   const int g = h / (H / G);
   const bool live = col < P;
@@ -310,7 +311,7 @@ FMX_EXPORT int fmx_ssm_prepare(const void* proj, long long stride, const float* 
 
 FMX_EXPORT int fmx_ssm_scan(const float* xbc, const float* dd, const float* d_skip, const int* row_start,
                             const int* row_slot, float* state, long long slot_stride, float* out, int R, int H, int G, int N,
-                            int P, int max_slots, int lanes, cudaStream_t stream) {
+                            int P, int max_slots, int lanes, int max_tokens, cudaStream_t stream) {
   if (R == 0) return 0;
   if (R < 0 || H <= 0 || G <= 0 || H % G || N <= 0 || P <= 0 || N > 1024)
     return fmx_fail("fmx_ssm_scan: bad sizes R=%d H=%d G=%d N=%d P=%d", R, H, G, N, P);
@@ -323,7 +324,7 @@ FMX_EXPORT int fmx_ssm_scan(const float* xbc, const float* dd, const float* d_sk
     if (smem > 48 * 1024)                                                                                              \
       cudaFuncSetAttribute(ssm_scan_kernel<NPL, L, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
     fmx_launch(ssm_scan_kernel<NPL, L, TB>, grid, dim3(128), smem, stream, xbc, dd, d_skip, row_start, row_slot, state, \
-               slot_stride, out, H, G, N, P, max_slots);                                                               \
+               slot_stride, out, H, G, N, P, max_slots, max_tokens);                                                               \
   } while (0)
   // lanes per column: eight values of state per lane where the state's size allows
   if (lanes == 0) lanes = N <= 64 ? 8 : N <= 128 ? 16 : 32;

@@ -19,6 +19,7 @@ def launch_count() -> int:
     return _lib.launches
 
 F32, BF16 = 0, 1
+WALK_ANY = 0x7fffffff            # a walk token by token that takes rows of any length
 BAD_TOKEN, BAD_SLOT, BAD_PAGE, BAD_ROW = 1, 2, 3, 4
 
 
@@ -584,8 +585,57 @@ def delta_rule(qkv, gb, ctx, state, H, G, D, Dv, lanes: int = 0) -> torch.Tensor
     T = qkv.shape[0]
     out = torch.empty((T, H * Dv), dtype=torch.float32, device=qkv.device)
     call("common", "fmx_delta_rule", qkv.data_ptr(), gb.data_ptr(), ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(),
-         state.data_ptr(), state.stride(0), out.data_ptr(), ctx.R, H, G, D, Dv, state.shape[0], int(lanes), _stream())
+         state.data_ptr(), state.stride(0), out.data_ptr(), ctx.R, H, G, D, Dv, state.shape[0], int(lanes), WALK_ANY, _stream())
     return out
+
+
+def chunk_min_tokens(D: int) -> int:
+    """Rows of at least so many tokens are walked in runs of 32 as matrix products, shorter ones token by token.  Alone, 64 tokens
+    of 64 rows of state take as long either way (the delta rule 19 and 18 us, the plain write 14 and 18), 128 tokens 36 and 18;
+    32 tokens of 128 rows 24 and 19 (18 and 19), 64 tokens 43 and 22.  Decoding rows beside a portion stay on the walk: 63 of
+    them and 128 tokens took 62 us all walked, 131 all in runs."""
+    return 4096 // D
+
+
+def chunk_scan_takes(ctx, D: int, Dv: int) -> bool:
+    """Do the kernels that walk runs of 32 tokens as matrix products take this step's portions (`delta_rule_chunks`,
+    `ssm_scan_chunks`)?  64 or 128 rows of state, values in steps of 16, and a portion long enough to gain by it.  They are as exact
+    as the walk token by token, but a sum's order follows the runs of a portion: a caller that needs the same bits however a
+    prompt is cut (the 32-bit path) takes that walk."""
+    return D in (64, 128) and Dv % 16 == 0 and ctx.max_q_len >= chunk_min_tokens(D)
+
+
+def _has_short_rows(ctx, least: int) -> bool:
+    if ctx.R == 1:
+        return False                      # the longest row is the only one
+    starts = getattr(ctx, "h_row_start", None)
+    return not starts or any(b - a < least for a, b in zip(starts, starts[1:]))
+
+
+def _chunk_scan(kind, x, gates, skip, ctx, state, H, G, D, Dv) -> torch.Tensor:
+    _need_cuda(x, gates, state)
+    assert x.is_contiguous() and x.dtype == torch.float32 and gates.is_contiguous() and gates.dtype == torch.float32
+    T, least = x.shape[0], chunk_min_tokens(D)
+    out = torch.empty((T, H * Dv), dtype=torch.float32, device=x.device)
+    ws = torch.empty(int(load("chunks").fmx_chunk_scan_bytes(T, ctx.R, H, G, D, int(skip is None))), dtype=torch.uint8, device=x.device)
+    more = (skip.data_ptr(),) if skip is not None else ()
+    if _has_short_rows(ctx, least):
+        call("common", f"fmx_{kind}", x.data_ptr(), gates.data_ptr(), *more, ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(),
+             state.data_ptr(), state.stride(0), out.data_ptr(), ctx.R, H, G, D, Dv, state.shape[0], 0, least - 1, _stream())
+    call("chunks", f"fmx_chunk_{kind}", x.data_ptr(), gates.data_ptr(), *more, ctx.row_start.data_ptr(),
+         ctx.row_slot.data_ptr(), state.data_ptr(), state.stride(0), out.data_ptr(), ws.data_ptr(), ws.numel(), T, ctx.R, H, G, D, Dv,
+         state.shape[0], int(ctx.max_q_len), least, _stream())
+    return out
+
+
+def delta_rule_chunks(qkv, gb, ctx, state, H, G, D, Dv) -> torch.Tensor:
+    """`delta_rule` with the step's portions in runs of 32 tokens as matrix products (see `chunk_scan_takes`)."""
+    return _chunk_scan("delta_rule", qkv, gb, None, ctx, state, H, G, D, Dv)
+
+
+def ssm_scan_chunks(xbc, dd, d_skip, ctx, state, H, G, N, P) -> torch.Tensor:
+    """`ssm_scan`, likewise."""
+    return _chunk_scan("ssm_scan", xbc, dd, d_skip, ctx, state, H, G, N, P)
 
 
 def gated_rmsnorm(o, gate, weight, eps, H, Dv, out_dtype, out=None) -> torch.Tensor:
@@ -669,7 +719,7 @@ def ssm_scan(xbc, dd, d_skip, ctx, state, H, G, N, P, lanes: int = 0) -> torch.T
     out = torch.empty((T, H * P), dtype=torch.float32, device=xbc.device)
     call("common", "fmx_ssm_scan", xbc.data_ptr(), dd.data_ptr(), d_skip.data_ptr(), ctx.row_start.data_ptr(),
          ctx.row_slot.data_ptr(), state.data_ptr(), state.stride(0), out.data_ptr(), ctx.R, H, G, N, P, state.shape[0],
-         int(lanes), _stream())
+         int(lanes), WALK_ANY, _stream())
     return out
 
 

@@ -37,7 +37,7 @@ _SIGNATURES = {
         "fmx_qk_prepare": [_P, _L, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _L, _I, _P, _P],
         "fmx_delta_prepare": [_P, _L, _P, _L, _P, _P, _P, _P, _P, _P, _P, _L, _L, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I,
                               _P, _P],
-        "fmx_delta_rule": [_P, _P, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _P],
+        "fmx_delta_rule": [_P, _P, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
         "fmx_gated_rmsnorm": [_P, _P, _L, _P, _P, _L, _I, _I, _I, _F, _I, _P],
         "fmx_activation": [_P, _L, _P, _L, _I, _I, _I, _I, _P],
         "fmx_paged_attention_masked": [_P, _L, _I, _P, _P, _I, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _L, _F, _F, _I, _I,
@@ -56,7 +56,7 @@ _SIGNATURES = {
                                  _F, _F, _P, _P],
         "fmx_latent_rope_prepare": [_P, _L, _I, _P, _L, _P, _P, _P, _F, _P, _P, _L, _I, _P, _I, _I, _I, _I, _I, _I, _P, _P],
         "fmx_ssm_prepare": [_P, _L, _P, _P, _P, _P, _P, _P, _P, _P, _L, _L, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
-        "fmx_ssm_scan": [_P, _P, _P, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _P],
+        "fmx_ssm_scan": [_P, _P, _P, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
         "fmx_gated_group_rmsnorm": [_P, _P, _L, _P, _P, _L, _I, _I, _I, _F, _I, _P],
         "fmx_act_mul": [_P, _P, _I, _I, _I, _I, _I, _P],
         "fmx_embed_scaled": [_P, _I, _P, _P, _I, _I, _L, _F, _P, _I, _P],
@@ -105,6 +105,10 @@ _SIGNATURES = {
         "fmx_mlstm_chunks": [_P, _L, _P, _P, _P, _P, _L, _P, _P, _I, _I, _I, _I, _I, _I, _P],
         "fmx_mlstm_scan": [_P, _L, _P, _P, _P, _P, _L, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
         "fmx_mlstm_step": [_P, _L, _I, _P, _L, _P, _F, _P, _P, _P, _L, _L, _P, _F, _P, _L, _I, _I, _I, _I, _I, _I, _P],
+    },
+    "chunks": {
+        "fmx_chunk_delta_rule": [_P, _P, _P, _P, _P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
+        "fmx_chunk_ssm_scan": [_P, _P, _P, _P, _P, _P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     },
     "mixattn": {
         "fmx_mixattn": [_P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _L, _F, _F, _I, _I, _P, _P, _I, _I, _P, _P],
@@ -156,6 +160,9 @@ def load(group: str) -> ctypes.CDLL:
     if group in ("tc", "tc_expiry"):
         lib.fmx_gemm_tcgen05_plan_width.argtypes = [_I, _I, _I]
         lib.fmx_gemm_tcgen05_plan_fills.argtypes = [_I, _I, _I]
+    if group == "chunks":
+        lib.fmx_chunk_scan_bytes.argtypes = [_I, _I, _I, _I, _I, _I]
+        lib.fmx_chunk_scan_bytes.restype = c_longlong
     lib.fmx_last_error.restype = ctypes.c_char_p
     family = "attn_vd" if values_differ else "attn" if group.startswith("attn_hd") else "tc" if group == "tc_expiry" else \
         "mixattn" if group.startswith("mixattn_v") else group

@@ -78,7 +78,9 @@ class GatedDeltaMixer(Mixer):
         ab = self.ba.forward(x, out_dtype=torch.float32)
         qkv, gb = k.delta_prepare(proj, ab, self.conv_w, self.a_log, self.dt_bias, ctx, cache.state, self.s_floats,
                                   self.H, self.G, self.D, self.Dv, self.taps)
-        o = k.delta_rule(qkv, gb, ctx, cache.state, self.H, self.G, self.D, self.Dv)
+        takes = getattr(k, "chunk_scan_takes", None) if self.rt.dtype == torch.bfloat16 else None
+        rule = k.delta_rule_chunks if takes is not None and takes(ctx, self.D, self.Dv) else k.delta_rule
+        o = rule(qkv, gb, ctx, cache.state, self.H, self.G, self.D, self.Dv)
         return k.gated_rmsnorm(o, proj[:, self.channels:], self.norm_w, self.eps, self.H, self.Dv, self.rt.dtype, out=out)
 
     def forward(self, x, ctx, cache):

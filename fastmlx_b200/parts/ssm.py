@@ -78,6 +78,8 @@ class StateSpaceMixer(Mixer):
         # convolution, SiLU, step sizes and decays: x | B | C in 32-bit, (dt | decay) per head
         xbc, dd = k.ssm_prepare(proj, self.conv_w, self.conv_b, self.a_log, self.dt_bias, ctx, cache.state, self.s_floats,
                                 self.H, self.G, self.N, self.P, self.taps)
-        y = k.ssm_scan(xbc, dd, self.d_skip, ctx, cache.state, self.H, self.G, self.N, self.P)
+        takes = getattr(k, "chunk_scan_takes", None) if self.rt.dtype == torch.bfloat16 else None
+        scan = k.ssm_scan_chunks if takes is not None and takes(ctx, self.N, self.P) else k.ssm_scan
+        y = scan(xbc, dd, self.d_skip, ctx, cache.state, self.H, self.G, self.N, self.P)
         y = k.gated_group_rmsnorm(y, proj[:, :self.inner], self.norm_w, self.eps, self.norm_groups, self.rt.dtype)
         return self.o.forward(y)

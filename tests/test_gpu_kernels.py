@@ -792,3 +792,57 @@ def test_greedy_head_chooses_the_largest_logit(M, V, K):
             assert int(ids[0]) == 3
     best_words, ticket = k().greedy_workspace(DEV)
     assert int(ticket) == 0 and int(best_words.abs().sum()) == 0
+
+
+@pytest.mark.parametrize("rule", ["delta", "plain"])
+@pytest.mark.parametrize("lens,H,G,D,P", [((64,), 4, 2, 64, 64), ((65, 1, 97, 31, 128), 4, 2, 64, 48), ((63, 200), 3, 3, 64, 16),
+                                          ((32, 33, 7), 4, 1, 128, 128), ((31, 64), 2, 2, 128, 16), ((1, 2, 40, 96), 64, 8, 128, 32)])
+def test_portions_in_runs_of_tokens(rule, lens, H, G, D, P):
+    """The kernels that walk runs of 32 tokens as matrix products, against 64-bit arithmetic and beside the walk token by token:
+    portions of whole runs and a token more or less, rows too short for them, decays that are zero or nearly one, slots with state
+    and slots out of order; what lies behind a slot's matrices stays."""
+    torch.manual_seed(D + len(lens))
+    starts = [0] + list(torch.tensor(lens).cumsum(0).tolist())
+    T, R = starts[-1], len(lens)
+    order = list(range(R))[::-1]
+    ctx = SimpleNamespace(R=R, row_start=torch.tensor(starts, dtype=torch.int32, device=DEV), max_q_len=max(lens), h_row_start=starts,
+                          row_slot=torch.tensor(order, dtype=torch.int32, device=DEV))
+    q, kk, v = torch.randn(T, G, D), torch.nn.functional.normalize(torch.randn(T, G, D) + 0.3, dim=-1), torch.randn(T, H, P)
+    q = torch.nn.functional.normalize(q, dim=-1)
+    decay, w = torch.rand(T, H) ** torch.rand(H), torch.rand(T, H)
+    decay[torch.rand(T, H) < 0.05] = 0.0
+    decay[:, 0] = 1.0 - 1e-3 * torch.rand(T)
+    state = torch.randn(R, H * P * D + 12)
+    skip = torch.randn(H)
+    if rule == "delta":
+        x, gates = torch.cat([q.flatten(1), kk.flatten(1), v.flatten(1)], 1), torch.cat([decay, w], 1)
+        walk, runs = k().delta_rule, k().delta_rule_chunks
+        call = lambda fn, s: fn(x.to(DEV), gates.to(DEV), ctx, s, H, G, D, P)
+    else:
+        x, gates = torch.cat([v.flatten(1), kk.flatten(1), q.flatten(1)], 1), torch.cat([w, decay], 1)
+        walk, runs = k().ssm_scan, k().ssm_scan_chunks
+        call = lambda fn, s: fn(x.to(DEV), gates.to(DEV), skip.to(DEV), ctx, s, H, G, D, P)
+    assert k().chunk_scan_takes(ctx, D, P)
+    s1, s2 = state.to(DEV), state.to(DEV)
+    o1, o2 = call(walk, s1).cpu().double().view(T, H, P), call(runs, s2).cpu().double().view(T, H, P)
+    assert torch.equal(s2[:, H * P * D:].cpu(), state[:, H * P * D:])
+    f = lambda t: t.double().repeat_interleave(H // G, 1)
+    want, left = torch.empty(T, H, P, dtype=torch.float64), state.double().clone()
+    for r in range(R):
+        S = left[order[r], :H * P * D].view(H, P, D)
+        for t in range(starts[r], starts[r + 1]):
+            S = S * decay[t].double()[:, None, None]
+            u = v[t].double()
+            if rule == "delta":
+                u = u - torch.einsum("hpd,hd->hp", S, f(kk[t:t + 1])[0])
+            S = S + (w[t].double()[:, None] * u)[:, :, None] * f(kk[t:t + 1])[0][:, None, :]
+            want[t] = torch.einsum("hpd,hd->hp", S, f(q[t:t + 1])[0]) + (0 if rule == "delta" else skip.double()[:, None] * v[t].double())
+        left[order[r], :H * P * D] = S.flatten()
+    # roundings of 2^-24 of the largest value a sum meets, some dozens of which meet in a value at random signs
+    for got, ref in ((o2, want), (s2[:, :H * P * D].cpu().double(), left[:, :H * P * D])):
+        assert (got - ref).abs().max() < 40 * 2.0 ** -24 * ref.abs().max()
+    err = lambda o: ((o - want).norm() / want.norm()).item()
+    assert err(o2) < 1.5 * err(o1) + 2e-8
+    for r in range(R):                               # rows too short for runs are walked: the same bits
+        if lens[r] < k().chunk_min_tokens(D):
+            assert torch.equal(o1[starts[r]:starts[r + 1]], o2[starts[r]:starts[r + 1]])
