@@ -34,7 +34,8 @@ GROUPS = {
     "chan": "chan",
     # the matrix memory with exponential gates
     "mlstm": "mlstm",
-    # recurrences with a decay per head over portions, in runs of tokens as matrix products
+    # 32-bit contractions on the tensor cores, operands as three bfloat16 terms: recurrences with a decay per head in runs of
+    # tokens, sigmoid attention with mixed heads over portions
     "chunks": "chunks",
     # host code: the native step executor (no kernel of its own)
     "host": "host",

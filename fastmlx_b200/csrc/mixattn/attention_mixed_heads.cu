@@ -16,8 +16,9 @@
 //
 // Queries are 32-bit, keys and values are exact in 32-bit, and every sum is made of 32-bit multiply-adds in an order that
 // the indices alone fix (over heads and over keys one chain in index order; a dot product two chains, over the even and
-// the odd runs of eight dimensions): no tensor cores, because a weight that is a 32-bit sum of
-// 32-bit sigmoids has no two-term bfloat16 form that the mix would keep.  Nothing is normalised over the keys, so a
+// the odd runs of eight dimensions).  On the tensor cores a weight that is a 32-bit sum of 32-bit sigmoids takes three
+// bfloat16 terms: ../chunks/attention_mixed_heads_tc.cu does so for portions of the sizes that it takes; single tokens, which
+// would leave seven of its eight columns empty, and the other sizes run here.  Nothing is normalised over the keys, so a
 // token's keys may be shared out over `splits` blocks whose partial outputs a second kernel adds up in split order.
 //
 // One library per (FMX_VPL, FMX_PER): FMX_VPL value dimensions per lane (values up to 32 * FMX_VPL wide), FMX_PER query
@@ -98,7 +99,7 @@ mixed_heads_attention_kernel(const float* q, long long q_stride, const bf16* kv,
                              long long out_stride, int n_tokens, int nh, int nkv, int hd, int vd, int page_size,
                              long long num_pages, float scale, float softcap, int window, int R,
                              const float* __restrict__ head_bias, const float* __restrict__ mix, int TQ, int splits,
-                             int* status) {
+                             int max_tokens, int* status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_wait();
   pdl_trigger();
@@ -110,6 +111,7 @@ mixed_heads_attention_kernel(const float* q, long long q_stride, const bf16* kv,
   }
   const int first = row_start[row];
   if ((t0 - first) % TQ != 0) return;                 // another block's tile holds this token
+  if (row_start[row + 1] - first > max_tokens) return;          // a row for the kernel on the tensor cores
   const int n_q = min(TQ, row_start[row + 1] - t0);
   const int per = nh / nkv;
   const Layout L = layout_for(TQ, nh, nkv, hd);
@@ -458,12 +460,12 @@ FMX_EXPORT int fmx_mixattn_plan(int n_tokens, int nh, int nkv, int hd, int vd, i
 
 // q [T, nh*hd] 32-bit; kv: bfloat16 pages of [nkv, page, hd] keys and [nkv, page, vd] values; out [T, nh*vd] bfloat16
 // in rows of out_stride; part: splits * T * nh * vd floats where splits > 1; mix [nh, nh] and head_bias [nh] (or null)
-// 32-bit.  row_start [R + 1]: where each row's tokens start in the step.
+// 32-bit.  row_start [R + 1]: where each row's tokens start in the step.  Rows of more than max_tokens tokens are left out.
 FMX_EXPORT int fmx_mixattn(const float* q, long long q_stride, const void* kv, const int* block_tables, int bt_stride,
                            const int* token_row, const int* positions, const int* row_start, float* part, void* out,
                            long long out_stride, int n_tokens, int nh, int nkv, int hd, int vd, int page_size,
                            long long num_pages, float scale, float softcap, int window, int R, const float* head_bias,
-                           const float* mix, int max_q_len, int splits, int* status, cudaStream_t stream) {
+                           const float* mix, int max_q_len, int splits, int max_tokens, int* status, cudaStream_t stream) {
   if (n_tokens == 0) return 0;
   if (n_tokens < 0 || page_size <= 0 || window < 0 || splits < 1 || (splits > 1 && part == nullptr) || mix == nullptr)
     return fmx_fail("fmx_mixattn: bad sizes T=%d page=%d window=%d splits=%d", n_tokens, page_size, window, splits);
@@ -483,7 +485,7 @@ FMX_EXPORT int fmx_mixattn(const float* q, long long q_stride, const void* kv, c
     }
     fmx_launch(kernel, grid, dim3(nw * 32), L.total, stream, q, q_stride, (const bf16*)kv, block_tables, bt_stride, token_row,
                positions, row_start, part, (bf16*)out, out_stride, n_tokens, nh, nkv, hd, vd, page_size, num_pages, scale,
-               softcap, window, R, head_bias, mix, tq, splits, status);
+               softcap, window, R, head_bias, mix, tq, splits, max_tokens, status);
     return 0;
   };
   int rc;

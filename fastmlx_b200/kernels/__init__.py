@@ -809,17 +809,25 @@ def mixed_heads_library(nh: int, nkv: int, hd: int, vd: int, q=None, kv=None) ->
     return f"mixattn_v{vpl}_p{per}" if vpl and per else None
 
 
+# A tile on the tensor cores takes as long for one token as for its eight.  32 rows behind 500 tokens: 2 tokens each 155 us on
+# 32-bit multiply-adds, 4 each 195 us, on the tensor cores 48.
+MIXED_TC_MIN_TOKENS = 4
+
+
 def sigmoid_attention(q, kv, ctx, group, nh, nkv, hd, vd, scale, softcap, window, page_size, head_bias, mix, out=None,
-                      out_dtype=None, tiled: bool | None = None) -> torch.Tensor:
+                      out_dtype=None, tiled: bool | None = None, tensor_cores: bool | None = None) -> torch.Tensor:
     """Attention without a softmax: a visible key weighs sigmoid(cap(scale q.k) + head_bias[head]); the heads' weights are
     mixed by `mix` ([nh, nh], 32-bit: row h lists what head h takes of every head's weights) and head h applies its mixed
     weights to the values of its own key/value head.  Queries q[T, nh*hd] of their own type over pages of [nkv, page, hd]
     keys and [nkv, page, vd] values; scores, weights and the sums over keys are 32-bit.  -> [T, nh*vd].
 
     Two kernels: over bfloat16 pages a block owns all heads of a tile of tokens and mixes the weights before they meet
-    the values (prompt portions and single tokens; a single token's keys may be shared out over several blocks); else,
+    the values (prompt portions and single tokens; a single token's keys may be shared out over several blocks), rows of at
+    least MIXED_TC_MIN_TOKENS tokens on the tensor cores with three-term operands where their kernel takes the sizes (heads of at
+    most 64 values in steps of 16, at most 8 key heads of at most 4 query heads); else,
     and on the 32-bit path, one warp per (token, head, value head) sums the unmixed heads' outputs, which a second
-    kernel mixes.  `tiled`: force the choice (None: the tiled kernel where it takes the sizes)."""
+    kernel mixes.  `tiled`: force the choice (None: the tiled kernel where it takes the sizes); `tensor_cores=False`: all
+    rows on 32-bit multiply-adds."""
     _need_cuda(q, kv, head_bias, mix, out)
     assert kv.is_contiguous() and q.stride(1) == 1
     T = q.shape[0]
@@ -831,15 +839,25 @@ def sigmoid_attention(q, kv, ctx, group, nh, nkv, hd, vd, scale, softcap, window
     bt = group.block_tables
     name = mixed_heads_library(nh, nkv, hd, vd, q, kv) if tiled is not False and out.dtype == torch.bfloat16 else None
     if name is not None:
-        lib = load(name)
-        splits = int(lib.fmx_mixattn_plan(T, nh, nkv, hd, vd, int(ctx.max_q_len), int(ctx.max_ctx_after)))
+        def launch(fn, lib, part, *last):
+            call(lib, fn, q.data_ptr(), q.stride(0), kv.data_ptr(), bt.data_ptr(), bt.stride(0), ctx.token_row.data_ptr(),
+                 ctx.positions.data_ptr(), ctx.row_start.data_ptr(), _ptr(part), out.data_ptr(), out.stride(0), T, nh, nkv, hd, vd,
+                 int(page_size), kv.shape[0], float(scale), float(softcap or 0.0), int(window), bt.shape[0], _ptr(head_bias),
+                 mix.data_ptr(), *last, _ptr(ctx.status), _stream())
+
+        def parts(splits):
+            return torch.empty((splits, T, nh * vd), dtype=torch.float32, device=q.device) if splits > 1 else None
+        least = WALK_ANY
+        if tensor_cores is not False and ctx.max_q_len >= MIXED_TC_MIN_TOKENS and kv.data_ptr() % 16 == 0:
+            splits = int(load("chunks").fmx_mixattn_tc_plan(T, ctx.R, nh, nkv, hd, vd, int(ctx.max_q_len), int(ctx.max_ctx_after)))
+            if splits > 0:
+                least = MIXED_TC_MIN_TOKENS
+                launch("fmx_mixattn_tc", "chunks", parts(splits), least, splits)
+                if not _has_short_rows(ctx, least):
+                    return out
+        splits = int(load(name).fmx_mixattn_plan(T, nh, nkv, hd, vd, int(ctx.max_q_len), int(ctx.max_ctx_after)))
         if splits > 0:
-            part = torch.empty((splits, T, nh * vd), dtype=torch.float32, device=q.device) if splits > 1 else None
-            call(name, "fmx_mixattn", q.data_ptr(), q.stride(0), kv.data_ptr(), bt.data_ptr(), bt.stride(0),
-                 ctx.token_row.data_ptr(), ctx.positions.data_ptr(), ctx.row_start.data_ptr(), _ptr(part), out.data_ptr(),
-                 out.stride(0), T, nh, nkv, hd, vd, int(page_size), kv.shape[0], float(scale), float(softcap or 0.0),
-                 int(window), bt.shape[0], _ptr(head_bias), mix.data_ptr(), int(ctx.max_q_len), splits, _ptr(ctx.status),
-                 _stream())
+            launch("fmx_mixattn", name, parts(splits), int(ctx.max_q_len), splits, least - 1 if least != WALK_ANY else least)
             return out
     assert tiled is not True, "the tiled kernel does not take these sizes"
     part = torch.empty((T, nh, nkv, vd), dtype=torch.float32, device=q.device)

@@ -107,11 +107,13 @@ _SIGNATURES = {
         "fmx_mlstm_step": [_P, _L, _I, _P, _L, _P, _F, _P, _P, _P, _L, _L, _P, _F, _P, _L, _I, _I, _I, _I, _I, _I, _P],
     },
     "chunks": {
+        "fmx_mixattn_tc": [_P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _L, _F, _F, _I, _I, _P, _P, _I, _I, _P, _P],
+        "fmx_mixattn_tc_plan": [_I, _I, _I, _I, _I, _I, _I, _I],
         "fmx_chunk_delta_rule": [_P, _P, _P, _P, _P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
         "fmx_chunk_ssm_scan": [_P, _P, _P, _P, _P, _P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     },
     "mixattn": {
-        "fmx_mixattn": [_P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _L, _F, _F, _I, _I, _P, _P, _I, _I, _P, _P],
+        "fmx_mixattn": [_P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _L, _F, _F, _I, _I, _P, _P, _I, _I, _I, _P, _P],
         "fmx_mixattn_plan": [_I, _I, _I, _I, _I, _I, _I],
     },
     "attn": {

@@ -846,3 +846,56 @@ def test_portions_in_runs_of_tokens(rule, lens, H, G, D, P):
     for r in range(R):                               # rows too short for runs are walked: the same bits
         if lens[r] < k().chunk_min_tokens(D):
             assert torch.equal(o1[starts[r]:starts[r + 1]], o2[starts[r]:starts[r + 1]])
+
+
+@pytest.mark.parametrize("lens,ctxs,nh,nkv,hd,vd,page,window,cap", [
+    ((4,), (0,), 2, 1, 16, 16, 16, 0, 30.0), ((9, 1, 33), (0, 40, 31), 8, 8, 32, 64, 8, 0, 30.0), ((40, 3, 8), (3, 0, 57), 32, 8, 64, 64, 16, 20, 30.0),
+    ((50,), (77,), 6, 3, 48, 32, 16, 0, 0.0), ((17, 5), (200, 0), 12, 3, 64, 16, 5, 0, 2.0), ((264, 31), (0, 700), 32, 8, 64, 64, 16, 0, 30.0)])
+def test_mixed_heads_on_tensor_cores(lens, ctxs, nh, nkv, hd, vd, page, window, cap):
+    """Sigmoid attention with mixed heads over portions with three-term operands, against 64-bit arithmetic and beside the kernel of
+    32-bit multiply-adds: tiles of tokens and keys with remainders, rows that stay on the other kernel, fewer heads than a tile
+    has, windows, scores far beyond the small tangent's range, pages whose unused places hold NaN, keys shared out over blocks."""
+    torch.manual_seed(nh + hd)
+    R, starts = len(lens), [0] + list(torch.tensor(lens).cumsum(0).tolist())
+    T, blocks = starts[-1], [-(-(c + n) // page) for c, n in zip(ctxs, lens)]
+    perm = torch.randperm(sum(blocks) + 3).tolist()
+    bt = torch.full((R, max(blocks) + 1), -1, dtype=torch.int32)
+    kv = torch.full((sum(blocks) + 3, nkv * page * (hd + vd)), float("nan")).bfloat16()
+    K = [torch.randn(c + n, nkv, hd).bfloat16() for c, n in zip(ctxs, lens)]
+    V = [torch.randn(c + n, nkv, vd).bfloat16() for c, n in zip(ctxs, lens)]
+    for r in range(R):
+        for b in range(blocks[r]):
+            p = bt[r, b] = perm.pop()
+            k_, v_ = K[r][b * page:(b + 1) * page], V[r][b * page:(b + 1) * page]
+            kv[p, :nkv * page * hd].view(nkv, page, hd)[:, :len(k_)] = k_.transpose(0, 1)
+            kv[p, nkv * page * hd:].view(nkv, page, vd)[:, :len(v_)] = v_.transpose(0, 1)
+    kv = (kv.view(-1, 2, nkv, page, hd) if hd == vd else kv).to(DEV)
+    q, mix, bias = torch.randn(T, nh * hd) * 2, torch.eye(nh) + 0.1 * torch.randn(nh, nh), torch.randn(nh) * 0.5 - 3
+    pos = torch.cat([torch.arange(c, c + n) for c, n in zip(ctxs, lens)])
+    ctx = SimpleNamespace(R=R, T=T, positions=pos.int().to(DEV), token_row=torch.arange(R).repeat_interleave(torch.tensor(lens)).int().to(DEV),
+                          row_start=torch.tensor(starts, dtype=torch.int32, device=DEV), h_row_start=starts, max_q_len=max(lens),
+                          max_ctx_after=max(c + n for c, n in zip(ctxs, lens)), status=torch.zeros(4, dtype=torch.int32, device=DEV))
+    run = lambda tc: k().sigmoid_attention(q.to(DEV), kv, ctx, SimpleNamespace(block_tables=bt.to(DEV)), nh, nkv, hd, vd, hd ** -0.5, cap, window,
+                                           page, bias.to(DEV), mix.to(DEV), tensor_cores=tc).cpu().double().view(T, nh, vd)
+    plan = k().load("chunks").fmx_mixattn_tc_plan(T, R, nh, nkv, hd, vd, ctx.max_q_len, ctx.max_ctx_after)
+    assert plan >= 1 and (plan > 1 or ctx.max_ctx_after < 256)
+    fma, got = run(False), run(None)
+    assert ctx.status.tolist()[0] == 0
+    want, size = torch.empty(T, nh, vd, dtype=torch.float64), torch.empty(T, nh, vd, dtype=torch.float64)
+    for r in range(R):
+        at = slice(starts[r], starts[r + 1])
+        kk, vv = (t[r].double().repeat_interleave(nh // nkv, 1) for t in (K, V))
+        s = torch.einsum("qhd,khd->hqk", q[at].double().view(-1, nh, hd), kk) * hd ** -0.5
+        s = cap * torch.tanh(s / cap) if cap else s
+        kp, qp = torch.arange(len(kk)), pos[at]
+        hidden = (kp[None] > qp[:, None]) | ((kp[None] <= qp[:, None] - window) if window else False)
+        w = torch.sigmoid(s + bias.double()[:, None, None]).masked_fill(hidden, 0.0)
+        want[at] = torch.einsum("hqk,khd->qhd", torch.einsum("hg,gqk->hqk", mix.double(), w), vv)
+        size[at] = torch.einsum("hqk,khd->qhd", torch.einsum("hg,gqk->hqk", mix.double().abs(), w), vv.abs())
+    # the rounding to bfloat16, and 2^-24 of what a value's sums add up to for some dozens of roundings in 32-bit
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 48 * 2.0 ** -24 * size).all()
+    off = lambda o: (o != want.bfloat16().double()).double().mean().item()
+    assert off(got) < off(fma) + 1e-3
+    for r in range(R):
+        if lens[r] < k().MIXED_TC_MIN_TOKENS:        # these rows run where they ran
+            assert torch.equal(got[starts[r]:starts[r + 1]], fma[starts[r]:starts[r + 1]])
