@@ -17,8 +17,7 @@
 // Everything is 32-bit but the projections that come in and the activations that go out.
 #include <math.h>
 #include "common.cuh"
-#include "conv_state.cuh"
-#include "packed.cuh"
+#include "conv_strip.cuh"
 
 namespace {
 __device__ __forceinline__ float softplus_f(float a) { return fmaxf(a, 0.f) + log1pf(expf(-fabsf(a))); }
@@ -137,6 +136,35 @@ channel_delta_prepare_kernel(const T* proj, long long stride, const T* b, long l
   for (int k = 0; k < MAXI; ++k) {
     const int e = lane + 32 * k;
     if (e < D) dst[e] = v[k] * mul;
+  }
+}
+
+// The same by strips of tokens (conv_strip.cuh); behind the blocks of channels those of decays, four of a token to a thread, whose
+// first ones work the write strengths out too.
+template <int LG>
+__global__ void __launch_bounds__(128)
+channel_delta_prepare_strip_kernel(ConvStrip a, int blocks, const bf16* b, long long b_stride, const float* z, long long z_stride,
+                                   const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* out_g, float* out_beta, int H,
+                                   int D) {
+  pdl_wait();
+  pdl_trigger();
+  if ((int)blockIdx.y < blocks) {
+    conv_strip<LG>(a, blockIdx.x, blockIdx.y);
+    return;
+  }
+  const int t0 = blockIdx.x * a.strip, t1 = min(a.T, t0 + a.strip), e = (((int)blockIdx.y - blocks) * 128 + threadIdx.x) * 4;
+  if ((int)blockIdx.y == blocks)
+    for (int i = threadIdx.x; i < (t1 - t0) * H; i += 128) {
+      const int t = t0 + i / H, h = i % H;
+      out_beta[(long long)t * H + h] = 1.0f / (1.0f + expf(-to_f(b[(long long)t * b_stride + h])));
+    }
+  if (e >= H * D) return;
+  const float rate = expf(a_log[e / D]);
+  const float4 bias = load4(dt_bias + e);
+  for (int t = t0; t < t1; ++t) {
+    const float4 x = load4(z + (long long)t * z_stride + e);
+    store4(out_g + (long long)t * H * D + e, make_float4(expf(-rate * softplus_f(x.x + bias.x)), expf(-rate * softplus_f(x.y + bias.y)),
+                                                        expf(-rate * softplus_f(x.z + bias.z)), expf(-rate * softplus_f(x.w + bias.w))));
   }
 }
 
@@ -456,6 +484,27 @@ FMX_EXPORT int fmx_channel_delta_prepare(const void* proj, long long stride, con
     return fmx_fail("fmx_channel_delta_prepare: bad sizes T=%d R=%d H=%d G=%d D=%d Dv=%d taps=%d", T, R, H, G, D, Dv, taps);
   const int C = 2 * G * D + H * Dv;
   if (stride < C || b_stride < H || z_stride < (long long)H * D) return fmx_fail("fmx_channel_delta_prepare: rows too narrow");
+  if (dtype == FMX_BF16) {
+    ConvStrip a = {(const bf16*)proj, stride, conv_w, nullptr, token_row, row_start, row_slot, state, slot_stride, conv_off, out_qkv, T, C, R,
+                   max_slots, 1, 2 * G * D, G * D, 1.0f / sqrtf((float)D), single != 0, status};
+    if (strip_takes(a, taps, D) && z_stride % 4 == 0 && ((uintptr_t)z & 15) == 0 && ((uintptr_t)dt_bias & 15) == 0 && ((uintptr_t)out_g & 15) == 0) {
+      const int blocks = (C + STRIP_CHANNELS - 1) / STRIP_CHANNELS, more = (H * D + 511) / 512;
+      a.strip = strip_length(T, blocks + more);
+      const dim3 grid((T + a.strip - 1) / a.strip, blocks + more);
+#define FMX_CDS(LG)                                                                                                    \
+  fmx_launch(channel_delta_prepare_strip_kernel<LG>, grid, dim3(128), 0, stream, a, blocks, (const bf16*)b, b_stride, z, z_stride, a_log, \
+             dt_bias, out_g, out_beta, H, D)
+      if (D == 32) FMX_CDS(8);
+      else if (D == 64) FMX_CDS(16);
+      else FMX_CDS(32);
+#undef FMX_CDS
+      if (!single)
+        fmx_launch(conv_state_update_kernel<bf16>, dim3((C + 127) / 128, R), dim3(128), 0, stream, (const bf16*)proj, stride, row_start,
+                   row_slot, state, slot_stride, conv_off, C, taps, max_slots);
+      FMX_LAUNCH_CHECK();
+      return 0;
+    }
+  }
   // two channels at a time: every head, row and slot starts on a pair
   const bool two = D % 2 == 0 && Dv % 2 == 0 && stride % 2 == 0 && z_stride % 2 == 0 && slot_stride % 2 == 0 && conv_off % 2 == 0 &&
                    ((uintptr_t)z & 7) == 0 && ((uintptr_t)dt_bias & 7) == 0 && ((uintptr_t)state & 7) == 0 &&

@@ -29,13 +29,13 @@ head_norm_gate_kernel(const float* o, const TG* gate, long long gate_stride, con
   const TG* gp = gate + t * gate_stride + (long long)h * Dv;
   T* dst = out + t * out_stride + (long long)h * Dv;
   const float mul = over_normaliser(nq, gates, item);
-  const float* wp = w + (long long)h * w_stride;
+  const float* wp = w == nullptr ? w : w + (long long)h * w_stride;
   float ss = 0.f;
   for (int e = lane; e < Dv; e += 32) ss = fmaf(op[e] * mul, op[e] * mul, ss);
   const float rstd = mul / sqrtf(warp_sum(ss) / (float)Dv + eps);
   for (int e = lane; e < Dv; e += 32) {
     const float x = to_f(gp[e]), sg = 1.0f / (1.0f + expf(-x));
-    dst[e] = from_f<T>(op[e] * rstd * wp[e] * (silu ? x * sg : sg));
+    dst[e] = from_f<T>(op[e] * rstd * (w == nullptr ? 1.0f : wp[e]) * (silu ? x * sg : sg));
   }
 }
 
@@ -61,7 +61,8 @@ head_norm_gate_vec_kernel(const float* o, const TG* gate, long long gate_stride,
   for (int d = LG / 2; d >= 1; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
   if (!live) return;
   const float rstd = 1.0f / sqrtf(ss / (float)Dv + eps);
-  const float4 g = load4(gate + t * gate_stride + (long long)h * Dv + e), ww = load4(w + (long long)h * w_stride + e);
+  const float4 g = load4(gate + t * gate_stride + (long long)h * Dv + e);
+  const float4 ww = w == nullptr ? make_float4(1.f, 1.f, 1.f, 1.f) : load4(w + (long long)h * w_stride + e);
   auto act = [&](float v) { const float sg = 1.0f / (1.0f + expf(-v)); return silu ? v * sg : sg; };
   store4(out + t * out_stride + (long long)h * Dv + e, make_float4(x.x * rstd * ww.x * act(g.x), x.y * rstd * ww.y * act(g.y),
                                                                   x.z * rstd * ww.z * act(g.z), x.w * rstd * ww.w * act(g.w)));
@@ -69,7 +70,7 @@ head_norm_gate_vec_kernel(const float* o, const TG* gate, long long gate_stride,
 }  // namespace
 
 // o [T, H*Dv] 32-bit; gate rows of gate_stride elements of type g_dtype; out rows of out_stride elements of type dtype; head h's
-// weights start at w + h * w_stride (0: one weight of Dv values for all heads).  nq [T, H] and gates [T, H, 4], or both null: o is first
+// weights start at w + h * w_stride (0: one weight of Dv values for all heads; w null: none).  nq [T, H] and gates [T, H, 4], or both null: o is first
 // divided by max(|nq|, gates[.., 2]) + 1e-6.
 FMX_EXPORT int fmx_head_norm_gate(const float* o, const void* gate, long long gate_stride, int g_dtype, const float* w, void* out,
                                   long long out_stride, int dtype, int T, int H, int Dv, float eps, int silu, int w_stride, const float* nq,

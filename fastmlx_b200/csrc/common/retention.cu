@@ -4,18 +4,22 @@
 //     S <- decay_h S + k v^T;   o = S^T q,
 // S [D, P] in 32-bit in a state slot of the request, carried from step to step.  That is the state-space
 // recurrence of ssm.cu with a step size of 1, a decay that no token changes, as many groups as heads and no skip
-// term, so the recurrence itself runs on ssm_scan; the two kernels here stand in front of it and behind it.
+// term, so the recurrence itself runs on ssm_scan; what is here stands in front of it and behind it.
 //
 //   retention_prepare    per token: q and k of every head rotated over their first `rot` dimensions (dimension i
 //                        paired with i + rot/2; angle, sine and cosine in 32-bit), k multiplied by `k_scale` after
 //                        the rotation; out [T, C] in 32-bit, C = H*P + 2*H*D, laid out as the scan takes its
 //                        operands: v | k | q; and per head a step size of 1 and the head's decay, [T, 2H].
-//   retention_gate_norm  one warp per (token, head): o divided by its root mean square over the head (no weight),
-//                        times silu(gate), out in the run's type.
+//   retention_gate_norm  o divided by its root mean square over the head (no weight), times silu(gate), out in the
+//                        run's type: the kernels of head_norm.cu.
 //
 // Everything is 32-bit but the projection that comes in and the activations that go out.
 #include <math.h>
 #include "common.cuh"
+
+extern "C" int fmx_head_norm_gate(const float* o, const void* gate, long long gate_stride, int g_dtype, const float* w, void* out,
+                                  long long out_stride, int dtype, int T, int H, int Dv, float eps, int silu, int w_stride, const float* nq,
+                                  const float* gates, cudaStream_t stream);
 
 namespace {
 // proj [T, stride]: q (H*D) | k (H*D) | v (H*P)
@@ -64,28 +68,6 @@ retention_prepare_kernel(const T* proj, long long stride, const int* positions, 
   }
 }
 
-template <typename TG, typename T>
-__global__ void __launch_bounds__(128)
-retention_gate_norm_kernel(const float* o, const TG* gate, long long g_stride, T* out, long long out_stride, long long n_heads,
-                           int H, int P, float eps) {
-  pdl_wait();
-  pdl_trigger();
-  const int lane = threadIdx.x & 31;
-  const long long w = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (w >= n_heads) return;
-  const long long t = w / H;
-  const int h = (int)(w - t * H);
-  const float* op = o + w * P;
-  float ss = 0.f;
-  for (int e = lane; e < P; e += 32) ss = fmaf(op[e], op[e], ss);
-  const float rstd = 1.0f / sqrtf(warp_sum(ss) / (float)P + eps);
-  const TG* gp = gate + t * g_stride + (long long)h * P;
-  T* dst = out + t * out_stride + (long long)h * P;
-  for (int e = lane; e < P; e += 32) {
-    const float g = to_f(gp[e]);
-    dst[e] = from_f<T>(op[e] * rstd * (g / (1.0f + expf(-g))));
-  }
-}
 }  // namespace
 
 // rot = 0: nothing is rotated (inv_freq may then be null).  dtype: the projection's type.
@@ -113,19 +95,5 @@ FMX_EXPORT int fmx_retention_prepare(const void* proj, long long stride, int dty
 // o [T, H*P] 32-bit; gate rows of g_stride elements of type g_dtype; out rows of out_stride elements of type dtype.
 FMX_EXPORT int fmx_retention_gate_norm(const float* o, const void* gate, long long g_stride, int g_dtype, void* out,
                                        long long out_stride, int dtype, int T, int H, int P, float eps, cudaStream_t stream) {
-  if (T == 0) return 0;
-  if (T < 0 || H <= 0 || P <= 0 || g_stride < (long long)H * P || out_stride < (long long)H * P)
-    return fmx_fail("fmx_retention_gate_norm: bad sizes T=%d H=%d P=%d", T, H, P);
-  const long long n = (long long)T * H, grid = (n + 3) / 4;
-  if (grid > 2147483647LL) return fmx_fail("fmx_retention_gate_norm: batch too large");
-#define FMX_RGN(TG, TO)                                                                                               \
-  fmx_launch(retention_gate_norm_kernel<TG, TO>, dim3((unsigned)grid), dim3(128), 0, stream, o, (const TG*)gate, g_stride, \
-             (TO*)out, out_stride, n, H, P, eps)
-  if (g_dtype == FMX_F32 && dtype == FMX_F32) FMX_RGN(float, float);
-  else if (g_dtype == FMX_F32 && dtype == FMX_BF16) FMX_RGN(float, bf16);
-  else if (g_dtype == FMX_BF16 && dtype == FMX_BF16) FMX_RGN(bf16, bf16);
-  else return fmx_fail("fmx_retention_gate_norm: unknown dtypes %d, %d", g_dtype, dtype);
-#undef FMX_RGN
-  FMX_LAUNCH_CHECK();
-  return 0;
+  return fmx_head_norm_gate(o, gate, g_stride, g_dtype, nullptr, out, out_stride, dtype, T, H, P, eps, 1, 0, nullptr, nullptr, stream);
 }

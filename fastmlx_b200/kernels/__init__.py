@@ -573,7 +573,7 @@ def delta_prepare(proj, ab, conv_w, a_log, dt_bias, ctx, state, conv_off, H, G, 
     call("common", "fmx_delta_prepare", proj.data_ptr(), proj.stride(0), ab.data_ptr(), ab.stride(0), conv_w.data_ptr(),
          a_log.data_ptr(), dt_bias.data_ptr(), ctx.token_row.data_ptr(), ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(),
          state.data_ptr(), state.stride(0), int(conv_off), qkv.data_ptr(), gb.data_ptr(), T, ctx.R, H, G, D, Dv, int(taps),
-         state.shape[0], _dt(proj), _ptr(ctx.status), _stream())
+         state.shape[0], _dt(proj), int(ctx.max_q_len == 1), _ptr(ctx.status), _stream())
     return qkv, gb
 
 
@@ -707,7 +707,7 @@ def ssm_prepare(proj, conv_w, conv_b, a_log, dt_bias, ctx, state, conv_off, H, G
     call("common", "fmx_ssm_prepare", proj.data_ptr(), proj.stride(0), conv_w.data_ptr(), conv_b.data_ptr(), a_log.data_ptr(),
          dt_bias.data_ptr(), ctx.token_row.data_ptr(), ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(), state.data_ptr(),
          state.stride(0), int(conv_off), xbc.data_ptr(), dd.data_ptr(), T, ctx.R, H, G, N, P, int(taps), state.shape[0],
-         _dt(proj), _ptr(ctx.status), _stream())
+         _dt(proj), int(ctx.max_q_len == 1), _ptr(ctx.status), _stream())
     return xbc, dd
 
 

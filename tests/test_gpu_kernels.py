@@ -899,3 +899,60 @@ def test_mixed_heads_on_tensor_cores(lens, ctxs, nh, nkv, hd, vd, page, window, 
     for r in range(R):
         if lens[r] < k().MIXED_TC_MIN_TOKENS:        # these rows run where they ran
             assert torch.equal(got[starts[r]:starts[r + 1]], fma[starts[r]:starts[r + 1]])
+
+
+@pytest.mark.parametrize("form", ["delta", "ssm", "channel"])
+@pytest.mark.parametrize("lens", [(1,), (1, 1, 1, 1, 1), (2, 1, 3), (5, 40, 1, 17), (700, 4, 3)])
+def test_convolutions_by_strips_of_tokens(form, lens):
+    """The kernels that walk strips of tokens with the last inputs in registers (four taps, channels in fours) beside those token by
+    token, which rows of an odd stride take: the same sums in the same order, unit vectors to their sums' rounding, the same slots;
+    a row of a captured step that is not there, rows shorter than the taps, strips that hold several rows."""
+    torch.manual_seed(len(lens))
+    H, G, D, P, taps = 12, 4, 64, 64, 4
+    starts = [0] + list(torch.tensor(lens).cumsum(0).tolist())
+    T, R = starts[-1] + 1, len(lens) + 1                               # the last row's slot is -1
+    starts.append(T)
+    single = max(lens) == 1
+    ctx = SimpleNamespace(R=R, max_q_len=max(lens), row_start=torch.tensor(starts, dtype=torch.int32, device=DEV), status=torch.zeros(4, dtype=torch.int32, device=DEV),
+                          token_row=torch.arange(R).repeat_interleave(torch.tensor(starts).diff()).int().to(DEV),
+                          row_slot=torch.tensor(list(range(R - 1))[::-1] + [-1], dtype=torch.int32, device=DEV))
+    C = 2 * G * D + H * P
+    width = {"delta": C + 8, "ssm": H * P + C + H, "channel": C + H}[form]
+    proj = torch.randn(T, width).bfloat16()
+    conv, cb, a_log, dtb = torch.randn(C, taps).to(DEV) * 0.5, torch.randn(C).to(DEV) * 0.1, torch.randn(H).to(DEV), torch.randn(H * D).to(DEV)
+    ab, z, off = torch.randn(T, 2 * H).to(DEV), torch.randn(T, H * D).to(DEV), H * P * D
+    state = torch.randn(R, off + (taps - 1) * C)
+
+    def run(odd):
+        x = torch.zeros(T, width + (1 if odd else (-width) % 4)).bfloat16().to(DEV)
+        x[:, :width] = proj.to(DEV)
+        s = state.to(DEV)
+        if form == "delta":
+            out = k().delta_prepare(x, ab, conv, a_log, dtb[:H], ctx, s, off, H, G, D, P, taps)
+        elif form == "ssm":
+            out = k().ssm_prepare(x, conv, cb, a_log, dtb[:H], ctx, s, off, H, G, D, P, taps)
+        else:
+            out = k().channel_delta_prepare(x, x[:, C:C + H], z, conv, a_log, dtb, ctx, s, off, H, G, D, P, taps)
+        return [t.cpu() for t in out], s.cpu()
+    (want, ws), (got, gs) = run(True), run(False)
+    assert ctx.status.tolist()[0] == 0 and single == (T == R)
+    unit = 0 if form == "ssm" else 2 * G * D
+    assert torch.equal(got[0][:, unit:], want[0][:, unit:]) and torch.equal(gs, ws)
+    assert (got[0][:, :unit] - want[0][:, :unit]).abs().max() <= 4e-7 if unit else True
+    assert (got[0][-1] == 0).all()
+    for g, w in zip(got[1:], want[1:]):
+        assert (g - w).abs().max() <= 2.0 ** -22 * w.abs().max()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n", [4, 36, 512, 516, 2048, 2052])
+def test_gated_group_rmsnorm_in_fours(n, dtype):
+    """Parts of at most 2,048 values in fours stay in registers; wider ones, and rows that do not start on fours, take the other kernel."""
+    T, groups = 5, 3
+    y, z, w = rnd(T, groups * n, dtype=torch.float32), rnd(T, groups * n + 3, dtype=dtype, seed=1), 1 + 0.1 * rnd(groups * n, dtype=torch.float32, seed=2)
+    zz = z[:, :groups * n]
+    got = k().gated_group_rmsnorm(y.to(DEV), zz.contiguous().to(DEV), w.to(DEV), 1e-6, groups, dtype)
+    odd = k().gated_group_rmsnorm(y.to(DEV), z.to(DEV)[:, :groups * n], w.to(DEV), 1e-6, groups, dtype)
+    want = plain_ops.gated_group_rmsnorm(y, zz, w, 1e-6, groups, torch.float64)
+    for o in (got, odd):
+        close(o, want, dtype, "gated_group_rmsnorm", scale=None)
