@@ -11,7 +11,7 @@
 // [nkv, page_size, vd] values.  Angles (position * inv_freq[j]), sines, cosines, the sum of
 // squares and the division are 32-bit; the sum of squares of a head is taken in an order that
 // depends on the head size alone.
-#include "common.cuh"
+#include "packed.cuh"
 
 namespace {
 constexpr int QKP_WARPS = 4;
@@ -222,6 +222,157 @@ qk_prepare_whole_kernel(const TI* qkv, long long row_stride, const int* position
     vdst[((long long)g * page_size + off) * vd + e] = from_f<T>((to_f(vsrc[it]) + (vbias != nullptr ? vbias[it] : 0.f)) * v_scale);
   }
 }
+// Both of them for head sizes of 32, 64 and 128 whose rotated pairs lie in fours: LG = hd / 4 lanes hold a head, four neighbouring
+// values each.  A rotation's partner values come by a shuffle of whole fours, a head's sum of squares by one over its lanes.
+// Bound by memory; the kernels above, a value a lane with every head through shared memory, are bound by their instructions.
+// 2,499 tokens of 32 + 8 + 8 heads of 64 values, half of each rotated: 66 -> 16 us; 1,531 tokens
+// normed whole, 32-bit in: 45 -> 15 us.
+template <typename TI, typename T, int LG>
+__global__ void __launch_bounds__(128)
+qk_prepare_vec_kernel(const TI* qkv, long long row_stride, const int* positions, const float* __restrict__ inv_freq,
+                      const long long* slot_mapping, float* q_out, T* kv, int nh, int nkv, int vd, int rot, int interleaved,
+                      float norm_eps, int page_size, long long num_pages, int* status, const float* __restrict__ bias,
+                      const float* __restrict__ q_weight, const float* __restrict__ k_weight, int norm_first, int whole,
+                      int values_from_keys, float amplitude, float v_scale, const TI* v_first, long long v_first_stride,
+                      const float* __restrict__ v_share) {
+  constexpr int hd = 4 * LG, GROUPS = 128 / LG;
+  __shared__ __align__(16) float sn[hd / 2], cs[hd / 2];
+  pdl_wait();
+  pdl_trigger();
+  const int t = blockIdx.x, grp = threadIdx.x / LG, sub = threadIdx.x % LG, e = 4 * sub;
+  const int half = rot / 2, heads = nh + nkv;
+  const TI* row = qkv + (long long)t * row_stride;
+  if ((int)threadIdx.x < half) {
+    float sj, cj;
+    sincosf((float)positions[t] * inv_freq[threadIdx.x], &sj, &cj);
+    sn[threadIdx.x] = sj * amplitude;
+    cs[threadIdx.x] = cj * amplitude;
+  }
+  long long slot = (kv != nullptr && slot_mapping != nullptr) ? slot_mapping[t] : -1;
+  if (slot >= num_pages * page_size) {
+    if (threadIdx.x == 0) fmx_set_status(status, FMX_BAD_SLOT, slot, t);
+    slot = -1;
+  }
+  const long long page = slot >= 0 ? slot / page_size : 0;
+  const int off = slot >= 0 ? (int)(slot - page * page_size) : 0;
+  T* keys = kv + page * ((long long)nkv * page_size * (hd + vd));
+  T* values = keys + (long long)nkv * page_size * hd;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
+  auto input = [&](int h) {
+    float4 v = load4(row + (long long)h * hd + e);
+    if (bias != nullptr) {
+      const float4 b = load4(bias + (long long)h * hd + e);
+      v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+    }
+    return v;
+  };
+  auto squares = [](float4 v) { return fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))); };
+  auto head_sum = [](float ss) {
+#pragma unroll
+    for (int d = LG / 2; d >= 1; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+    return ss;
+  };
+  auto times = [](float4 v, float m, float4 w) { return make_float4(v.x * m * w.x, v.y * m * w.y, v.z * m * w.z, v.w * m * w.w); };
+  const bool normed = norm_eps >= 0.f;
+  float mq = 1.f, mk = 1.f;
+  if (whole && normed) {                       // the whole projection's root mean squares (the grid has one block per token)
+    float sq = 0.f, sk = 0.f;
+    for (int h = grp; h < heads; h += GROUPS) {
+      const float s = squares(input(h));
+      if (h < nh) sq += s;
+      else sk += s;
+    }
+    mq = 1.0f / sqrtf(block_sum<128>(sq) / (float)(nh * hd) + norm_eps);
+    const float all = block_sum<128>(sk);
+    if (nkv > 0) mk = 1.0f / sqrtf(all / (float)(nkv * hd) + norm_eps);
+  }
+  __syncthreads();                             // sines and cosines are there
+  for (int h0 = blockIdx.y * GROUPS; h0 < heads; h0 += GROUPS * gridDim.y) {
+    const int h = h0 + grp;
+    const bool live = h < heads;               // (every lane takes part in the exchanges)
+    float4 v = live ? input(h) : zero;
+    const float* hw = h < nh ? q_weight : k_weight;
+    const float4 w = live && hw != nullptr ? load4(hw + (whole ? (long long)(h < nh ? h : h - nh) * hd : 0) + e) : one;
+    if (live && h >= nh && slot >= 0 && values_from_keys)          // the value: the key as it was projected
+      store4(values + ((long long)(h - nh) * page_size + off) * vd + e, make_float4(v.x * v_scale, v.y * v_scale, v.z * v_scale, v.w * v_scale));
+    if (whole) v = times(v, h < nh ? mq : mk, w);
+    else if (norm_first && normed) v = times(v, 1.0f / sqrtf(head_sum(squares(v)) / (float)hd + norm_eps), w);
+    if (rot > 0 && interleaved) {
+      if (e < rot) {
+        float4 r;
+        rope_pair(v.x, v.y, sn[e / 2], cs[e / 2], r.x, r.y);
+        rope_pair(v.z, v.w, sn[e / 2 + 1], cs[e / 2 + 1], r.z, r.w);
+        v = r;
+      }
+    } else if (rot > 0) {
+      const bool first = e < half;
+      const int from = e >= rot ? sub : first ? sub + half / 4 : sub - half / 4, j = e >= rot ? 0 : first ? e : e - half;
+      const float4 o = make_float4(__shfl_sync(0xffffffffu, v.x, from, LG), __shfl_sync(0xffffffffu, v.y, from, LG),
+                                   __shfl_sync(0xffffffffu, v.z, from, LG), __shfl_sync(0xffffffffu, v.w, from, LG));
+      if (e < rot) {
+        const float4 s4 = load4(sn + j), c4 = load4(cs + j);
+        float x, y;
+        float4 r;
+        auto turn = [&](float own, float other, float sj, float cj) {
+          if (first) rope_pair(own, other, sj, cj, x, y);
+          else rope_pair(other, own, sj, cj, y, x);                // x: this element's new value in either case
+          return x;
+        };
+        r.x = turn(v.x, o.x, s4.x, c4.x);
+        r.y = turn(v.y, o.y, s4.y, c4.y);
+        r.z = turn(v.z, o.z, s4.z, c4.z);
+        r.w = turn(v.w, o.w, s4.w, c4.w);
+        v = r;
+      }
+    }
+    if (!whole && !norm_first && normed) v = times(v, 1.0f / sqrtf(head_sum(squares(v)) / (float)hd + norm_eps), w);
+    if (!live) continue;
+    if (h < nh) store4(q_out + ((long long)t * nh + h) * hd + e, v);
+    else if (slot >= 0) store4(keys + ((long long)(h - nh) * page_size + off) * hd + e, v);
+  }
+  if (slot < 0 || blockIdx.y != 0 || values_from_keys) return;
+  const TI* vsrc = row + (long long)heads * hd;
+  const float share = v_share != nullptr ? v_share[0] : 0.f;
+  for (int it = threadIdx.x * 4; it < nkv * vd; it += 512) {
+    const int g = it / vd, d = it - g * vd;
+    float4 v = load4(vsrc + it);
+    const float4 b = bias != nullptr ? load4(bias + (long long)heads * hd + it) : zero;
+    v = make_float4((v.x + b.x) * v_scale, (v.y + b.y) * v_scale, (v.z + b.z) * v_scale, (v.w + b.w) * v_scale);
+    if (v_first != nullptr) {
+      const float4 f = load4(v_first + (long long)t * v_first_stride + it);
+      v = make_float4((1.0f - share) * v.x + share * f.x, (1.0f - share) * v.y + share * f.y, (1.0f - share) * v.z + share * f.z,
+                      (1.0f - share) * v.w + share * f.w);
+    }
+    store4(values + ((long long)g * page_size + off) * vd + d, v);
+  }
+}
+
+// Do head and row sizes and addresses let a lane take four values at a time?
+template <typename TI, typename T>
+bool qk_vec_takes(const void* qkv, long long row_stride, const float* q_out, const void* kv, int hd, int vd, int rot, int interleaved,
+                  const float* bias, const float* q_weight, const float* k_weight, const void* v_first, long long v_first_stride) {
+  auto at = [](const void* p, size_t bytes) { return ((uintptr_t)p & (bytes - 1)) == 0; };
+  return (hd == 32 || hd == 64 || hd == 128) && vd % 4 == 0 && rot % (interleaved ? 4 : 8) == 0 && row_stride % 4 == 0 && v_first_stride % 4 == 0 &&
+         at(qkv, 4 * sizeof(TI)) && at(v_first, 4 * sizeof(TI)) && at(kv, 4 * sizeof(T)) && at(q_out, 16) && at(bias, 16) && at(q_weight, 16) &&
+         at(k_weight, 16);
+}
+template <typename TI, typename T>
+void qk_vec_launch(const void* qkv, long long row_stride, const int* positions, const float* inv_freq, const long long* slot_mapping, float* q_out,
+                   void* kv, int tokens, int nh, int nkv, int hd, int vd, int rot, int interleaved, float norm_eps, int page_size, long long num_pages,
+                   int* status, const float* bias, const float* q_weight, const float* k_weight, int norm_first, int whole, int values_from_keys,
+                   float amplitude, float v_scale, const void* v_first, long long v_first_stride, const float* v_share, cudaStream_t stream) {
+  // few tokens: blocks share a token's heads out, so that they are not walked one after another
+  const int groups = 512 / hd, passes = (nh + nkv + groups - 1) / groups;
+  const dim3 grid(tokens, whole || passes < 1 ? 1 : tokens <= 256 ? passes : (passes + 2) / 3);
+#define FMX_QKV(LG)                                                                                                        \
+  fmx_launch(qk_prepare_vec_kernel<TI, T, LG>, grid, dim3(128), 0, stream, (const TI*)qkv, row_stride, positions, inv_freq, \
+             slot_mapping, q_out, (T*)kv, nh, nkv, vd, rot, interleaved, norm_eps, page_size, num_pages, status, bias,     \
+             q_weight, k_weight, norm_first, whole, values_from_keys, amplitude, v_scale, (const TI*)v_first, v_first_stride, v_share)
+  if (hd == 32) FMX_QKV(8);
+  else if (hd == 64) FMX_QKV(16);
+  else FMX_QKV(32);
+#undef FMX_QKV
+}
 }  // namespace
 
 // rot = 0: nothing is rotated; norm_eps < 0: heads are not normalised; kv or slot_mapping null:
@@ -248,16 +399,20 @@ FMX_EXPORT int fmx_qk_prepare_mix(const void* qkv, long long row_stride, const i
   const int passes = (nh + nkv + QKP_WARPS - 1) / QKP_WARPS;
   const int head_blocks = passes < 1 ? 1 : T <= 256 ? passes : (passes + 2) / 3;
 #define FMX_QKP(TI, TKV)                                                                                                  \
-  fmx_launch(qk_prepare_kernel<TI, TKV>, dim3(T, head_blocks), dim3(QKP_WARPS * 32), smem, stream, (const TI*)qkv, row_stride, positions, \
+  if (qk_vec_takes<TI, TKV>(qkv, row_stride, q_out, kv, hd, vd, rot, interleaved, bias, q_weight, k_weight, v_first, v_first_stride)) \
+    qk_vec_launch<TI, TKV>(qkv, row_stride, positions, inv_freq, slot_mapping, q_out, kv, T, nh, nkv, hd, vd, rot, interleaved, norm_eps, \
+                           page_size, num_pages, status, bias, q_weight, k_weight, norm_first, 0, 0, amplitude, v_scale, v_first, \
+                           v_first_stride, v_share, stream);                                                              \
+  else fmx_launch(qk_prepare_kernel<TI, TKV>, dim3(T, head_blocks), dim3(QKP_WARPS * 32), smem, stream, (const TI*)qkv, row_stride, positions, \
              inv_freq, slot_mapping, q_out, (TKV*)kv, nh, nkv, hd, vd, rot, interleaved, norm_eps, page_size, num_pages,  \
              status, bias, q_weight, k_weight, norm_first, amplitude, v_scale, (const TI*)v_first, v_first_stride, v_share)
-  if (in_dtype == FMX_F32 && dtype == FMX_F32)
+  if (in_dtype == FMX_F32 && dtype == FMX_F32) {
     FMX_QKP(float, float);
-  else if (in_dtype == FMX_BF16 && dtype == FMX_BF16)
+  } else if (in_dtype == FMX_BF16 && dtype == FMX_BF16) {
     FMX_QKP(bf16, bf16);
-  else if (in_dtype == FMX_F32 && dtype == FMX_BF16)
+  } else if (in_dtype == FMX_F32 && dtype == FMX_BF16) {
     FMX_QKP(float, bf16);
-  else
+  } else
     return fmx_fail("fmx_qk_prepare: no kernel for an input of type %d and a cache of type %d", in_dtype, dtype);
 #undef FMX_QKP
   FMX_LAUNCH_CHECK();
@@ -298,16 +453,20 @@ FMX_EXPORT int fmx_qk_prepare_whole(const void* qkv, long long row_stride, const
     return fmx_fail("fmx_qk_prepare_whole: row stride too small");
   const size_t smem = ((size_t)rot + (size_t)QKP_WARPS * hd) * sizeof(float);
 #define FMX_QKW(TI, TKV)                                                                                                 \
-  fmx_launch(qk_prepare_whole_kernel<TI, TKV>, dim3(T), dim3(QKP_WARPS * 32), smem, stream, (const TI*)qkv, row_stride,  \
+  if (qk_vec_takes<TI, TKV>(qkv, row_stride, q_out, kv, hd, vd, rot, interleaved, bias, q_weight, k_weight, nullptr, 0)) \
+    qk_vec_launch<TI, TKV>(qkv, row_stride, positions, inv_freq, slot_mapping, q_out, kv, T, nh, nkv, hd, vd, rot, interleaved, norm_eps, \
+                           page_size, num_pages, status, bias, q_weight, k_weight, 1, 1, values_from_keys, amplitude, v_scale, nullptr, 0, \
+                           nullptr, stream);                                                                             \
+  else fmx_launch(qk_prepare_whole_kernel<TI, TKV>, dim3(T), dim3(QKP_WARPS * 32), smem, stream, (const TI*)qkv, row_stride,  \
              positions, inv_freq, slot_mapping, q_out, (TKV*)kv, nh, nkv, hd, vd, rot, interleaved, norm_eps, page_size, \
              num_pages, status, bias, q_weight, k_weight, values_from_keys, amplitude, v_scale)
-  if (in_dtype == FMX_F32 && dtype == FMX_F32)
+  if (in_dtype == FMX_F32 && dtype == FMX_F32) {
     FMX_QKW(float, float);
-  else if (in_dtype == FMX_BF16 && dtype == FMX_BF16)
+  } else if (in_dtype == FMX_BF16 && dtype == FMX_BF16) {
     FMX_QKW(bf16, bf16);
-  else if (in_dtype == FMX_F32 && dtype == FMX_BF16)
+  } else if (in_dtype == FMX_F32 && dtype == FMX_BF16) {
     FMX_QKW(float, bf16);
-  else
+  } else
     return fmx_fail("fmx_qk_prepare_whole: no kernel for an input of type %d and a cache of type %d", in_dtype, dtype);
 #undef FMX_QKW
   FMX_LAUNCH_CHECK();

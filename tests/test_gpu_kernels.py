@@ -956,3 +956,41 @@ def test_gated_group_rmsnorm_in_fours(n, dtype):
     want = plain_ops.gated_group_rmsnorm(y, zz, w, 1e-6, groups, torch.float64)
     for o in (got, odd):
         close(o, want, dtype, "gated_group_rmsnorm", scale=None)
+
+
+@pytest.mark.parametrize("tin,tkv", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("hd,vd,rot,inter,form", [(64, 64, 64, False, "last"), (64, 64, 32, False, "first"), (128, 64, 128, True, "first"),
+                                                 (32, 96, 16, False, "none"), (128, 128, 64, False, "whole"), (64, 64, 0, False, "whole keys"),
+                                                 (64, 32, 12, True, "last")])
+def test_queries_and_keys_in_fours(tin, tkv, hd, vd, rot, inter, form):
+    """Queries and keys made ready four values a lane beside the kernels of one value a lane, which rows that do not start on fours
+    take: both orders of norm and rotation, norms over the whole projection, values that are the keys, biases, mixed values, partial
+    and interleaved rotations, tokens that are stored nowhere."""
+    torch.manual_seed(hd + rot)
+    T, nh, nkv, page = 7, 6, 3, 4
+    from_keys = form == "whole keys"
+    width = (nh + nkv) * hd + (0 if from_keys else nkv * vd)
+    row = torch.randn(T, width).to(tin)
+    slots = torch.tensor([5, 0, 11, -1, 7, 2, 3], device=DEV)
+    pos, freq = torch.tensor([0, 3, 900, 17, 4, 1, 8191], dtype=torch.int32, device=DEV), (torch.rand(rot // 2) if rot else torch.zeros(1)).to(DEV)
+    whole = form.startswith("whole")
+    bias = torch.randn(width).to(DEV) if form in ("first", "whole") else None
+    wq, wk = torch.rand(nh * hd if whole else hd).to(DEV) + 0.5, torch.rand(nkv * hd if whole else hd).to(DEV) + 0.5
+    first, share = torch.randn(T, nkv * vd).to(tin).to(DEV), torch.tensor([0.3], device=DEV)
+
+    def run(odd):
+        x = torch.zeros(T, width + (1 if odd else (-width) % 4)).to(tin).to(DEV)
+        x[:, :width] = row.to(DEV)
+        kv = torch.zeros(3, nkv * page * (hd + vd), device=DEV).to(tkv)
+        status = torch.zeros(4, dtype=torch.int32, device=DEV)
+        more = dict(v_first=first, v_share=share) if form == "last" else {}
+        q = k().qk_prepare(x, pos, freq, rot, inter, None if form == "none" else 1e-6, slots, kv, nh, nkv, hd, vd, status, bias=bias,
+                           q_weight=None if form == "none" else wq, k_weight=None if form == "none" else wk,
+                           norm_first=form == "first" or whole, whole=whole, values_from_keys=from_keys, amplitude=1.25, v_scale=0.5, **more)
+        return q.cpu(), kv.cpu(), status.tolist()[0]
+    (q1, kv1, st1), (q2, kv2, st2) = run(True), run(False)
+    assert st1 == st2 == 0
+    assert (q1 - q2).abs().max() <= 2.0 ** -21 * q1.abs().max()          # the norms' sums in another order
+    assert (kv1.float() - kv2.float()).abs().max() <= (2.0 ** -21 if tkv == torch.float32 else 2.0 ** -7) * kv1.float().abs().max()
+    if tkv == torch.bfloat16:
+        assert (kv1 != kv2).float().mean() < 2e-3
