@@ -234,7 +234,7 @@ channel_gla_prepare_vec_kernel(const T* proj, long long stride, const float* z, 
 template <bool DELTA, int RPL, int L, int CPT, int GT, int TB>
 __global__ void __launch_bounds__(128)
 channel_scan_kernel(const float* qkv, const float* decay, const float* beta, const int* row_start, const int* row_slot,
-                    float* state, long long slot_stride, float* out, int H, int G, int D, int Dv, int max_slots) {
+                    float* state, long long slot_stride, float* out, int H, int G, int D, int Dv, int max_slots, int max_tokens) {
   constexpr int COLS = 128 / L * CPT, DP = RPL * L, NP = RPL / 2, NV = GT * CPT;
   constexpr int ROWF = 3 * DP + COLS + 4;         // floats of one token: k | q | g | values | beta, 3 key dot products
   static_assert(NV <= L && TB % GT == 0 && COLS % 4 == 0, "sizes");
@@ -252,6 +252,7 @@ channel_scan_kernel(const float* qkv, const float* decay, const float* beta, con
   const int slot = row_slot[r];
   if (slot < 0 || slot >= max_slots) return;
   const int first = row_start[r], n = row_start[r + 1] - first;
+  if (n > max_tokens) return;                     // a row for the kernels that walk runs of tokens
   const int C = 2 * G * D + H * Dv;
   const int g = h / (H / G);
   float* sp[CPT];
@@ -573,7 +574,7 @@ FMX_EXPORT int fmx_channel_gla_prepare(const void* proj, long long stride, const
 // share a column, cpt (1, 2, 4): columns that they hold; 0: the choice is made here.
 FMX_EXPORT int fmx_channel_scan(const float* qkv, const float* decay, const float* beta, const int* row_start,
                                 const int* row_slot, float* state, long long slot_stride, float* out, int R, int H, int G, int D,
-                                int Dv, int max_slots, int single, int lanes, int cpt, cudaStream_t stream) {
+                                int Dv, int max_slots, int single, int lanes, int cpt, int max_tokens, cudaStream_t stream) {
   if (R == 0) return 0;
   if (R < 0 || H <= 0 || G <= 0 || H % G || D <= 0 || Dv <= 0 || D > 512)
     return fmx_fail("fmx_channel_scan: bad sizes R=%d H=%d G=%d D=%d Dv=%d", R, H, G, D, Dv);
@@ -605,7 +606,7 @@ FMX_EXPORT int fmx_channel_scan(const float* qkv, const float* decay, const floa
     if (smem > 48 * 1024)                                                                                              \
       cudaFuncSetAttribute(channel_scan_kernel<DELTA, RPL, L, CPT, GT, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
     fmx_launch(channel_scan_kernel<DELTA, RPL, L, CPT, GT, TB>, dim3((Dv + cols - 1) / cols, H, R), dim3(128), smem, stream, qkv, \
-               decay, beta, row_start, row_slot, state, slot_stride, out, H, G, D, Dv, max_slots);                     \
+               decay, beta, row_start, row_slot, state, slot_stride, out, H, G, D, Dv, max_slots, max_tokens);                     \
   } while (0)
 #define FMX_CS_G(RPL, L, CPT, TB)                                                                                      \
   do {                                                                                                                 \

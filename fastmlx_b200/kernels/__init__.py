@@ -918,7 +918,35 @@ def channel_scan(qkv, g, beta, ctx, state, H, G, D, Dv, lanes: int = 0, cpt: int
     out = torch.empty((T, H * Dv), dtype=torch.float32, device=qkv.device)
     call("chan", "fmx_channel_scan", qkv.data_ptr(), g.data_ptr(), _ptr(beta), ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(),
          state.data_ptr(), state.stride(0), out.data_ptr(), ctx.R, H, G, D, Dv, state.shape[0], int(ctx.max_q_len == 1), int(lanes), int(cpt),
-         _stream())
+         WALK_ANY, _stream())
+    return out
+
+
+def channel_chunks_least(D: int, delta: bool) -> int:
+    """Rows of at least so many tokens go in runs of 32 as matrix products, shorter ones token by token.  With the delta rule, alone:
+    64 rows of state 64 tokens 16 us walked and 18 in runs, 128 tokens 28 and 23; 128 rows of state 32 tokens 17 and 25, 64 tokens 29
+    and 28.  Without it the walk has half the steps: 64 rows of state 128 tokens 20 and 19 us, 256 tokens 36 and 25."""
+    return 8192 // D if delta else 256
+
+
+def channel_scan_takes(ctx, D: int, Dv: int, delta: bool) -> bool:
+    """`chunk_scan_takes` for decays by key channel (`channel_scan_chunks`).  Without the delta rule 64 rows of state alone: 2,048 tokens
+    of 32 heads 262 us walked and 198 in runs, with 128 rows of state 308 either way."""
+    return D in ((64, 128) if delta else (64,)) and Dv % 16 == 0 and ctx.max_q_len >= channel_chunks_least(D, delta)
+
+
+def channel_scan_chunks(qkv, g, beta, ctx, state, H, G, D, Dv) -> torch.Tensor:
+    """`channel_scan` with the step's portions in runs of 32 tokens as matrix products (see `channel_scan_takes`)."""
+    _need_cuda(qkv, g, beta, state)
+    assert qkv.is_contiguous() and g.is_contiguous() and (beta is None or beta.is_contiguous())
+    T, least = qkv.shape[0], channel_chunks_least(D, beta is not None)
+    out = torch.empty((T, H * Dv), dtype=torch.float32, device=qkv.device)
+    ws = torch.empty(int(load("chunks").fmx_channel_chunks_bytes(T, ctx.R, H, D, int(beta is not None))), dtype=torch.uint8, device=qkv.device)
+    if _has_short_rows(ctx, least):
+        call("chan", "fmx_channel_scan", qkv.data_ptr(), g.data_ptr(), _ptr(beta), ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(),
+             state.data_ptr(), state.stride(0), out.data_ptr(), ctx.R, H, G, D, Dv, state.shape[0], 0, 0, 0, least - 1, _stream())
+    call("chunks", "fmx_channel_chunks", qkv.data_ptr(), g.data_ptr(), _ptr(beta), ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(),
+         state.data_ptr(), state.stride(0), out.data_ptr(), ws.data_ptr(), ws.numel(), T, ctx.R, H, G, D, Dv, state.shape[0], least, _stream())
     return out
 
 

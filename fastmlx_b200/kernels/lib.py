@@ -98,7 +98,7 @@ _SIGNATURES = {
         "fmx_channel_delta_prepare": [_P, _L, _P, _L, _P, _L, _P, _P, _P, _P, _P, _P, _P, _L, _L, _P, _P, _P, _I, _I, _I, _I, _I,
                                       _I, _I, _I, _I, _I, _P, _P],
         "fmx_channel_gla_prepare": [_P, _L, _P, _L, _P, _P, _P, _I, _I, _I, _I, _F, _F, _I, _P],
-        "fmx_channel_scan": [_P, _P, _P, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
+        "fmx_channel_scan": [_P, _P, _P, _P, _P, _P, _L, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     },
     "mlstm": {
         "fmx_mlstm_gates": [_P, _L, _P, _F, _P, _P, _P, _L, _L, _P, _I, _I, _I, _I, _P],
@@ -110,6 +110,7 @@ _SIGNATURES = {
         "fmx_mixattn_tc": [_P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _L, _F, _F, _I, _I, _P, _P, _I, _I, _P, _P],
         "fmx_mixattn_tc_plan": [_I, _I, _I, _I, _I, _I, _I, _I],
         "fmx_chunk_delta_rule": [_P, _P, _P, _P, _P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
+        "fmx_channel_chunks": [_P, _P, _P, _P, _P, _P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _P],
         "fmx_chunk_ssm_scan": [_P, _P, _P, _P, _P, _P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     },
     "mixattn": {
@@ -165,6 +166,8 @@ def load(group: str) -> ctypes.CDLL:
     if group == "chunks":
         lib.fmx_chunk_scan_bytes.argtypes = [_I, _I, _I, _I, _I, _I]
         lib.fmx_chunk_scan_bytes.restype = c_longlong
+        lib.fmx_channel_chunks_bytes.argtypes = [_I, _I, _I, _I, _I]
+        lib.fmx_channel_chunks_bytes.restype = c_longlong
     lib.fmx_last_error.restype = ctypes.c_char_p
     family = "attn_vd" if values_differ else "attn" if group.startswith("attn_hd") else "tc" if group == "tc_expiry" else \
         "mixattn" if group.startswith("mixattn_v") else group

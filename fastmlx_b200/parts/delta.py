@@ -173,7 +173,9 @@ class ChannelDeltaMixer(Mixer):
         qkv, g, beta = k.channel_delta_prepare(proj, proj[:, c + r:c + r + self.H], zg[:, :n], self.conv_w, self.a_log,
                                                self.dt_bias, ctx, cache.state, self.s_floats, self.H, self.G, self.D, self.Dv,
                                                self.taps)
-        o = k.channel_scan(qkv, g, beta, ctx, cache.state, self.H, self.G, self.D, self.Dv)
+        takes = getattr(k, "channel_scan_takes", None) if self.rt.dtype == torch.bfloat16 else None
+        scan = k.channel_scan_chunks if takes is not None and takes(ctx, self.D, self.Dv, True) else k.channel_scan
+        o = scan(qkv, g, beta, ctx, cache.state, self.H, self.G, self.D, self.Dv)
         return k.head_norm_gate(o, zg[:, n:], self.norm_w, self.eps, self.H, self.Dv, self.rt.dtype, "sigmoid", out=out)
 
     def forward(self, x, ctx, cache):

@@ -994,3 +994,55 @@ def test_queries_and_keys_in_fours(tin, tkv, hd, vd, rot, inter, form):
     assert (kv1.float() - kv2.float()).abs().max() <= (2.0 ** -21 if tkv == torch.float32 else 2.0 ** -7) * kv1.float().abs().max()
     if tkv == torch.bfloat16:
         assert (kv1 != kv2).float().mean() < 2e-3
+@pytest.mark.parametrize("delta,lens,H,G,D,P", [
+    (True, (128,), 4, 2, 64, 64), (True, (129, 1, 161, 127, 192), 4, 2, 64, 48), (True, (64, 65, 63), 4, 1, 128, 128), (True, (31, 128), 2, 2, 128, 16),
+    (True, (3, 72, 96), 32, 8, 128, 96), (False, (256,), 3, 3, 64, 64), (False, (257, 5, 255, 300), 4, 4, 64, 48), (False, (1, 288), 32, 32, 64, 32)])
+def test_channel_decays_in_runs_of_tokens(delta, lens, H, G, D, P):
+    """The kernels that walk runs of 32 tokens whose state decays by key channel, against 64-bit arithmetic and beside the walk token
+    by token: decays that are zero, that vanish within a run and that are nearly one, portions of whole runs and a token more or
+    less, rows too short for runs, a workspace that holds a few runs only."""
+    torch.manual_seed(D + len(lens))
+    starts, R = [0] + list(torch.tensor(lens).cumsum(0).tolist()), len(lens)
+    T, order = starts[-1], list(range(R))[::-1]
+    ctx = SimpleNamespace(R=R, row_start=torch.tensor(starts, dtype=torch.int32, device=DEV), max_q_len=max(lens), h_row_start=starts,
+                          row_slot=torch.tensor(order, dtype=torch.int32, device=DEV))
+    unit = lambda *s: torch.nn.functional.normalize(torch.randn(*s) + 0.2, dim=-1)
+    q, kk, v, beta = unit(T, G, D), unit(T, G, D), torch.randn(T, H, P), torch.rand(T, H)
+    decay = torch.rand(T, H, D) ** (torch.rand(H, D) * 3)
+    decay[torch.rand(T, H, D) < 0.02] = 0.0
+    decay[:, 0, ::2] = 1.0 - 1e-3 * torch.rand(T, (D + 1) // 2)
+    decay[:, -1, 1::4] = 1e-6
+    x, state = torch.cat([q.flatten(1), kk.flatten(1), v.flatten(1)], 1).to(DEV), torch.randn(R, H * P * D + 12)
+    g, b = decay.flatten(1).to(DEV), beta.to(DEV) if delta else None
+    assert k().channel_scan_takes(ctx, D, P, delta) and not k().channel_scan_takes(ctx, 128, P, False)
+    s1, s2, s3 = state.to(DEV), state.to(DEV), state.to(DEV)
+    o1 = k().channel_scan(x, g, b, ctx, s1, H, G, D, P).cpu().double().view(T, H, P)
+    o2 = k().channel_scan_chunks(x, g, b, ctx, s2, H, G, D, P).cpu().double().view(T, H, P)
+    out, one = torch.zeros(T, H * P, device=DEV), int(k().load("chunks").fmx_channel_chunks_bytes(1, 1, H, D, int(delta)))
+    ws = torch.empty(2 * one, dtype=torch.uint8, device=DEV)              # two runs at a time
+    k().call("chunks", "fmx_channel_chunks", x.data_ptr(), g.data_ptr(), k()._ptr(b), ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(), s3.data_ptr(),
+             s3.stride(0), out.data_ptr(), ws.data_ptr(), ws.numel(), T, R, H, G, D, P, R, k().channel_chunks_least(D, delta), k()._stream())
+    f = lambda t: t.double().repeat_interleave(H // G, 1)
+    qd, kd, want, left = f(q), f(kk), torch.empty(T, H, P, dtype=torch.float64), state.double().clone()
+    for r in range(R):
+        S = left[order[r], :H * P * D].view(H, P, D)
+        for t in range(starts[r], starts[r + 1]):
+            S = S * decay[t].double()[:, None, :]
+            u = v[t].double()
+            if delta:
+                u = beta[t].double()[:, None] * (u - torch.einsum("hpd,hd->hp", S, kd[t]))
+            S = S + u[:, :, None] * kd[t][:, None, :]
+            want[t] = torch.einsum("hpd,hd->hp", S, qd[t])
+        left[order[r], :H * P * D] = S.flatten()
+    # roundings of 2^-24 of the largest value a sum meets, some dozens of which meet in a value at random signs
+    for got, ref in ((o2, want), (s2[:, :H * P * D].cpu().double(), left[:, :H * P * D])):
+        assert (got - ref).abs().max() < 40 * 2.0 ** -24 * ref.abs().max()
+    err = lambda o: ((o - want).norm() / want.norm()).item()
+    assert err(o2) < 1.5 * err(o1) + 2e-8
+    assert torch.equal(s2[:, H * P * D:].cpu(), state[:, H * P * D:])
+    for r in range(R):
+        at = slice(starts[r], starts[r + 1])
+        if lens[r] < k().channel_chunks_least(D, delta):        # walked: the same bits; and left alone by the kernel for runs
+            assert torch.equal(o1[at], o2[at]) and (out[at] == 0).all() and torch.equal(s3[order[r]].cpu(), state[order[r]])
+        else:                                        # in waves of two runs the same bits as in one
+            assert torch.equal(out[at].cpu().double().view(-1, H, P), o2[at]) and torch.equal(s3[order[r]], s2[order[r]])
