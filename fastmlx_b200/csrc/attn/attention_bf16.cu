@@ -34,6 +34,7 @@
 #include <math.h>
 #include <type_traits>
 #include "common.cuh"
+#include "tanh_small.cuh"
 
 #ifndef FMX_HD
 #error "compile with -DFMX_HD=<head size>"
@@ -380,6 +381,29 @@ __device__ __forceinline__ void softmax_step(float (&s)[NT][4], float (&m)[2], f
                                              float scale_cap = 0.f, int keep = 0) {
   const int t = threadIdx.x & 3;
   float mx[2] = {-INFINITY, -INFINITY};
+  // Capped before the mask, all scores together, without a branch in each (see tanh_small.cuh): 2,499 tokens of three portions
+  // behind 700, window 1,024, 32 heads of 64 values 200 -> 178 us.
+  if (CAP) {
+    bool large = false;
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        s[j][e] *= scale_cap;
+        large |= !(fabsf(s[j][e]) <= TANH_SMALL);
+      }
+    if (__any_sync(0xffffffffu, large)) {
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[j][e] = cap_l2 * tanhf(s[j][e]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[j][e] = cap_l2 * tanh_small(s[j][e]);
+    }
+  }
 #pragma unroll
   for (int j = 0; j < NT; ++j)
 #pragma unroll
@@ -387,10 +411,7 @@ __device__ __forceinline__ void softmax_step(float (&s)[NT][4], float (&m)[2], f
       const int x = e >> 1;
       const int key = key0 + 8 * j + 2 * t + (e & 1);
       float v = -INFINITY;
-      if (!MASK || (key <= lim[x] && (key >= lo[x] || key < keep))) {      // the cap is worked out for visible scores only
-        if (CAP) v = cap_l2 * tanhf(s[j][e] * scale_cap);
-        else v = s[j][e] * sl2;
-      }
+      if (!MASK || (key <= lim[x] && (key >= lo[x] || key < keep))) v = CAP ? s[j][e] : s[j][e] * sl2;
       s[j][e] = v;
       mx[x] = fmaxf(mx[x], v);
     }

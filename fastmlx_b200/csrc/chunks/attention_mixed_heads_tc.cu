@@ -23,6 +23,7 @@
 // 64 tokens behind 2,000: 595 and 48 us.  Values that are not the bfloat16 nearest to 64-bit arithmetic's: 4.0e-4 and 1.7e-4.
 #include <math.h>
 #include "split_mma.cuh"
+#include "tanh_small.cuh"
 
 namespace {
 constexpr int TQ = 8, TK = 32, KVH = 8, PER = 4, HEADS = KVH * PER;      // at most KVH key heads of PER query heads
@@ -39,19 +40,7 @@ __device__ __forceinline__ void ldmatrix4_trans(unsigned (&r)[4], const bf16* p)
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
 }
 
-// cap(s) = c tanh(s / c).  Lambert's continued fraction for the tangent, cut after five levels, for |y| <= 0.8:
-//     tanh y = y - y a (315 + 14 a) / (945 + 420 a + 15 a^2),   a = y^2,
-// off by y^10 / 9.8e6 at most (1.1e-8 at 0.8), and no branch: sixteen of a thread's scores run side by side, where the
-// library's function, with its branch in each, took 220 cycles a score.  Larger arguments take the library's function,
-// all of a warp's scores together.
-constexpr float TANH_SMALL = 0.8f;
-__device__ __forceinline__ float rcp_approx(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 __device__ __forceinline__ float ex2_approx(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
-__device__ __forceinline__ float tanh_small(float y) {
-  const float a = y * y;
-  const float c = a * fmaf(a, 14.f, 315.f) * rcp_approx(fmaf(a, fmaf(a, 15.f, 420.f), 945.f));
-  return fmaf(-y, c, y);
-}
 
 // Places for the rows' tiles of 8 tokens: row r's first is row_start / 8 + r; rows do not overlap, whatever their lengths.
 __global__ void __launch_bounds__(THREADS, 1)
