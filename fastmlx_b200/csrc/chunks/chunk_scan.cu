@@ -42,11 +42,14 @@ __device__ __forceinline__ int first_run(int row_start, int r) { return row_star
 
 // x [T, C]: q of group g at qoff + g D, k at koff + g D.  decay, weight: per token and head, rows of gstride.
 // qk [run][G][q, k][3][32][D], pt [run][H][P, T (delta rule)][3][32][32] and floats [A_t: 32, E_s: 32].
+// Warps of a block: a block of 128 rows fills a third of an SM's shared memory, and with eight warps its phases are half as long
+// (1,777 tokens, 8 groups of 8 heads: 38 -> 31 us); of 64 rows five blocks of four warps share an SM (34 and 34 us).
+template <int D> constexpr int PREP_WARPS = D > 64 ? 8 : 4;
 template <int D, bool DELTA>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(32 * PREP_WARPS<D>)
 chunk_prepare_kernel(const float* x, long long C, int qoff, int koff, const float* decay, const float* weight, int gstride,
                      const int* row_start, int min_tokens, int H, int G, bf16* qk, bf16* pt) {
-  constexpr int LD = D + 4;
+  constexpr int LD = D + 4, THREADS = 32 * PREP_WARPS<D>;
   extern __shared__ __align__(16) float psm[];
   float* qs = psm;                              // [32][LD]
   float* ks = qs + RUN * LD;
@@ -61,7 +64,7 @@ chunk_prepare_kernel(const float* x, long long C, int qoff, int koff, const floa
   const int t0 = first + c * RUN, cnt = min(RUN, n - c * RUN);
   const long long run = first_run(first, r) + c;
   bf16* planes = qk + (run * G + g) * QK_SIZE<D>;
-  for (int e = tid; e < 2 * RUN * (D / 4); e += 128) {
+  for (int e = tid; e < 2 * RUN * (D / 4); e += THREADS) {
     const int which = e / (RUN * (D / 4)), row = e / (D / 4) % RUN, d = e % (D / 4) * 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (row < cnt) v = load4(x + (long long)(t0 + row) * C + (which ? koff : qoff) + g * D + d);
@@ -75,38 +78,39 @@ chunk_prepare_kernel(const float* x, long long C, int qoff, int koff, const floa
   }
   __syncthreads();
   {
-    const int t = tid >> 2, s0 = tid & 3;       // a thread's eight columns s0, s0 + 4, ...: neighbours read neighbouring rows
-    float tq[RUN / 4], tk[RUN / 4];
+    constexpr int PER = THREADS / RUN, NC = RUN / PER;       // a thread's columns: s0, s0 + PER, ...; neighbours read neighbouring rows
+    const int t = tid / PER, s0 = tid % PER;
+    float tq[NC], tk[NC];
 #pragma unroll
-    for (int j = 0; j < RUN / 4; ++j) tq[j] = tk[j] = 0.f;
+    for (int j = 0; j < NC; ++j) tq[j] = tk[j] = 0.f;
     auto fma4 = [](float4& c, float4 u, float4 v) {
       c.x = fmaf(u.x, v.x, c.x); c.y = fmaf(u.y, v.y, c.y); c.z = fmaf(u.z, v.z, c.z); c.w = fmaf(u.w, v.w, c.w);
     };
 #pragma unroll 1
     for (int d0 = 0; d0 < D; d0 += 16) {        // sums of 16 products in four chains, then of those: as short chains as the walk's
-      float4 aq[RUN / 4], ak[RUN / 4];
+      float4 aq[NC], ak[NC];
 #pragma unroll
-      for (int j = 0; j < RUN / 4; ++j) aq[j] = ak[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int j = 0; j < NC; ++j) aq[j] = ak[j] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int d = d0; d < d0 + 16; d += 4) {
         const float4 q4 = load4(qs + t * LD + d), k4 = load4(ks + t * LD + d);
 #pragma unroll
-        for (int j = 0; j < RUN / 4; ++j) {
-          const float4 s4 = load4(ks + (s0 + 4 * j) * LD + d);
+        for (int j = 0; j < NC; ++j) {
+          const float4 s4 = load4(ks + (s0 + PER * j) * LD + d);
           fma4(aq[j], q4, s4);
           if (DELTA) fma4(ak[j], k4, s4);
         }
       }
 #pragma unroll
-      for (int j = 0; j < RUN / 4; ++j) {
+      for (int j = 0; j < NC; ++j) {
         tq[j] += (aq[j].x + aq[j].y) + (aq[j].z + aq[j].w);
         if (DELTA) tk[j] += (ak[j].x + ak[j].y) + (ak[j].z + ak[j].w);
       }
     }
 #pragma unroll
-    for (int j = 0; j < RUN / 4; ++j) {
-      qkm[t * GRAM_LD + s0 + 4 * j] = tq[j];
-      if (DELTA) kkm[t * GRAM_LD + s0 + 4 * j] = tk[j];
+    for (int j = 0; j < NC; ++j) {
+      qkm[t * GRAM_LD + s0 + PER * j] = tq[j];
+      if (DELTA) kkm[t * GRAM_LD + s0 + PER * j] = tk[j];
     }
   }
   __syncthreads();
@@ -124,7 +128,7 @@ chunk_prepare_kernel(const float* x, long long C, int qoff, int koff, const floa
     }
   };
   const int per = H / G;
-  for (int hh = warp; hh < per; hh += 4) {
+  for (int hh = warp; hh < per; hh += PREP_WARPS<D>) {
     const int h = g * per + hh;
     const bool live = lane < cnt;
     const float a = live ? decay[(long long)(t0 + lane) * gstride + h] : 1.f;
@@ -423,10 +427,10 @@ long long ws_bytes(int T, int R, int H, int G, int D, bool delta) {
 template <int D, bool DELTA> int launch(const Args& a, cudaStream_t stream) {
   bf16* qk = reinterpret_cast<bf16*>(a.ws);
   bf16* pt = qk + runs_of(a.T, a.R) * a.G * QK_SIZE<D>;
-  constexpr int prep = (2 * RUN * (D + 4) + 6 * RUN * GRAM_LD) * 4;
+  constexpr int prep = (2 * RUN * (D + 4) + (2 + PREP_WARPS<D>) * RUN * GRAM_LD) * 4;
   if (prep > 48 * 1024)
     cudaFuncSetAttribute(chunk_prepare_kernel<D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep);
-  fmx_launch(chunk_prepare_kernel<D, DELTA>, dim3((a.max_q + RUN - 1) / RUN, a.G, a.R), dim3(128), prep, stream, a.x, a.C, a.qoff, a.koff,
+  fmx_launch(chunk_prepare_kernel<D, DELTA>, dim3((a.max_q + RUN - 1) / RUN, a.G, a.R), dim3(32 * PREP_WARPS<D>), prep, stream, a.x, a.C, a.qoff, a.koff,
              a.decay, a.weight, 2 * a.H, a.row_start, a.min_tokens, a.H, a.G, qk, pt);
   // 32 columns a block where blocks of 16 would be more than two for each SM: half the operands' traffic
   const bool pair = a.P % 32 == 0 && (long long)a.R * a.H * (a.P / 16) > (long long)(D > 64 ? 1 : 2) * fmx_num_sms();
