@@ -1046,3 +1046,17 @@ def test_channel_decays_in_runs_of_tokens(delta, lens, H, G, D, P):
             assert torch.equal(o1[at], o2[at]) and (out[at] == 0).all() and torch.equal(s3[order[r]].cpu(), state[order[r]])
         else:                                        # in waves of two runs the same bits as in one
             assert torch.equal(out[at].cpu().double().view(-1, H, P), o2[at]) and torch.equal(s3[order[r]], s2[order[r]])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,D,P,rot", [(3, 16, 8, 16), (5, 64, 64, 64), (2, 128, 36, 32), (4, 12, 4, 8), (3, 64, 32, 0)])
+def test_retention_prepare_in_fours(dtype, H, D, P, rot):
+    """A retention's operands four values a thread: the same bits as the kernel of one value a thread, which rows of an odd stride take."""
+    T, width = 9, 2 * H * D + H * P
+    x = rnd(T, width, dtype=dtype).to(DEV)
+    odd = torch.zeros(T, width + 1, dtype=dtype, device=DEV)
+    odd[:, :width] = x
+    pos, freq, decay = torch.arange(0, 900, 100, dtype=torch.int32, device=DEV), torch.rand(max(1, rot // 2), device=DEV), torch.rand(H, device=DEV)
+    a = k().retention_prepare(x, pos, freq, decay, H, D, P, rot, 0.3)
+    b = k().retention_prepare(odd[:, :width], pos, freq, decay, H, D, P, rot, 0.3)
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
