@@ -17,10 +17,9 @@
 //
 // The operands of a run and head are 57 KB (64 rows of state) or 94 KB (128), so a step's runs go in waves whose workspace is
 // bounded.  An infinity or a NaN spreads over its own request's run of 32 tokens, as in chunk_scan.cu.
-// 32 heads of 128 x 128 on 8 key heads, one request of 2,048 tokens: 769 us token by token, 359 here.  In a step of two requests,
-// 2,048 tokens together: 545 token by token; 130 to prepare and 228 for the runs here, 3.5 us each.  Measured with a preparation of
-// 150 us where this one takes 130: 64 x 64, one request, 384 and 237; without the delta rule 64 x 64 262 and 198, and 128 x 128,
-// 308 either way, which stays with the walk.  Against 64-bit, one request: 1.6e-7 of the result's norm, 2.2e-7 token by token.
+// Two requests of 2,048 tokens together, 32 heads of 128 x 128 on 8 key heads: 657 us token by token (545 without the launch), 355 here:
+// 130 to prepare, 228 for the runs, 3.5 us each.  64 x 64, one request: 384 and 237.  Against 64-bit: 1.3e-7 of the result's
+// norm, 1.4e-7 token by token.  Without the delta rule 64 x 64 262 and 198; 128 x 128, 308 either way, stays with the walk.
 #include <math.h>
 #include "split_mma.cuh"
 
