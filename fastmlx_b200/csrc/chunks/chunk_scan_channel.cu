@@ -17,8 +17,8 @@
 //
 // The operands of a run and head are 57 KB (64 rows of state) or 94 KB (128), so a step's runs go in waves whose workspace is
 // bounded.  An infinity or a NaN spreads over its own request's run of 32 tokens, as in chunk_scan.cu.
-// Two requests of 2,048 tokens together, 32 heads of 128 x 128 on 8 key heads: 657 us token by token (545 without the launch), 355 here:
-// 130 to prepare, 228 for the runs, 3.5 us each.  64 x 64, one request: 384 and 237.  Against 64-bit: 1.3e-7 of the result's
+// Two requests of 2,048 tokens together, 32 heads of 128 x 128 on 8 key heads: 657 us token by token (545 alone in a step), 374 here:
+// 150 to prepare, 227 for the runs, 3.5 us each.  64 x 64, one request: 384 and 237.  Against 64-bit: 1.3e-7 of the result's
 // norm, 1.4e-7 token by token.  Without the delta rule 64 x 64 262 and 198; 128 x 128, 308 either way, stays with the walk.
 #include <math.h>
 #include "split_mma.cuh"
@@ -57,23 +57,22 @@ template <int N, int LD, int OUT_LD> __device__ __forceinline__ void emit_terms(
 }
 
 // Eight warps: a lane holds a token's k, a warp an eighth of the channels, and as t goes on a lane's k decays and meets q_t and k_t,
-// which all lanes read together; no sum crosses lanes, the warps' shares are added up in order, eight tokens at a time.  What
-// the state will meet leaves from registers: a thread takes two neighbouring channels of half a run.  Bound by its instructions' latency:
-// three blocks of 128 channels share an SM's shared memory.  2,048 tokens of 32 heads: 150 us with sixteen tokens at a time and the
-// results staged in shared memory (two blocks an SM), 130 us so.
-constexpr int PREP_THREADS = 256, PREP_WARPS = 8, SHARE_LD = RUN + 1;
-template <int D> constexpr int PREP_SMEM = (RUN * (3 * D + 4) + 2 * RUN * GRAM_LD + PREP_WARPS * 16 * SHARE_LD) * 4;
+// which all lanes read together; no sum crosses lanes, the warps' shares are added up in order.  Bound by the latency of a
+// block's phases (with four warps a run and head took twice as long), of which two blocks share an SM.
+constexpr int PREP_THREADS = 256, PREP_WARPS = 8;
+template <int D> constexpr int PREP_SMEM = (3 * RUN * (D + 4) + (PREP_WARPS + 2) * RUN * GRAM_LD) * 4;
 
 template <int D, bool DELTA>
 __global__ void __launch_bounds__(PREP_THREADS)
 channel_prepare_kernel(ChannelArgs a) {
   constexpr int LD = D + 4, DS = D / PREP_WARPS;
   extern __shared__ __align__(16) float psm[];
-  float* ks = psm;                             // [32][LD]: every lane reads a row of its own
-  float* qs = ks + RUN * LD;                   // [32][D]
-  float* gs = qs + RUN * D;
-  float* pm = gs + RUN * D;                    // [P, M][32][GRAM_LD]
-  float* part = pm + 2 * RUN * GRAM_LD;        // [8 warps][P, M][8][SHARE_LD]
+  float* qs = psm;                             // [32][LD]; then A q
+  float* ks = qs + RUN * LD;
+  float* gs = ks + RUN * LD;
+  float* pm = gs + RUN * LD;                   // [P, M][32][GRAM_LD]
+  float* part = pm + 2 * RUN * GRAM_LD;        // [8 warps][P, M][16][GRAM_LD]; then (A_32 / A) k | A k, [32][LD] each
+  static_assert(2 * LD <= PREP_WARPS * GRAM_LD, "both fit");
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int place = a.lo + (int)blockIdx.x;
   pdl_wait();
@@ -90,7 +89,7 @@ channel_prepare_kernel(ChannelArgs a) {
     float4 v = which == 2 ? make_float4(1.f, 1.f, 1.f, 1.f) : make_float4(0.f, 0.f, 0.f, 0.f);
     if (row < cnt) v = which == 2 ? load4(a.decay + (long long)(t0 + row) * a.H * D + (long long)h * D + d)
                                   : load4(a.qkv + (long long)(t0 + row) * C + (long long)(which * a.G + g) * D + d);
-    store4(which == 0 ? qs + row * D + d : which == 1 ? ks + row * LD + d : gs + row * D + d, v);
+    store4((which == 0 ? qs : which == 1 ? ks : gs) + row * LD + d, v);
   }
   const float beta = DELTA && lane < cnt ? a.beta[(long long)(t0 + lane) * a.H + h] : 0.f;       // of token `lane`
   __syncthreads();
@@ -102,11 +101,11 @@ channel_prepare_kernel(ChannelArgs a) {
     kd[i / 2 + 1] = pair_of(v.z, v.w);
   }
 #pragma unroll 1
-  for (int t1 = 0; t1 < RUN; t1 += 8) {        // eight tokens' shares at a time
+  for (int t1 = 0; t1 < RUN; t1 += 16) {       // sixteen tokens' shares at a time
 #pragma unroll 2
-    for (int t = t1; t < t1 + 8; ++t) {
-      const ulonglong2* gt = reinterpret_cast<const ulonglong2*>(gs + t * D + warp * DS);
-      const ulonglong2* qt = reinterpret_cast<const ulonglong2*>(qs + t * D + warp * DS);
+    for (int t = t1; t < t1 + 16; ++t) {
+      const ulonglong2* gt = reinterpret_cast<const ulonglong2*>(gs + t * LD + warp * DS);
+      const ulonglong2* qt = reinterpret_cast<const ulonglong2*>(qs + t * LD + warp * DS);
       const ulonglong2* kt = reinterpret_cast<const ulonglong2*>(ks + t * LD + warp * DS);
       ulonglong2 gv[DS / 4], qv[DS / 4], kv[DS / 4];
 #pragma unroll
@@ -132,17 +131,17 @@ channel_prepare_kernel(ChannelArgs a) {
           m[1] = fma2(kd[2 * i + 1], kv[i].y, m[1]);
         }
       }
-      part[(warp * 16 + t - t1) * SHARE_LD + lane] = pair_sum(p[0]) + pair_sum(p[1]);
-      if (DELTA) part[(warp * 16 + 8 + t - t1) * SHARE_LD + lane] = pair_sum(m[0]) + pair_sum(m[1]);
+      part[(warp * 32 + t - t1) * GRAM_LD + lane] = pair_sum(p[0]) + pair_sum(p[1]);
+      if (DELTA) part[(warp * 32 + 16 + t - t1) * GRAM_LD + lane] = pair_sum(m[0]) + pair_sum(m[1]);
     }
     __syncthreads();
     // the warps' shares; P up to t = s, M (times beta_t) up to t = s + 1; a warp takes a row
-    for (int e = warp; e < (DELTA ? 16 : 8); e += PREP_WARPS) {
-      const int which = e >> 3, t = t1 + (e & 7);
-      const float* src = part + e * SHARE_LD + lane;
+    for (int e = warp; e < (DELTA ? 32 : 16); e += PREP_WARPS) {
+      const int which = e >> 4, t = t1 + (e & 15);
+      const float* src = part + e * GRAM_LD + lane;
       float s[PREP_WARPS];
 #pragma unroll
-      for (int i = 0; i < PREP_WARPS; ++i) s[i] = src[i * 16 * SHARE_LD];
+      for (int i = 0; i < PREP_WARPS; ++i) s[i] = src[i * 32 * GRAM_LD];
       float v = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
       if (which) v *= __shfl_sync(0xffffffffu, beta, t);
       pm[(which * RUN + t) * GRAM_LD + lane] = (which ? lane < t : lane <= t) ? v : 0.f;
@@ -177,45 +176,32 @@ channel_prepare_kernel(ChannelArgs a) {
   }
   constexpr int threads = DELTA ? PREP_THREADS - 32 : PREP_THREADS;
   const int at = DELTA ? tid - 32 : tid;
+  float *ke = part, *ka = part + RUN * LD;
   float* last = reinterpret_cast<float*>(back + K_PLANE<D> + (DELTA ? 2 : 1) * PLANE);
-  // A k (delta rule), A q and (A_32 / A) k: two neighbouring channels of sixteen tokens to a thread
-  for (int x = at; x < (DELTA ? 3 : 2) * D; x += threads) {
-    const int what = DELTA ? x / D : x / D + 1, d = x % (D / 2) * 2, t1 = x / (D / 2) % 2 * 16;
-    bf16* dst = what == 0 ? front : what == 1 ? front + (DELTA ? K_PLANE<D> : 0) : back;
-    float2 e = make_float2(1.f, 1.f);          // the decays up to a token, or those behind it
-    auto decays = [&](int t) {
-      const float2 g2 = *reinterpret_cast<const float2*>(gs + t * D + d);
-      e.x *= g2.x;
-      e.y *= g2.y;
-    };
-    auto leave = [&](int t, const float* src) {
-      const float2 v = *reinterpret_cast<const float2*>(src + d);
-      unsigned u[3];
-      three_terms(v.x * e.x, v.y * e.y, u[0], u[1], u[2]);
-#pragma unroll
-      for (int i = 0; i < 3; ++i) *reinterpret_cast<unsigned*>(dst + (i * RUN + t) * K_LD<D> + d) = u[i];
-    };
-    if (what == 2) {
-      if (t1 == 0)
-#pragma unroll 8
-        for (int t = RUN - 1; t >= 16; --t) decays(t);
-#pragma unroll 4
-      for (int t = t1 + 15; t >= t1; --t) {
-        leave(t, ks + t * LD);
-        decays(t);
+  for (int x = at; x < 2 * D; x += threads) {  // a column each: the decays behind a token, or those up to it
+    const int d = x < D ? x : x - D;
+    float e = 1.f;
+    if (x < D) {
+#pragma unroll 16
+      for (int t = RUN - 1; t >= 0; --t) {
+        ke[t * LD + d] = ks[t * LD + d] * e;
+        e *= gs[t * LD + d];
       }
     } else {
-      if (t1)
-#pragma unroll 8
-        for (int t = 0; t < 16; ++t) decays(t);
-#pragma unroll 4
-      for (int t = t1; t < t1 + 16; ++t) {
-        decays(t);
-        leave(t, what == 0 ? ks + t * LD : qs + t * D);
+#pragma unroll 16
+      for (int t = 0; t < RUN; ++t) {
+        e *= gs[t * LD + d];
+        qs[t * LD + d] *= e;
+        if (DELTA) ka[t * LD + d] = ks[t * LD + d] * e;
       }
-      if (what == 1 && t1) *reinterpret_cast<float2*>(last + d) = e;
+      last[d] = e;
     }
   }
+  if (DELTA) asm volatile("bar.sync 1, 224;\n" ::: "memory");
+  else __syncthreads();
+  if (DELTA) emit_terms<D, LD, K_LD<D>>(ka, front, at, threads);
+  emit_terms<D, LD, K_LD<D>>(qs, front + (DELTA ? K_PLANE<D> : 0), at, threads);
+  emit_terms<D, LD, K_LD<D>>(ke, back, at, threads);
   emit_terms<RUN, GRAM_LD, PT_LD>(pm, back + K_PLANE<D>, at, threads);
 }
 
