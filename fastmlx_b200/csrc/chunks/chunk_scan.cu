@@ -21,20 +21,15 @@
 //                  the decayed q . k^T and T, as three terms.  All runs at once.
 //   chunk_scan     per (request, head, 16 or 32 columns of S): the runs in order.
 //
-// A token that holds an infinity or a NaN makes the outputs of its own request's run of 32 tokens NaN, also those in front of it
-// in the run; other requests are not touched.
+// An infinity or a NaN reaches what the walk lets it reach, its own token and the ones behind it (in its own column where a value holds
+// it), as a NaN: its second term is inf - inf.  A run that holds one sums over earlier tokens without the zeros of later ones (lower_sums).
 #include <math.h>
-#include "split_mma.cuh"
+#include "runs.cuh"
 
 namespace {
-constexpr int RUN = 32;                         // tokens of a run
-// Rows of the workspaces are as far apart as chunk_scan wants them in shared memory (eight 16-byte pieces of eight rows meet no
-// bank twice), so that a run's operands are two runs of bytes to copy: k and q of a group, and P, T and numbers of a head.
-constexpr int PT_LD = RUN + 8;
-constexpr int GRAM_LD = RUN + 4;
+// A run's operands: k and q of a group, and P, T and numbers of a head.
 template <int D> constexpr int QK_LD = D + 8;
 template <int D> constexpr int QK_SIZE = 2 * 3 * RUN * QK_LD<D>;              // bf16 of q and k of a run and group
-constexpr int PLANE = 3 * RUN * PT_LD;                                        // bf16 of one 32 x 32 matrix in three terms
 template <bool DELTA> constexpr int PT_SIZE = (DELTA ? 2 : 1) * PLANE + 4 * RUN;   // P, T and, as floats, A_t and E_s
 
 // The place of a row's first run in the workspaces: rows do not overlap, whatever their lengths.
@@ -46,7 +41,7 @@ __device__ __forceinline__ int first_run(int row_start, int r) { return row_star
 // (1,777 tokens, 8 groups of 8 heads: 38 -> 31 us); of 64 rows five blocks of four warps share an SM (34 and 34 us).
 template <int D> constexpr int PREP_WARPS = D > 64 ? 8 : 4;
 template <int D, bool DELTA>
-__global__ void __launch_bounds__(32 * PREP_WARPS<D>)
+__global__ void __launch_bounds__(32 * PREP_WARPS<D>, D > 64 ? 2 : 5)          // as many blocks as shared memory holds
 chunk_prepare_kernel(const float* x, long long C, int qoff, int koff, const float* decay, const float* weight, int gstride,
                      const int* row_start, int min_tokens, int H, int G, bf16* qk, bf16* pt) {
   constexpr int LD = D + 4, THREADS = 32 * PREP_WARPS<D>;
@@ -156,25 +151,7 @@ chunk_prepare_kernel(const float* x, long long C, int qoff, int koff, const floa
 #pragma unroll
       for (int t = 0; t < RUN; ++t) mine[t * GRAM_LD + lane] = rows[t];
       __syncwarp();
-      // lane j solves for column j of T from the top down: T_ij = [i = j] - sum_{l < i} M_il T_lj
-      float T[RUN];
-#pragma unroll
-      for (int i = 0; i < RUN; ++i) {
-        float p[4] = {lane == i ? 1.f : 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int l = 0; l < i; l += 4) {
-          const float4 m = load4(mine + i * GRAM_LD + l);
-          p[0] = fmaf(-m.x, T[l], p[0]);
-          if (l + 1 < i) p[1] = fmaf(-m.y, T[l + 1], p[1]);
-          if (l + 2 < i) p[2] = fmaf(-m.z, T[l + 2], p[2]);
-          if (l + 3 < i) p[3] = fmaf(-m.w, T[l + 3], p[3]);
-        }
-        T[i] = (p[0] + p[1]) + (p[2] + p[3]);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < RUN; ++i) mine[i * GRAM_LD + lane] = T[i] * w;      // its columns take beta
-      __syncwarp();
+      solve_unit_lower(mine, lane, w);
       emit(out + PLANE);
       __syncwarp();
     }
@@ -245,9 +222,6 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
   unsigned* efr = ufr + Z::U_WORDS;
   unsigned* rfr = efr + Z::U_WORDS;
   const float sk = DELTA ? 0.f : skip[h];
-  auto meet = [&]() {                            // the four warps of these 16 columns
-    asm volatile("bar.sync %0, 128;\n" ::"r"(1 + mt) : "memory");
-  };
   const int row = lane >> 2, two = (lane & 3) * 2;            // a thread's columns of S: row, row + 8; within a tile of 8: two, two + 1
   float* sp = state + (long long)slot * slot_stride + ((long long)h * P + c0 + mt * 16) * D + w * (D / 4);
   float S[NS][4];
@@ -331,7 +305,7 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
       v[0] = fmaf(-A0, kS.at(0), v[0]); v[1] = fmaf(-A1, kS.at(1), v[1]);
       v[2] = fmaf(-A0, kS.at(2), v[2]); v[3] = fmaf(-A1, kS.at(3), v[3]);
       share_tile(rfr, v);
-      meet();
+      const bool odd = meet_any(1 + mt, not_finite(v));
       Sums u;
       u.zero();
 #pragma unroll
@@ -343,12 +317,14 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
         }
 #pragma unroll
       for (int i = 0; i < 4; ++i) v[i] = u.at(i);
+      if (odd) lower_sums(v, dp + PLANE, rfr, t0, row);
     }
+    const bool mine = not_finite(v);
     share_tile(ufr, v);
     v[0] *= E0; v[1] *= E1; v[2] *= E0; v[3] *= E1;
     share_tile(efr, v);
     if (!DELTA) read_out();                       // behind the tiles that the others wait for
-    meet();
+    const bool odd = meet_any(1 + mt, mine);
     // S <- A_32 S + sum_s (E_s u_s) k_s^T for this warp's rows of state, and what the run's own tokens give: the decayed
     // q . k^T times u
     Sums y, d[NS];
@@ -381,7 +357,10 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
       for (int i = 0; i < 4; ++i) S[j][i] = fmaf(S[j][i], last, d[j].at(i));
     share_state();                                // the others' reads of these fragments lie in front of the last meeting
     const int t = c * RUN + t0;
-    float res[4] = {fmaf(A0, o.at(0), y.at(0)), fmaf(A1, o.at(1), y.at(1)), fmaf(A0, o.at(2), y.at(2)), fmaf(A1, o.at(3), y.at(3))};
+    float res[4] = {y.at(0), y.at(1), y.at(2), y.at(3)};
+    if (odd) lower_sums(res, dp, ufr, t0, row);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) res[i] = fmaf(i & 1 ? A1 : A0, o.at(i), res[i]);
     if (!DELTA) {
       res[0] = fmaf(sk, x0, res[0]); res[1] = fmaf(sk, x1, res[1]);
       res[2] = fmaf(sk, x2, res[2]); res[3] = fmaf(sk, x3, res[3]);

@@ -16,15 +16,14 @@
 //   channel_chunks    per (request, head, 16 or 32 columns of S): the runs in order.
 //
 // The operands of a run and head are 57 KB (64 rows of state) or 94 KB (128), so a step's runs go in waves whose workspace is
-// bounded.  An infinity or a NaN spreads over its own request's run of 32 tokens, as in chunk_scan.cu.
+// bounded.  An infinity or a NaN reaches what it reaches in chunk_scan.cu.
 // Two requests of 2,048 tokens together, 32 heads of 128 x 128 on 8 key heads: 657 us token by token (545 alone in a step), 374 here:
 // 150 to prepare, 227 for the runs, 3.5 us each.  64 x 64, one request: 384 and 237.  Against 64-bit: 1.3e-7 of the result's
 // norm, 1.4e-7 token by token.  Without the delta rule 64 x 64 262 and 198; 128 x 128, 308 either way, stays with the walk.
 #include <math.h>
-#include "split_mma.cuh"
+#include "runs.cuh"
 
 namespace {
-constexpr int RUN = 32, PT_LD = RUN + 8, GRAM_LD = RUN + 4, PLANE = 3 * RUN * PT_LD;
 template <int D> constexpr int K_LD = D + 8;
 template <int D> constexpr int K_PLANE = 3 * RUN * K_LD<D>;                   // bf16 of one 32 x D matrix in three terms
 // a run and head: in front A k (delta rule) and A q; behind them (A_32 / A) k, P, T (delta rule) and, as floats, A_32
@@ -151,26 +150,8 @@ channel_prepare_kernel(ChannelArgs a) {
   bf16* front = a.ws + ((long long)blockIdx.x * a.H + h) * (FRONT<D, DELTA> + BACK<D, DELTA>);
   bf16* back = front + FRONT<D, DELTA>;
   if (DELTA && warp == 0) {
-    // lane j solves for column j of T from the top down: T_ij = [i = j] - sum_{l < i} M_il T_lj
     float* M = pm + RUN * GRAM_LD;
-    float T[RUN];
-#pragma unroll
-    for (int i = 0; i < RUN; ++i) {
-      float p[4] = {lane == i ? 1.f : 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int l = 0; l < i; l += 4) {
-        const float4 m = load4(M + i * GRAM_LD + l);
-        p[0] = fmaf(-m.x, T[l], p[0]);
-        if (l + 1 < i) p[1] = fmaf(-m.y, T[l + 1], p[1]);
-        if (l + 2 < i) p[2] = fmaf(-m.z, T[l + 2], p[2]);
-        if (l + 3 < i) p[3] = fmaf(-m.w, T[l + 3], p[3]);
-      }
-      T[i] = (p[0] + p[1]) + (p[2] + p[3]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < RUN; ++i) M[i * GRAM_LD + lane] = T[i] * beta;      // its columns take beta
-    __syncwarp();
+    solve_unit_lower(M, lane, beta);
     emit_terms<RUN, GRAM_LD, PT_LD>(M, back + K_PLANE<D> + PLANE, lane, 32);
     return;
   }
@@ -260,7 +241,7 @@ channel_chunks_kernel(ChannelArgs a) {
 #pragma unroll 8
       for (int e = lane * 16; e < BACK<D, DELTA> * 2; e += 512) cp16(csm + Z::FRONT_BYTES + e, src + e, true);
       landed();
-      __syncthreads();                         // (2) its back is there, its front has been read
+      __syncthreads_or(0);                     // (2) its back is there, its front has been read
     }
     return;
   }
@@ -341,7 +322,7 @@ channel_chunks_kernel(ChannelArgs a) {
     } else {
       share_tile(ufr, v);
     }
-    __syncthreads();                           // (2)
+    bool odd = __syncthreads_or(not_finite(v));        // (2)
     if (DELTA) {                               // u = T diag(beta) (v - (A k) S)
       unsigned bt[3][4];
       Sums u;
@@ -357,8 +338,10 @@ channel_chunks_kernel(ChannelArgs a) {
         }
 #pragma unroll
       for (int i = 0; i < 4; ++i) v[i] = u.at(i);
+      if (odd) lower_sums(v, dp + PLANE, rfr, t0, row);
+      const bool mine = not_finite(v);
       share_tile(ufr, v);
-      asm volatile("bar.sync %0, 128;\n" ::"r"(1 + mt) : "memory");
+      odd = meet_any(1 + mt, mine);
     }
     Sums y, d[NS];
     y.zero();
@@ -390,13 +373,17 @@ channel_chunks_kernel(ChannelArgs a) {
     }
     share_state();                             // the others' reads of these fragments lie in front of (2)
     const int t = c * RUN + t0;
+    float res[4] = {y.at(0), y.at(1), y.at(2), y.at(3)};
+    if (odd) lower_sums(res, dp, ufr, t0, row);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) res[i] += o.at(i);
     if (t < n) {
-      op[(long long)t * ostride + row] = o.at(0) + y.at(0);
-      op[(long long)t * ostride + row + 8] = o.at(2) + y.at(2);
+      op[(long long)t * ostride + row] = res[0];
+      op[(long long)t * ostride + row + 8] = res[2];
     }
     if (t + 1 < n) {
-      op[(long long)(t + 1) * ostride + row] = o.at(1) + y.at(1);
-      op[(long long)(t + 1) * ostride + row + 8] = o.at(3) + y.at(3);
+      op[(long long)(t + 1) * ostride + row] = res[1];
+      op[(long long)(t + 1) * ostride + row + 8] = res[3];
     }
   }
 #pragma unroll

@@ -848,6 +848,51 @@ def test_portions_in_runs_of_tokens(rule, lens, H, G, D, P):
             assert torch.equal(o1[starts[r]:starts[r + 1]], o2[starts[r]:starts[r + 1]])
 
 
+@pytest.mark.parametrize("what", ["value", "key", "query", "decay", "weight"])
+@pytest.mark.parametrize("form,D,P", [("delta", 64, 48), ("delta", 128, 32), ("plain", 64, 32), ("plain", 128, 48), ("channel delta", 64, 32),
+                                      ("channel delta", 128, 48), ("channel plain", 64, 48)])
+def test_values_that_are_not_finite_in_runs_of_tokens(form, D, P, what):
+    """An infinity or a NaN leaves the same values finite in runs of 32 tokens as in the walk token by token: those of the tokens in
+    front of it, also of its own run, of other requests and, where a value holds it, of the other columns."""
+    torch.manual_seed(D + P)
+    channel, delta = form.startswith("channel"), form.endswith("delta")
+    lens = (70, 128) if delta or not channel else (300, 257)
+    if channel and D == 64 and delta:
+        lens = (140, 128)
+    starts, R, H, G = [0] + list(torch.tensor(lens).cumsum(0).tolist()), len(lens), 4, 2 if delta else 4
+    T = starts[-1]
+    ctx = SimpleNamespace(R=R, row_start=torch.tensor(starts, dtype=torch.int32, device=DEV), max_q_len=max(lens), h_row_start=starts,
+                          row_slot=torch.arange(R, dtype=torch.int32, device=DEV))
+    unit = lambda *s: torch.nn.functional.normalize(torch.randn(*s), dim=-1)
+    q, kk, v, w = unit(T, G, D), unit(T, G, D), torch.randn(T, H, P), torch.rand(T, H) * 0.8 + 0.1
+    decay, skip = torch.rand(T, H, D if channel else 1) * 0.3 + 0.7, torch.randn(H)
+    for t, bad in ((37, float("inf")), (52, float("nan"))):        # a run's first and second half
+        if what == "value":
+            v[t, t % H, t % P] = bad
+        elif what == "weight":
+            w[t, t % H] = float("nan")
+        else:
+            {"key": kk, "query": q, "decay": decay}[what][t, t % (H if what == "decay" else G), -1] = bad
+    if what == "weight" and channel and not delta:
+        pytest.skip("no weight")
+    order = [q, kk, v] if delta or channel else [v, kk, q]
+    x, state = torch.cat([t.flatten(1) for t in order], 1).to(DEV), torch.randn(R, H * P * D).to(DEV)
+    s1, s2 = state.clone(), state.clone()
+    if channel:
+        more = (decay.flatten(1).to(DEV), w.to(DEV) if delta else None, ctx)
+        o = [fn(x, *more, s, H, G, D, P) for fn, s in ((k().channel_scan, s1), (k().channel_scan_chunks, s2))]
+    else:
+        more = (torch.cat([decay.flatten(1), w] if delta else [w, decay.flatten(1)], 1).to(DEV),) + (() if delta else (skip.to(DEV),))
+        fns = (k().delta_rule, k().delta_rule_chunks) if delta else (k().ssm_scan, k().ssm_scan_chunks)
+        o = [fn(x, *more, ctx, s, H, G, D, P) for fn, s in zip(fns, (s1, s2))]
+    for a, b in ((o[0], o[1]), (s1, s2)):
+        fine = torch.isfinite(a)
+        assert torch.equal(fine, torch.isfinite(b))
+        # as in the test above; 2^-24 of the largest value for some dozens of roundings
+        assert fine.any() and (a[fine] - b[fine]).abs().max() < 40 * 2.0 ** -24 * a[fine].abs().max()
+    assert torch.isfinite(o[1][:37]).all() and not torch.isfinite(o[1]).all()
+
+
 @pytest.mark.parametrize("lens,ctxs,nh,nkv,hd,vd,page,window,cap", [
     ((4,), (0,), 2, 1, 16, 16, 16, 0, 30.0), ((9, 1, 33), (0, 40, 31), 8, 8, 32, 64, 8, 0, 30.0), ((40, 3, 8), (3, 0, 57), 32, 8, 64, 64, 16, 20, 30.0),
     ((50,), (77,), 6, 3, 48, 32, 16, 0, 0.0), ((17, 5), (200, 0), 12, 3, 64, 16, 5, 0, 2.0), ((264, 31), (0, 700), 32, 8, 64, 64, 16, 0, 30.0)])
