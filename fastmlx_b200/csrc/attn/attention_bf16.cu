@@ -396,7 +396,7 @@ __device__ __forceinline__ void softmax_step(float (&s)[NT][4], float (&m)[2], f
 #pragma unroll
       for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[j][e] = cap_l2 * tanhf(s[j][e]);
+        for (int e = 0; e < 4; ++e) s[j][e] = cap_l2 * tanh_capped(s[j][e]);
     } else {
 #pragma unroll
       for (int j = 0; j < NT; ++j)

@@ -218,7 +218,7 @@ mixed_heads_tc_kernel(const float* q, long long q_stride, const bf16* kv, const 
 #pragma unroll
             for (int hh = 0; hh < HW; ++hh)
 #pragma unroll
-              for (int i = 0; i < 4; ++i) s[m][hh][i] = softcap * tanhf(s[m][hh][i]);
+              for (int i = 0; i < 4; ++i) s[m][hh][i] = softcap * tanh_capped(s[m][hh][i]);
         } else {
 #pragma unroll
           for (int m = 0; m < 2; ++m)

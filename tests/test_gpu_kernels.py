@@ -893,6 +893,47 @@ def test_values_that_are_not_finite_in_runs_of_tokens(form, D, P, what):
     assert torch.isfinite(o[1][:37]).all() and not torch.isfinite(o[1]).all()
 
 
+@pytest.mark.parametrize("weights", ["softmax", "sigmoid"])
+@pytest.mark.parametrize("window", [0, 20])
+def test_capped_scores_do_not_depend_on_later_keys(weights, window):
+    """A capped score takes a short form where it is small against the cap.  Which form it takes follows from the score alone: keys behind
+    a token, out of its sight and large, leave its output's bits; and both forms, side by side in a tile, stand against 64-bit."""
+    nh, nkv, hd, page, T, n, cap = 32, 8, 64, 16, 128, 100, 30.0
+    q, kv, ctx, grp = _attention_case(torch.bfloat16, nh, nkv, hd, page, [(0, T)], seed=5)
+    q = (q * 4).float()                              # scores of N(0, 4): below 0.8 of the cap
+    loud = kv.clone()
+    for j in range(n, T):
+        loud[int(grp.block_tables[0, j // page]), 0, :, j % page] *= 32
+    d, g = _full_ctx([(0, T)], ctx, grp)
+    d.T, d.h_row_start = T, [0, T]
+    mix, bias = torch.eye(nh) + 0.1 * torch.randn(nh, nh, generator=torch.Generator().manual_seed(6)), torch.full((nh,), -3.0)
+
+    def run(pages):
+        if weights == "softmax":
+            return k().paged_attention_wide(q.to(DEV), pages.to(DEV), d, g, nh, nkv, hd, hd ** -0.5, cap, window).cpu()
+        return k().sigmoid_attention(q.to(DEV), pages.to(DEV), d, g, nh, nkv, hd, hd, hd ** -0.5, cap, window, page, bias.to(DEV), mix.to(DEV)).cpu()
+    quiet, got = run(kv), run(loud)
+    assert torch.equal(quiet[:n], got[:n]) and not torch.equal(quiet[n:], got[n:])
+    K, V = (torch.cat([loud[int(p), i] for p in grp.block_tables[0, :T // page]], 1).double().repeat_interleave(nh // nkv, 0) for i in (0, 1))
+    s = torch.einsum("qhd,hkd->hqk", q.double().view(T, nh, hd), K) * hd ** -0.5
+    s = cap * torch.tanh(s / cap)
+    back = torch.arange(T)[:, None] - torch.arange(T)[None]
+    hidden = (back < 0) | ((back >= window) if window else False)
+    if weights == "softmax":
+        w = torch.softmax(s.masked_fill(hidden, -float("inf")), -1)
+        size = torch.einsum("hqk,hkd->qhd", w, V.abs())
+    else:
+        w = torch.sigmoid(s - 3.0).masked_fill(hidden, 0.0)
+        size = torch.einsum("hqk,hkd->qhd", torch.einsum("hg,gqk->hqk", mix.double().abs(), w), V.abs())
+        w = torch.einsum("hg,gqk->hqk", mix.double(), w)
+    want = torch.einsum("hqk,hkd->qhd", w, V).flatten(1)
+    # the rounding to bfloat16; operands of two terms are off by 2^-17: a weight, and by the queries a score, by 2^-17 of its products'
+    # sizes, which moves a weight by twice that; three terms (sigmoid): 2^-24 for some dozens of roundings, and a score's 64 products
+    products = (torch.einsum("qhd,hkd->hqk", q.double().view(T, nh, hd).abs(), K.abs()) * hd ** -0.5).masked_fill(hidden, 0.0).amax(-1).T[:, :, None]
+    eps = 2.0 ** -17 * (2 + 2 * products) if weights == "softmax" else 2.0 ** -24 * (48 + 64 * products)
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + (eps * size).flatten(1)).all()
+
+
 @pytest.mark.parametrize("lens,ctxs,nh,nkv,hd,vd,page,window,cap", [
     ((4,), (0,), 2, 1, 16, 16, 16, 0, 30.0), ((9, 1, 33), (0, 40, 31), 8, 8, 32, 64, 8, 0, 30.0), ((40, 3, 8), (3, 0, 57), 32, 8, 64, 64, 16, 20, 30.0),
     ((50,), (77,), 6, 3, 48, 32, 16, 0, 0.0), ((17, 5), (200, 0), 12, 3, 64, 16, 5, 0, 2.0), ((264, 31), (0, 700), 32, 8, 64, 64, 16, 0, 30.0)])
