@@ -5,7 +5,8 @@
 //     w_g(t, j) = sigmoid(cap(scale q_g(t) . k(j)) + b_g);   w'_h = sum_g M[h, g] w_g;   out_h(t) = sum_j w'_h(t, j) v(j)
 //
 // Keys and values are bfloat16; queries, weights, the mix and the mixed weights are 32-bit and enter their products as three
-// bfloat16 terms (split_mma.cuh), so no product is rounded more than a 32-bit multiply-add rounds it.
+// bfloat16 terms (split_mma.cuh), so no product is rounded more than a 32-bit multiply-add rounds it.  An infinite score
+// saturates its weight (`sum_of`); an infinite value, or an infinity in the mix, leaves NaN where 32-bit sums may leave an infinity.
 //
 // A block owns all heads of 8 tokens of one request and walks the keys in tiles of 32:
 //   scores   two warps per key/value head: S^T = K Q^T, 32 keys by 8 tokens for each of a warp's two query heads; Q's
@@ -200,6 +201,12 @@ mixed_heads_tc_kernel(const float* q, long long q_stride, const bf16* kv, const 
           for (int m = 0; m < 2; ++m) mma16816(low[m][hh], a[m], q1.x, q1.y);
         }
       }
+      // An infinity has no smaller terms (inf - inf), and one in a key meets queries' terms that are zero: where the sum is not finite,
+      // the leading terms alone say what it is
+      auto sum_of = [&](int m, int hh, int i) {
+        const float all = s[m][hh][i] + low[m][hh][i];
+        return all - all == 0.f ? all : s[m][hh][i];
+      };
       if (softcap > 0.f) {
         bool large = false;
         const float to_y = scale * inv_cap;
@@ -209,7 +216,7 @@ mixed_heads_tc_kernel(const float* q, long long q_stride, const bf16* kv, const 
           for (int hh = 0; hh < HW; ++hh)
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              s[m][hh][i] = (s[m][hh][i] + low[m][hh][i]) * to_y;
+              s[m][hh][i] = sum_of(m, hh, i) * to_y;
               large |= fabsf(s[m][hh][i]) > TANH_SMALL;
             }
         if (__any_sync(0xffffffffu, large)) {
@@ -233,7 +240,7 @@ mixed_heads_tc_kernel(const float* q, long long q_stride, const bf16* kv, const 
 #pragma unroll
           for (int hh = 0; hh < HW; ++hh)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) s[m][hh][i] = (s[m][hh][i] + low[m][hh][i]) * scale;
+            for (int i = 0; i < 4; ++i) s[m][hh][i] = sum_of(m, hh, i) * scale;
       }
 #pragma unroll
       for (int m = 0; m < 2; ++m) {

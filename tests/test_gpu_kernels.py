@@ -987,6 +987,29 @@ def test_mixed_heads_on_tensor_cores(lens, ctxs, nh, nkv, hd, vd, page, window, 
             assert torch.equal(got[starts[r]:starts[r + 1]], fma[starts[r]:starts[r + 1]])
 
 
+@pytest.mark.parametrize("cap", [0.0, 30.0])
+@pytest.mark.parametrize("where", ["query", "key"])
+def test_infinite_scores_saturate_mixed_heads(where, cap):
+    """An infinite query or key value makes weights of zero and one, on the tensor cores as with 32-bit multiply-adds."""
+    nh, nkv, hd, page, T = 8, 4, 64, 16, 70
+    q, kv, ctx, grp = _attention_case(torch.bfloat16, nh, nkv, hd, page, [(30, T)], seed=8)
+    q, inf = q.float(), float("inf")
+    if where == "query":
+        q.view(T, nh, hd)[[3, 40, 41], [0, 5, 7], [0, 17, 63]] = torch.tensor([inf, -inf, inf])
+    else:
+        for j, g, e, x in ((5, 0, 0, inf), (62, 2, 33, -inf), (90, 3, 63, inf)):
+            kv[int(grp.block_tables[0, j // page]), 0, g, j % page, e] = x
+            q[:, g * 128 + e] = q[:, g * 128 + e].bfloat16().float()      # no smaller terms
+    d, g = _full_ctx([(30, T)], ctx, grp)
+    d.T, d.h_row_start = T, [0, T]
+    mix, bias = torch.eye(nh) + 0.1 * torch.randn(nh, nh), torch.full((nh,), -2.0)
+    want, got = (k().sigmoid_attention(q.to(DEV), kv.to(DEV), d, g, nh, nkv, hd, hd, hd ** -0.5, cap, 0, page, bias.to(DEV), mix.to(DEV),
+                                       tensor_cores=tc).cpu().double() for tc in (False, None))
+    assert torch.isfinite(want).all() and torch.isfinite(got).all()
+    # two roundings to bfloat16, and those of the 32-bit sums
+    assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 2.0 ** -16 * want.abs().max()).all()
+
+
 @pytest.mark.parametrize("form", ["delta", "ssm", "channel"])
 @pytest.mark.parametrize("lens", [(1,), (1, 1, 1, 1, 1), (2, 1, 3), (5, 40, 1, 17), (700, 4, 3)])
 def test_convolutions_by_strips_of_tokens(form, lens):
