@@ -393,11 +393,12 @@ bool sizes_fit(int nh, int nkv, int hd, int vd) {
 // How many blocks share out the keys of 8 tokens, or 0 where the kernel does not take the sizes.  A prompt's last tiles walk the
 // most keys: with one block each they alone would run at the end (1,531 tokens: the longest of 192 walks 48 tiles, an
 // SM's share is 31).  So many that the longest share is about an SM's; at least four tiles of keys to a block, and at most
-// 256 MB of partial sums.
-FMX_EXPORT int fmx_mixattn_tc_plan(int n_tokens, int rows, int nh, int nkv, int hd, int vd, int max_q_len, int max_ctx) {
+// 256 MB of partial sums.  Behind a window (0: none) 8 tokens walk the tiles that window + 7 keys lie in.
+FMX_EXPORT int fmx_mixattn_tc_plan(int n_tokens, int rows, int nh, int nkv, int hd, int vd, int max_q_len, int max_ctx, int window) {
   if (!sizes_fit(nh, nkv, hd, vd) || n_tokens <= 0) return 0;
-  const long long tiles = n_tokens / TQ + rows, longest = (max_ctx + TK - 1) / TK;
-  const long long usual = longest - max_q_len / 2 / TK;              // a row's tiles on average
+  const long long tiles = n_tokens / TQ + rows, whole = (max_ctx + TK - 1) / TK;
+  const long long held = window > 0 ? ((long long)window + TQ - 3) / TK + 2 : whole, longest = held < whole ? held : whole;
+  const long long half = whole - max_q_len / 2 / TK, usual = half < longest ? half : longest;        // a row's tiles on average
   const long long total = tiles * (usual > 0 ? usual : 1);
   long long s = (longest * fmx_num_sms() + total - 1) / total;
   if (s > longest / 4) s = longest / 4;

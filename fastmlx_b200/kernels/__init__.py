@@ -849,7 +849,8 @@ def sigmoid_attention(q, kv, ctx, group, nh, nkv, hd, vd, scale, softcap, window
             return torch.empty((splits, T, nh * vd), dtype=torch.float32, device=q.device) if splits > 1 else None
         least = WALK_ANY
         if tensor_cores is not False and ctx.max_q_len >= MIXED_TC_MIN_TOKENS and kv.data_ptr() % 16 == 0:
-            splits = int(load("chunks").fmx_mixattn_tc_plan(T, ctx.R, nh, nkv, hd, vd, int(ctx.max_q_len), int(ctx.max_ctx_after)))
+            splits = int(load("chunks").fmx_mixattn_tc_plan(T, ctx.R, nh, nkv, hd, vd, int(ctx.max_q_len), int(ctx.max_ctx_after),
+                                                            int(window)))
             if splits > 0:
                 least = MIXED_TC_MIN_TOKENS
                 launch("fmx_mixattn_tc", "chunks", parts(splits), least, splits)

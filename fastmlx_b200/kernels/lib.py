@@ -108,7 +108,7 @@ _SIGNATURES = {
     },
     "chunks": {
         "fmx_mixattn_tc": [_P, _L, _P, _P, _I, _P, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _L, _F, _F, _I, _I, _P, _P, _I, _I, _P, _P],
-        "fmx_mixattn_tc_plan": [_I, _I, _I, _I, _I, _I, _I, _I],
+        "fmx_mixattn_tc_plan": [_I, _I, _I, _I, _I, _I, _I, _I, _I],
         "fmx_chunk_delta_rule": [_P, _P, _P, _P, _P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],
         "fmx_channel_chunks": [_P, _P, _P, _P, _P, _P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _P],
         "fmx_chunk_ssm_scan": [_P, _P, _P, _P, _P, _P, _L, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P],

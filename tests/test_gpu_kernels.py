@@ -936,7 +936,8 @@ def test_capped_scores_do_not_depend_on_later_keys(weights, window):
 
 @pytest.mark.parametrize("lens,ctxs,nh,nkv,hd,vd,page,window,cap", [
     ((4,), (0,), 2, 1, 16, 16, 16, 0, 30.0), ((9, 1, 33), (0, 40, 31), 8, 8, 32, 64, 8, 0, 30.0), ((40, 3, 8), (3, 0, 57), 32, 8, 64, 64, 16, 20, 30.0),
-    ((50,), (77,), 6, 3, 48, 32, 16, 0, 0.0), ((17, 5), (200, 0), 12, 3, 64, 16, 5, 0, 2.0), ((264, 31), (0, 700), 32, 8, 64, 64, 16, 0, 30.0)])
+    ((50,), (77,), 6, 3, 48, 32, 16, 0, 0.0), ((17, 5), (200, 0), 12, 3, 64, 16, 5, 0, 2.0), ((264, 31), (0, 700), 32, 8, 64, 64, 16, 0, 30.0),
+    ((64, 31), (900, 700), 32, 8, 64, 64, 16, 300, 30.0)])
 def test_mixed_heads_on_tensor_cores(lens, ctxs, nh, nkv, hd, vd, page, window, cap):
     """Sigmoid attention with mixed heads over portions with three-term operands, against 64-bit arithmetic and beside the kernel of
     32-bit multiply-adds: tiles of tokens and keys with remainders, rows that stay on the other kernel, fewer heads than a tile
@@ -963,7 +964,7 @@ def test_mixed_heads_on_tensor_cores(lens, ctxs, nh, nkv, hd, vd, page, window, 
                           max_ctx_after=max(c + n for c, n in zip(ctxs, lens)), status=torch.zeros(4, dtype=torch.int32, device=DEV))
     run = lambda tc: k().sigmoid_attention(q.to(DEV), kv, ctx, SimpleNamespace(block_tables=bt.to(DEV)), nh, nkv, hd, vd, hd ** -0.5, cap, window,
                                            page, bias.to(DEV), mix.to(DEV), tensor_cores=tc).cpu().double().view(T, nh, vd)
-    plan = k().load("chunks").fmx_mixattn_tc_plan(T, R, nh, nkv, hd, vd, ctx.max_q_len, ctx.max_ctx_after)
+    plan = k().load("chunks").fmx_mixattn_tc_plan(T, R, nh, nkv, hd, vd, ctx.max_q_len, ctx.max_ctx_after, window)
     assert plan >= 1 and (plan > 1 or ctx.max_ctx_after < 256)
     fma, got = run(False), run(None)
     assert ctx.status.tolist()[0] == 0
@@ -985,6 +986,15 @@ def test_mixed_heads_on_tensor_cores(lens, ctxs, nh, nkv, hd, vd, page, window, 
     for r in range(R):
         if lens[r] < k().MIXED_TC_MIN_TOKENS:        # these rows run where they ran
             assert torch.equal(got[starts[r]:starts[r + 1]], fma[starts[r]:starts[r + 1]])
+
+
+@pytest.mark.parametrize("ctx", [2000, 60000])
+@pytest.mark.parametrize("window", [1, 26, 27, 90, 120, 121, 122, 500])
+def test_shares_of_a_window_are_no_fewer_than_four_tiles(ctx, window):
+    """Behind a window the keys are shared out as behind as much context: 8 tokens meet at most the tiles of 32 that window + 7 keys lie in."""
+    plan = k().load("chunks").fmx_mixattn_tc_plan
+    most = max((first + window + 6) // 32 + 1 for first in range(32))
+    assert plan(64, 1, 32, 8, 64, 64, 64, ctx, window) == max(1, min(most // 4, 32)) < plan(64, 1, 32, 8, 64, 64, 64, ctx, 0)
 
 
 @pytest.mark.parametrize("cap", [0.0, 30.0])
