@@ -43,7 +43,7 @@ template <int D> constexpr int PREP_WARPS = D > 64 ? 8 : 4;
 template <int D, bool DELTA>
 __global__ void __launch_bounds__(32 * PREP_WARPS<D>, D > 64 ? 2 : 5)          // as many blocks as shared memory holds
 chunk_prepare_kernel(const float* x, long long C, int qoff, int koff, const float* decay, const float* weight, int gstride,
-                     const int* row_start, int min_tokens, int H, int G, bf16* qk, bf16* pt) {
+                     const int* row_start, int min_tokens, int H, int G, bf16* qk, bf16* pt, int lo, int hi) {
   constexpr int LD = D + 4, THREADS = 32 * PREP_WARPS<D>;
   extern __shared__ __align__(16) float psm[];
   float* qs = psm;                              // [32][LD]
@@ -57,7 +57,8 @@ chunk_prepare_kernel(const float* x, long long C, int qoff, int koff, const floa
   const int first = row_start[r], n = row_start[r + 1] - first;
   if (c * RUN >= n || n < min_tokens) return;
   const int t0 = first + c * RUN, cnt = min(RUN, n - c * RUN);
-  const long long run = first_run(first, r) + c;
+  const long long run = first_run(first, r) + c - lo;
+  if (run < 0 || run >= hi - lo) return;         // a run of another wave
   bf16* planes = qk + (run * G + g) * QK_SIZE<D>;
   for (int e = tid; e < 2 * RUN * (D / 4); e += THREADS) {
     const int which = e / (RUN * (D / 4)), row = e / (D / 4) % RUN, d = e % (D / 4) * 4;
@@ -177,7 +178,8 @@ template <int D, int MT, bool DELTA> struct ScanSmem {
 template <int D, int MT, bool DELTA>
 __global__ void __launch_bounds__(128 * MT + 32)
 chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, int voff, const float* skip, const int* row_start,
-                  const int* row_slot, float* state, long long slot_stride, float* out, int min_tokens, int H, int G, int P, int max_slots) {
+                  const int* row_slot, float* state, long long slot_stride, float* out, int min_tokens, int H, int G, int P, int max_slots,
+                  int lo, int hi) {
   using Z = ScanSmem<D, MT, DELTA>;
   constexpr int KT = D / 16, NS = D / 32;        // k-tiles of S; 8-row tiles of S^T per warp
   extern __shared__ __align__(16) unsigned char csm[];
@@ -189,13 +191,15 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
   if (slot < 0 || slot >= max_slots) return;
   const int first = row_start[r], n = row_start[r + 1] - first;
   if (n < min_tokens) return;                    // walked token by token in a launch of its own
-  const int runs = (n + RUN - 1) / RUN, g = h / (H / G);
-  const long long run0 = first_run(first, r);
+  const int place = first_run(first, r), g = h / (H / G);
+  const int c_lo = max(0, lo - place), c_hi = min((n + RUN - 1) / RUN, hi - place);        // the row's runs of this wave
+  if (c_lo >= c_hi) return;
+  const long long run0 = place - lo;             // (of the row's first run, which may lie in front of the workspace)
   if (tid >= 128 * MT) {                         // the copying warp: a run's operands land while the run before it is walked
     auto cp16 = [](void* dst, const void* src, bool there) {
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0));
     };
-    for (int c = 0; c < runs; ++c) {
+    for (int c = c_lo; c < c_hi; ++c) {
       unsigned char* dst = csm + (c & 1) * Z::STAGE;
       const unsigned char* src = reinterpret_cast<const unsigned char*>(qk + ((run0 + c) * G + g) * QK_SIZE<D>);
 #pragma unroll 8
@@ -264,7 +268,7 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
   float* op = out + (long long)first * ostride + (long long)h * P + c0 + mt * 16;
   const int t0 = w * 8 + two;                    // this thread's tokens of a run: t0, t0 + 1
   const int rows8 = w * 8 + (lane & 7), quarter = (lane >> 3) * 8;
-  for (int c = 0; c < runs; ++c) {
+  for (int c = c_lo; c < c_hi; ++c) {
     __syncthreads();                             // the run's operands and S's fragments are there
     const bf16* dq = reinterpret_cast<const bf16*>(csm + (c & 1) * Z::STAGE);
     const bf16* dk = dq + 3 * RUN * QK_LD<D>;
@@ -395,35 +399,38 @@ struct Args {
 
 long long runs_of(int T, int R) { return (long long)T / RUN + R; }       // places for runs: see first_run
 
-template <int D, bool DELTA> long long bytes_of(int T, int R, int H, int G) {
-  return runs_of(T, R) * 2 * ((long long)G * QK_SIZE<D> + (long long)H * PT_SIZE<DELTA>);
-}
-long long ws_bytes(int T, int R, int H, int G, int D, bool delta) {
-  return D == 64 ? (delta ? bytes_of<64, true>(T, R, H, G) : bytes_of<64, false>(T, R, H, G))
-                 : (delta ? bytes_of<128, true>(T, R, H, G) : bytes_of<128, false>(T, R, H, G));
+template <int D, bool DELTA> long long bytes_of(int H, int G) { return 2 * ((long long)G * QK_SIZE<D> + (long long)H * PT_SIZE<DELTA>); }
+long long place_bytes(int H, int G, int D, bool delta) {
+  return D == 64 ? (delta ? bytes_of<64, true>(H, G) : bytes_of<64, false>(H, G))
+                 : (delta ? bytes_of<128, true>(H, G) : bytes_of<128, false>(H, G));
 }
 
-template <int D, bool DELTA> int launch(const Args& a, cudaStream_t stream) {
+// The step's runs in waves of `wave` places, whose operands the workspace holds; a state passes from wave to wave in its slot.
+template <int D, bool DELTA> int launch(const Args& a, int wave, cudaStream_t stream) {
   bf16* qk = reinterpret_cast<bf16*>(a.ws);
-  bf16* pt = qk + runs_of(a.T, a.R) * a.G * QK_SIZE<D>;
+  bf16* pt = qk + (long long)wave * a.G * QK_SIZE<D>;
   constexpr int prep = (2 * RUN * (D + 4) + (2 + PREP_WARPS<D>) * RUN * GRAM_LD) * 4;
   if (prep > 48 * 1024)
     cudaFuncSetAttribute(chunk_prepare_kernel<D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep);
-  fmx_launch(chunk_prepare_kernel<D, DELTA>, dim3((a.max_q + RUN - 1) / RUN, a.G, a.R), dim3(32 * PREP_WARPS<D>), prep, stream, a.x, a.C, a.qoff, a.koff,
-             a.decay, a.weight, 2 * a.H, a.row_start, a.min_tokens, a.H, a.G, qk, pt);
   // 32 columns a block where blocks of 16 would be more than two for each SM: half the operands' traffic
   const bool pair = a.P % 32 == 0 && (long long)a.R * a.H * (a.P / 16) > (long long)(D > 64 ? 1 : 2) * fmx_num_sms();
+  const long long places = runs_of(a.T, a.R);
+  for (long long at = 0; at < places; at += wave) {
+    const int lo = (int)at, hi = (int)(at + wave < places ? at + wave : places);
+    fmx_launch(chunk_prepare_kernel<D, DELTA>, dim3((a.max_q + RUN - 1) / RUN, a.G, a.R), dim3(32 * PREP_WARPS<D>), prep, stream, a.x, a.C, a.qoff,
+               a.koff, a.decay, a.weight, 2 * a.H, a.row_start, a.min_tokens, a.H, a.G, qk, pt, lo, hi);
 #define FMX_SCAN(MT)                                                                                                         \
   do {                                                                                                                       \
     constexpr size_t smem = ScanSmem<D, MT, DELTA>::BYTES;                                                                   \
     cudaFuncSetAttribute(chunk_scan_kernel<D, MT, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
     fmx_launch(chunk_scan_kernel<D, MT, DELTA>, dim3(a.P / (16 * MT), a.H, a.R), dim3(128 * MT + 32), smem, stream, (const bf16*)qk, \
-               (const bf16*)pt, a.x, a.C, a.voff, a.skip, a.row_start, a.row_slot, a.state, a.slot_stride, a.out, \
-               a.min_tokens, a.H, a.G, a.P, a.max_slots);                                                                                  \
+               (const bf16*)pt, a.x, a.C, a.voff, a.skip, a.row_start, a.row_slot, a.state, a.slot_stride, a.out, a.min_tokens, a.H, a.G, \
+               a.P, a.max_slots, lo, hi);                                                                                    \
   } while (0)
-  if (pair) FMX_SCAN(2);
-  else FMX_SCAN(1);
+    if (pair) FMX_SCAN(2);
+    else FMX_SCAN(1);
 #undef FMX_SCAN
+  }
   FMX_LAUNCH_CHECK();
   return 0;
 }
@@ -434,13 +441,20 @@ int check(const char* who, const Args& a, int D, bool delta, long long ws_size) 
   if (a.H > 65535 || a.R > 65535) return fmx_fail("%s: batch too large", who);
   if (a.C % 4 || a.slot_stride % 4 || (uintptr_t)a.x % 16 || (uintptr_t)a.state % 16 || (uintptr_t)a.ws % 16)
     return fmx_fail("%s: rows that do not start on 16 bytes", who);
-  if (ws_size < ws_bytes(a.T, a.R, a.H, a.G, D, delta)) return fmx_fail("%s: the workspace is too small", who);
+  if (ws_size < place_bytes(a.H, a.G, D, delta)) return fmx_fail("%s: the workspace is too small", who);
   return 0;
+}
+int wave_of(const Args& a, int D, bool delta, long long ws_size) {      // places that a workspace holds
+  const long long n = ws_size / place_bytes(a.H, a.G, D, delta), places = runs_of(a.T, a.R);
+  return (int)(n < places ? n : places);
 }
 }  // namespace
 
-// Bytes of workspace that T tokens of R rows take.
-FMX_EXPORT long long fmx_chunk_scan_bytes(int T, int R, int H, int G, int D, int delta) { return ws_bytes(T, R, H, G, D, delta != 0); }
+// Bytes of workspace that T tokens of R rows take: all their runs, or as many as 256 MB hold (the rest follow in waves).
+FMX_EXPORT long long fmx_chunk_scan_bytes(int T, int R, int H, int G, int D, int delta) {
+  const long long one = place_bytes(H, G, D, delta != 0), places = runs_of(T, R), most = (256LL << 20) / one;
+  return one * (places < most ? places : most < 1 ? 1 : most);
+}
 
 // The gated delta rule (see fmx_delta_rule) over the rows of at least min_tokens tokens; max_q: the longest one.
 FMX_EXPORT int fmx_chunk_delta_rule(const float* qkv, const float* gb, const int* row_start, const int* row_slot, float* state,
@@ -450,7 +464,8 @@ FMX_EXPORT int fmx_chunk_delta_rule(const float* qkv, const float* gb, const int
   const Args a = {qkv, gb, gb + H, nullptr, 2LL * G * D + (long long)H * Dv, 0, G * D, 2 * G * D, row_start, row_slot, state, slot_stride,
                   out, ws, T, R, H, G, Dv, max_slots, max_q, min_tokens};
   if (int bad = check("fmx_chunk_delta_rule", a, D, true, ws_size)) return bad;
-  return D == 64 ? launch<64, true>(a, stream) : launch<128, true>(a, stream);
+  const int wave = wave_of(a, D, true, ws_size);
+  return D == 64 ? launch<64, true>(a, wave, stream) : launch<128, true>(a, wave, stream);
 }
 
 // The state-space recurrence (see fmx_ssm_scan) over them.
@@ -462,5 +477,6 @@ FMX_EXPORT int fmx_chunk_ssm_scan(const float* xbc, const float* dd, const float
   const Args a = {xbc, dd + H, dd, d_skip, (long long)inner + 2LL * G * N, inner + G * N, inner, 0, row_start, row_slot, state, slot_stride,
                   out, ws, T, R, H, G, P, max_slots, max_q, min_tokens};
   if (int bad = check("fmx_chunk_ssm_scan", a, N, false, ws_size)) return bad;
-  return N == 64 ? launch<64, false>(a, stream) : launch<128, false>(a, stream);
+  const int wave = wave_of(a, N, false, ws_size);
+  return N == 64 ? launch<64, false>(a, wave, stream) : launch<128, false>(a, wave, stream);
 }

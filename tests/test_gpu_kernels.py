@@ -826,6 +826,17 @@ def test_portions_in_runs_of_tokens(rule, lens, H, G, D, P):
     s1, s2 = state.to(DEV), state.to(DEV)
     o1, o2 = call(walk, s1).cpu().double().view(T, H, P), call(runs, s2).cpu().double().view(T, H, P)
     assert torch.equal(s2[:, H * P * D:].cpu(), state[:, H * P * D:])
+    bytes_of, least, skips = k().load("chunks").fmx_chunk_scan_bytes, k().chunk_min_tokens(D), () if rule == "delta" else (skip.to(DEV),)
+    s3, out, xd, gd = state.to(DEV), torch.zeros(T, H * P, device=DEV), x.to(DEV), gates.to(DEV)
+    ws = torch.empty(2 * int(bytes_of(1, 1, H, G, D, int(rule == "delta"))), dtype=torch.uint8, device=DEV)         # two runs at a time
+    k().call("chunks", "fmx_chunk_delta_rule" if rule == "delta" else "fmx_chunk_ssm_scan", xd.data_ptr(), gd.data_ptr(), *(t.data_ptr() for t in skips),
+             ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(), s3.data_ptr(), s3.stride(0), out.data_ptr(), ws.data_ptr(), ws.numel(), T, R, H, G, D,
+             P, R, max(lens), least, k()._stream())
+    assert bytes_of(10 ** 7, R, H, G, D, int(rule == "delta")) <= 256 << 20
+    for r in range(R):                               # the same bits in waves of two runs; rows too short for runs are left alone
+        at, run = slice(starts[r], starts[r + 1]), lens[r] >= least
+        assert torch.equal(out[at].cpu().double().view(-1, H, P), o2[at] if run else 0 * o2[at])
+        assert torch.equal(s3[order[r]].cpu(), s2[order[r]].cpu() if run else state[order[r]])
     f = lambda t: t.double().repeat_interleave(H // G, 1)
     want, left = torch.empty(T, H, P, dtype=torch.float64), state.double().clone()
     for r in range(R):
