@@ -420,7 +420,7 @@ FMX_EXPORT int fmx_mixattn_tc(const float* q, long long q_stride, const void* kv
   if (out_stride < (long long)nh * vd) return fmx_fail("fmx_mixattn_tc: output rows too narrow");
   if (((uintptr_t)q & 7) || (q_stride & 1) || ((uintptr_t)kv & 15) || (splits > 1 && ((uintptr_t)part & 15)))
     return fmx_fail("fmx_mixattn_tc: queries must lie on 8 bytes, pages and partial sums on 16");
-  if (cudaFuncSetAttribute(mixed_heads_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess)
+  if (raise_shared<mixed_heads_tc_kernel>(SMEM) != cudaSuccess)
     return fmx_fail("fmx_mixattn_tc: the kernel's shared memory could not be raised");
   fmx_launch(mixed_heads_tc_kernel, dim3(n_tokens / TQ + R, splits), dim3(THREADS), SMEM, stream, q, q_stride, (const bf16*)kv, block_tables,
              bt_stride, positions, row_start, part, (bf16*)out, out_stride, n_tokens, nh, nkv, hd, vd, page_size, num_pages, scale, softcap,

@@ -410,8 +410,7 @@ template <int D, bool DELTA> int launch(const Args& a, int wave, cudaStream_t st
   bf16* qk = reinterpret_cast<bf16*>(a.ws);
   bf16* pt = qk + (long long)wave * a.G * QK_SIZE<D>;
   constexpr int prep = (2 * RUN * (D + 4) + (2 + PREP_WARPS<D>) * RUN * GRAM_LD) * 4;
-  if (prep > 48 * 1024)
-    cudaFuncSetAttribute(chunk_prepare_kernel<D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep);
+  if (prep > 48 * 1024) raise_shared<chunk_prepare_kernel<D, DELTA>>(prep);
   // 32 columns a block where blocks of 16 would be more than two for each SM: half the operands' traffic
   const bool pair = a.P % 32 == 0 && (long long)a.R * a.H * (a.P / 16) > (long long)(D > 64 ? 1 : 2) * fmx_num_sms();
   const long long places = runs_of(a.T, a.R);
@@ -422,7 +421,7 @@ template <int D, bool DELTA> int launch(const Args& a, int wave, cudaStream_t st
 #define FMX_SCAN(MT)                                                                                                         \
   do {                                                                                                                       \
     constexpr size_t smem = ScanSmem<D, MT, DELTA>::BYTES;                                                                   \
-    cudaFuncSetAttribute(chunk_scan_kernel<D, MT, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
+    raise_shared<chunk_scan_kernel<D, MT, DELTA>>(smem);                                                                     \
     fmx_launch(chunk_scan_kernel<D, MT, DELTA>, dim3(a.P / (16 * MT), a.H, a.R), dim3(128 * MT + 32), smem, stream, (const bf16*)qk, \
                (const bf16*)pt, a.x, a.C, a.voff, a.skip, a.row_start, a.row_slot, a.state, a.slot_stride, a.out, a.min_tokens, a.H, a.G, \
                a.P, a.max_slots, lo, hi);                                                                                    \

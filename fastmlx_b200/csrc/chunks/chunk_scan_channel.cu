@@ -395,18 +395,18 @@ channel_chunks_kernel(ChannelArgs a) {
 
 template <int D, bool DELTA> int launch(ChannelArgs a, int places, int per_wave, cudaStream_t stream) {
   constexpr int prep = PREP_SMEM<D>;
-  cudaFuncSetAttribute(channel_prepare_kernel<D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep);
+  raise_shared<channel_prepare_kernel<D, DELTA>>(prep);
   const bool pair = a.P % 32 == 0 && (long long)a.R * a.H * (a.P / 16) > (long long)(D > 64 ? 1 : 3) * fmx_num_sms();
   for (a.lo = 0; a.lo < places; a.lo += per_wave) {
     a.hi = a.lo + per_wave < places ? a.lo + per_wave : places;
     fmx_launch(channel_prepare_kernel<D, DELTA>, dim3(a.hi - a.lo, a.H), dim3(PREP_THREADS), prep, stream, a);
     if (pair) {
       constexpr size_t smem = ChannelSmem<D, 2, DELTA>::BYTES;
-      cudaFuncSetAttribute(channel_chunks_kernel<D, 2, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      raise_shared<channel_chunks_kernel<D, 2, DELTA>>(smem);
       fmx_launch(channel_chunks_kernel<D, 2, DELTA>, dim3(a.P / 32, a.H, a.R), dim3(288), smem, stream, a);
     } else {
       constexpr size_t smem = ChannelSmem<D, 1, DELTA>::BYTES;
-      cudaFuncSetAttribute(channel_chunks_kernel<D, 1, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      raise_shared<channel_chunks_kernel<D, 1, DELTA>>(smem);
       fmx_launch(channel_chunks_kernel<D, 1, DELTA>, dim3(a.P / 16, a.H, a.R), dim3(160), smem, stream, a);
     }
   }

@@ -4,6 +4,17 @@
 #include "packed.cuh"
 
 namespace {
+// Lets a kernel have `bytes` (always the same for one kernel) of dynamic shared memory: asked for once per thread and device.
+template <auto KERNEL> inline cudaError_t raise_shared(size_t bytes) {
+  static thread_local int raised = -1;
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess || device == raised) return e;
+  e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) raised = device;
+  return e;
+}
+
 // (x, y) -> three pairs of bfloat16 whose sums are x and y (to 2^-27 of them)
 __device__ __forceinline__ void three_terms(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);

@@ -48,6 +48,7 @@ class StepContext:
     h_row_ctx: list[int] = field(default_factory=list)
     h_row_slot: list[int] = field(default_factory=list)
     max_q_len: int = 0
+    min_q_len: int = 0                 # (0: not known)
     max_ctx_after: int = 0
     all_decode: bool = False           # every row brings exactly one token
     # a mixed step whose first rows bring one token each (the scheduler puts decoding requests first): how many,
@@ -230,6 +231,6 @@ def build_context(entries, manager, device, status, *, pad_rows: int = 0, pad_bl
         row_start=dview("row_start"), row_ctx=dview("row_ctx"), row_slot=dview("row_slot"),
         logit_rows=dview("want"), status=status, groups=groups, caches=manager.entries,
         h_row_start=rstart.tolist(), h_row_ctx=rctx.tolist(), h_row_slot=rslot.tolist(),
-        max_q_len=max(q_lens + [1]), max_ctx_after=max([c + q for c, q in zip(ctxs, q_lens)] + [1]),
+        max_q_len=max(q_lens + [1]), min_q_len=min(q_lens + [1] * (Rp > R)), max_ctx_after=max([c + q for c, q in zip(ctxs, q_lens)] + [1]),
         all_decode=all(q == 1 for q in q_lens), scratch={"h2d_bytes": host.nbytes, "layout_ints": total},
         **leading_decode_rows(q_lens, ctxs))

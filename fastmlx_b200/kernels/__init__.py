@@ -8,6 +8,8 @@ matrix mode.  Nothing here runs on the CPU.
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from . import lib as _lib
@@ -38,13 +40,14 @@ def _need_cuda(*ts):
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device      # (the latter asks each time whether CUDA is up)
 
 
 def _stream():
     """The current stream's handle.  A step makes a hundred and more launches, and building a
     torch.cuda.Stream object for each cost about 5 us of host time per launch."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_device())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -608,16 +611,60 @@ def chunk_scan_takes(ctx, D: int, Dv: int) -> bool:
 def _has_short_rows(ctx, least: int) -> bool:
     if ctx.R == 1:
         return False                      # the longest row is the only one
+    shortest = getattr(ctx, "min_q_len", 0)
+    if shortest:
+        return shortest < least
     starts = getattr(ctx, "h_row_start", None)
     return not starts or any(b - a < least for a, b in zip(starts, starts[1:]))
 
 
-def _chunk_scan(kind, x, gates, skip, ctx, state, H, G, D, Dv) -> torch.Tensor:
+# A step's recurrences go in runs from heads x (tokens of the step + tokens of its longest row) on.  The device gains by runs from
+# `chunk_min_tokens` and `channel_chunks_least` on, but a step of portions is launched from Python, and a second kernel and a
+# workspace cost the host 8 to 10 us a layer (with short rows walked beside them 20): below these a layer's launches take longer
+# than its kernels.  A layer from Python, walked and in runs, us: delta rule 64 rows of state, 32 heads, one row of 128 tokens 88 and 98,
+# 256 tokens 115 and 98; 128 rows 64 tokens 89 and 99, 96 tokens 114 and 99.  State space of 128 rows, 64 heads 64 tokens 70 and 81, 128
+# tokens 90 and 81; 128 heads 64 tokens 110 and 90.  Retention 64 rows, 32 heads 128 tokens 146 and 154, 384 tokens 192 and 160.
+# Channel decays 64 rows, 32 heads 256 tokens 106 and 113, 384 tokens 126 and 114; 128 rows 128 tokens 105 and 114, 192 tokens 130 and 114;
+# without the delta rule 384 tokens 91 and 98, 512 tokens 112 and 98.
+RUNS_FROM = {("delta", 64): 11264, ("delta", 128): 5120, ("plain", 64): 10240, ("plain", 128): 11264,
+             ("channel delta", 64): 20480, ("channel delta", 128): 9600, ("channel plain", 64): 28672}
+# Rows of so many tokens go in runs in such a step, shorter ones token by token: two launches one after the other cost more than
+# runs that are not full (delta rule of 64 rows, rows of 60, 100 and 140 tokens: 107 us with 60 walked, 101 all in runs; 85 walked).
+RUNS_LEAST_ROW = 16
+
+
+def rows_in_runs(rule: str, ctx, T: int, H: int, D: int, Dv: int) -> int:
+    """Rows of how many tokens go in runs of 32 in this step of T tokens (`least` of `delta_rule_chunks` and its like), or 0: all rows
+    are walked token by token."""
+    longest, delta = ctx.max_q_len, rule != "channel plain"
+    if longest < RUNS_LEAST_ROW or H * (T + longest) < RUNS_FROM.get((rule, D), WALK_ANY):
+        return 0
+    if rule.startswith("channel"):
+        # runs cost the device more for all tokens together and less along the longest row: of rows of 204 to 481 tokens, 2,048 together,
+        # without the delta rule 274 us and 248 walked (140 to 327, 700 together: 97 and 120); with it 128 rows, 60 to 140, 600 together,
+        # 215 and 209 (300 together: 132 and 143)
+        gains = 5 * longest >= 2 * T and channel_scan_takes(ctx, D, Dv, delta)
+    else:
+        gains = chunk_scan_takes(ctx, D, Dv)
+    return RUNS_LEAST_ROW if gains else 0
+
+
+@functools.lru_cache(maxsize=256)
+def _chunk_bytes(T, R, H, G, D, delta) -> int:
+    return int(load("chunks").fmx_chunk_scan_bytes(T, R, H, G, D, int(delta)))
+
+
+@functools.lru_cache(maxsize=256)
+def _channel_bytes(T, R, H, D, delta) -> int:
+    return int(load("chunks").fmx_channel_chunks_bytes(T, R, H, D, int(delta)))
+
+
+def _chunk_scan(kind, x, gates, skip, ctx, state, H, G, D, Dv, least) -> torch.Tensor:
     _need_cuda(x, gates, state)
     assert x.is_contiguous() and x.dtype == torch.float32 and gates.is_contiguous() and gates.dtype == torch.float32
-    T, least = x.shape[0], chunk_min_tokens(D)
+    T, least = x.shape[0], least or chunk_min_tokens(D)
     out = torch.empty((T, H * Dv), dtype=torch.float32, device=x.device)
-    ws = torch.empty(int(load("chunks").fmx_chunk_scan_bytes(T, ctx.R, H, G, D, int(skip is None))), dtype=torch.uint8, device=x.device)
+    ws = torch.empty(_chunk_bytes(T, ctx.R, H, G, D, skip is None), dtype=torch.uint8, device=x.device)
     more = (skip.data_ptr(),) if skip is not None else ()
     if _has_short_rows(ctx, least):
         call("common", f"fmx_{kind}", x.data_ptr(), gates.data_ptr(), *more, ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(),
@@ -628,14 +675,15 @@ def _chunk_scan(kind, x, gates, skip, ctx, state, H, G, D, Dv) -> torch.Tensor:
     return out
 
 
-def delta_rule_chunks(qkv, gb, ctx, state, H, G, D, Dv) -> torch.Tensor:
-    """`delta_rule` with the step's portions in runs of 32 tokens as matrix products (see `chunk_scan_takes`)."""
-    return _chunk_scan("delta_rule", qkv, gb, None, ctx, state, H, G, D, Dv)
+def delta_rule_chunks(qkv, gb, ctx, state, H, G, D, Dv, least: int = 0) -> torch.Tensor:
+    """`delta_rule` with the step's portions in runs of 32 tokens as matrix products (see `chunk_scan_takes`): rows of at least
+    `least` tokens (0: `chunk_min_tokens`)."""
+    return _chunk_scan("delta_rule", qkv, gb, None, ctx, state, H, G, D, Dv, least)
 
 
-def ssm_scan_chunks(xbc, dd, d_skip, ctx, state, H, G, N, P) -> torch.Tensor:
+def ssm_scan_chunks(xbc, dd, d_skip, ctx, state, H, G, N, P, least: int = 0) -> torch.Tensor:
     """`ssm_scan`, likewise."""
-    return _chunk_scan("ssm_scan", xbc, dd, d_skip, ctx, state, H, G, N, P)
+    return _chunk_scan("ssm_scan", xbc, dd, d_skip, ctx, state, H, G, N, P, least)
 
 
 def gated_rmsnorm(o, gate, weight, eps, H, Dv, out_dtype, out=None) -> torch.Tensor:
@@ -839,26 +887,24 @@ def sigmoid_attention(q, kv, ctx, group, nh, nkv, hd, vd, scale, softcap, window
     bt = group.block_tables
     name = mixed_heads_library(nh, nkv, hd, vd, q, kv) if tiled is not False and out.dtype == torch.bfloat16 else None
     if name is not None:
-        def launch(fn, lib, part, *last):
-            call(lib, fn, q.data_ptr(), q.stride(0), kv.data_ptr(), bt.data_ptr(), bt.stride(0), ctx.token_row.data_ptr(),
-                 ctx.positions.data_ptr(), ctx.row_start.data_ptr(), _ptr(part), out.data_ptr(), out.stride(0), T, nh, nkv, hd, vd,
-                 int(page_size), kv.shape[0], float(scale), float(softcap or 0.0), int(window), bt.shape[0], _ptr(head_bias),
-                 mix.data_ptr(), *last, _ptr(ctx.status), _stream())
-
-        def parts(splits):
-            return torch.empty((splits, T, nh * vd), dtype=torch.float32, device=q.device) if splits > 1 else None
-        least = WALK_ANY
-        if tensor_cores is not False and ctx.max_q_len >= MIXED_TC_MIN_TOKENS and kv.data_ptr() % 16 == 0:
-            splits = int(load("chunks").fmx_mixattn_tc_plan(T, ctx.R, nh, nkv, hd, vd, int(ctx.max_q_len), int(ctx.max_ctx_after),
-                                                            int(window)))
+        R, longest, ctx_len = bt.shape[0], int(ctx.max_q_len), int(ctx.max_ctx_after)
+        front = (q.data_ptr(), q.stride(0), kv.data_ptr(), bt.data_ptr(), bt.stride(0), ctx.token_row.data_ptr(), ctx.positions.data_ptr(),
+                 ctx.row_start.data_ptr())
+        back = (out.data_ptr(), out.stride(0), T, nh, nkv, hd, vd, int(page_size), kv.shape[0], float(scale), float(softcap or 0.0),
+                int(window), R, _ptr(head_bias), mix.data_ptr())
+        most = WALK_ANY                                  # longest row that the 32-bit multiply-adds take
+        if tensor_cores is not False and longest >= MIXED_TC_MIN_TOKENS and kv.data_ptr() % 16 == 0:
+            splits = load("chunks").fmx_mixattn_tc_plan(T, R, nh, nkv, hd, vd, longest, ctx_len, int(window))
             if splits > 0:
-                least = MIXED_TC_MIN_TOKENS
-                launch("fmx_mixattn_tc", "chunks", parts(splits), least, splits)
-                if not _has_short_rows(ctx, least):
+                part = torch.empty((splits, T, nh * vd), dtype=torch.float32, device=q.device) if splits > 1 else None
+                call("chunks", "fmx_mixattn_tc", *front, _ptr(part), *back, MIXED_TC_MIN_TOKENS, splits, _ptr(ctx.status), _stream())
+                if not _has_short_rows(ctx, MIXED_TC_MIN_TOKENS):
                     return out
-        splits = int(load(name).fmx_mixattn_plan(T, nh, nkv, hd, vd, int(ctx.max_q_len), int(ctx.max_ctx_after)))
+                most = MIXED_TC_MIN_TOKENS - 1
+        splits = load(name).fmx_mixattn_plan(T, nh, nkv, hd, vd, longest, ctx_len)
         if splits > 0:
-            launch("fmx_mixattn", name, parts(splits), int(ctx.max_q_len), splits, least - 1 if least != WALK_ANY else least)
+            part = torch.empty((splits, T, nh * vd), dtype=torch.float32, device=q.device) if splits > 1 else None
+            call(name, "fmx_mixattn", *front, _ptr(part), *back, longest, splits, most, _ptr(ctx.status), _stream())
             return out
     assert tiled is not True, "the tiled kernel does not take these sizes"
     part = torch.empty((T, nh, nkv, vd), dtype=torch.float32, device=q.device)
@@ -936,13 +982,14 @@ def channel_scan_takes(ctx, D: int, Dv: int, delta: bool) -> bool:
     return D in ((64, 128) if delta else (64,)) and Dv % 16 == 0 and ctx.max_q_len >= channel_chunks_least(D, delta)
 
 
-def channel_scan_chunks(qkv, g, beta, ctx, state, H, G, D, Dv) -> torch.Tensor:
-    """`channel_scan` with the step's portions in runs of 32 tokens as matrix products (see `channel_scan_takes`)."""
+def channel_scan_chunks(qkv, g, beta, ctx, state, H, G, D, Dv, least: int = 0) -> torch.Tensor:
+    """`channel_scan` with the step's portions in runs of 32 tokens as matrix products (see `channel_scan_takes`): rows of at least
+    `least` tokens (0: `channel_chunks_least`)."""
     _need_cuda(qkv, g, beta, state)
     assert qkv.is_contiguous() and g.is_contiguous() and (beta is None or beta.is_contiguous())
-    T, least = qkv.shape[0], channel_chunks_least(D, beta is not None)
+    T, least = qkv.shape[0], least or channel_chunks_least(D, beta is not None)
     out = torch.empty((T, H * Dv), dtype=torch.float32, device=qkv.device)
-    ws = torch.empty(int(load("chunks").fmx_channel_chunks_bytes(T, ctx.R, H, D, int(beta is not None))), dtype=torch.uint8, device=qkv.device)
+    ws = torch.empty(_channel_bytes(T, ctx.R, H, D, beta is not None), dtype=torch.uint8, device=qkv.device)
     if _has_short_rows(ctx, least):
         call("chan", "fmx_channel_scan", qkv.data_ptr(), g.data_ptr(), _ptr(beta), ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(),
              state.data_ptr(), state.stride(0), out.data_ptr(), ctx.R, H, G, D, Dv, state.shape[0], 0, 0, 0, least - 1, _stream())

@@ -182,7 +182,7 @@ def load(group: str) -> ctypes.CDLL:
 def call(group: str, name: str, *args) -> None:
     global launches
     launches += 1
-    lib = load(group)
+    lib = _libs.get(group) or load(group)
     rc = getattr(lib, name)(*args)
     if rc != 0:
         raise KernelError(lib.fmx_last_error().decode(errors="replace"))

@@ -135,6 +135,13 @@ def to_compute(t: torch.Tensor, rt: Runtime) -> torch.Tensor:
     return t.to(device=rt.device, dtype=rt.dtype).contiguous()
 
 
+def rows_in_runs(rule: str, rt, ctx, T: int, H: int, D: int, Dv: int) -> int:
+    """Rows of how many tokens a recurrence takes in runs of 32 tokens in this step, 0: none (`kernels.rows_in_runs`).  The 32-bit path,
+    whose sums must not depend on how a prompt was cut, walks token by token."""
+    choose = getattr(rt.k, "rows_in_runs", None) if rt.dtype == torch.bfloat16 else None
+    return choose(rule, ctx, T, H, D, Dv) if choose is not None else 0
+
+
 def to_f32_vector(t: torch.Tensor, rt: Runtime) -> torch.Tensor:
     """Norm weights and biases are held in 32-bit (exact for either stored dtype)."""
     return t.to(device=rt.device, dtype=torch.float32).contiguous()

@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from .base import FreeDim, Mixer, Runtime, StateSpec, WeightSpec, to_f32_vector
+from .base import FreeDim, Mixer, Runtime, StateSpec, WeightSpec, rows_in_runs, to_f32_vector
 from .linear import BlockDiagonalLinear, Linear
 
 
@@ -78,9 +78,9 @@ class GatedDeltaMixer(Mixer):
         ab = self.ba.forward(x, out_dtype=torch.float32)
         qkv, gb = k.delta_prepare(proj, ab, self.conv_w, self.a_log, self.dt_bias, ctx, cache.state, self.s_floats,
                                   self.H, self.G, self.D, self.Dv, self.taps)
-        takes = getattr(k, "chunk_scan_takes", None) if self.rt.dtype == torch.bfloat16 else None
-        rule = k.delta_rule_chunks if takes is not None and takes(ctx, self.D, self.Dv) else k.delta_rule
-        o = rule(qkv, gb, ctx, cache.state, self.H, self.G, self.D, self.Dv)
+        args = (qkv, gb, ctx, cache.state, self.H, self.G, self.D, self.Dv)
+        least = rows_in_runs("delta", self.rt, ctx, qkv.shape[0], self.H, self.D, self.Dv)
+        o = k.delta_rule_chunks(*args, least) if least else k.delta_rule(*args)
         return k.gated_rmsnorm(o, proj[:, self.channels:], self.norm_w, self.eps, self.H, self.Dv, self.rt.dtype, out=out)
 
     def forward(self, x, ctx, cache):
@@ -173,9 +173,9 @@ class ChannelDeltaMixer(Mixer):
         qkv, g, beta = k.channel_delta_prepare(proj, proj[:, c + r:c + r + self.H], zg[:, :n], self.conv_w, self.a_log,
                                                self.dt_bias, ctx, cache.state, self.s_floats, self.H, self.G, self.D, self.Dv,
                                                self.taps)
-        takes = getattr(k, "channel_scan_takes", None) if self.rt.dtype == torch.bfloat16 else None
-        scan = k.channel_scan_chunks if takes is not None and takes(ctx, self.D, self.Dv, True) else k.channel_scan
-        o = scan(qkv, g, beta, ctx, cache.state, self.H, self.G, self.D, self.Dv)
+        args = (qkv, g, beta, ctx, cache.state, self.H, self.G, self.D, self.Dv)
+        least = rows_in_runs("channel delta", self.rt, ctx, qkv.shape[0], self.H, self.D, self.Dv)
+        o = k.channel_scan_chunks(*args, least) if least else k.channel_scan(*args)
         return k.head_norm_gate(o, zg[:, n:], self.norm_w, self.eps, self.H, self.Dv, self.rt.dtype, "sigmoid", out=out)
 
     def forward(self, x, ctx, cache):

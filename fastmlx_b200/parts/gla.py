@@ -3,7 +3,7 @@ from __future__ import annotations
 
 import torch
 
-from .base import FreeDim, Mixer, Runtime, StateSpec, WeightSpec, to_f32_vector
+from .base import FreeDim, Mixer, Runtime, StateSpec, WeightSpec, rows_in_runs, to_f32_vector
 from .linear import BlockDiagonalLinear, Linear
 
 
@@ -75,9 +75,9 @@ class GatedLinearAttention(Mixer):
         n, m = 2 * self.H * self.D + self.inner_features, self.inner_features
         z = self.second.forward(proj[:, n + m:n + m + self.second.in_features], out_dtype=torch.float32)
         qkv, alpha = k.channel_gla_prepare(proj, z, self.bias, self.H, self.D, self.Dv, self.D ** -0.5, self.tau)
-        takes = getattr(k, "channel_scan_takes", None) if self.rt.dtype == torch.bfloat16 else None
-        scan = k.channel_scan_chunks if takes is not None and takes(ctx, self.D, self.Dv, False) else k.channel_scan
-        o = scan(qkv, alpha, None, ctx, cache.state, self.H, self.H, self.D, self.Dv)
+        args = (qkv, alpha, None, ctx, cache.state, self.H, self.H, self.D, self.Dv)
+        least = rows_in_runs("channel plain", self.rt, ctx, qkv.shape[0], self.H, self.D, self.Dv)
+        o = k.channel_scan_chunks(*args, least) if least else k.channel_scan(*args)
         return k.head_norm_gate(o, proj[:, n:n + m], self.norm_w, self.eps, self.H, self.Dv, self.rt.dtype, "silu", out=out)
 
     def forward(self, x, ctx, cache):

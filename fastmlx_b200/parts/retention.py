@@ -3,7 +3,7 @@ from __future__ import annotations
 
 import torch
 
-from .base import Mixer, Runtime, StateSpec
+from .base import Mixer, Runtime, StateSpec, rows_in_runs
 from .linear import Linear
 from .rope import inverse_frequencies
 
@@ -76,8 +76,8 @@ class RetentionMixer(Mixer):
             proj = self.proj.forward(x, out_dtype=torch.float32)
         qkv, dd = k.retention_prepare(proj, ctx.positions, self.inv_freq, self.decay, self.H, self.D, self.P, self.rot_dims,
                                       self.D ** -0.5)
-        takes = getattr(k, "chunk_scan_takes", None) if self.rt.dtype == torch.bfloat16 else None
-        scan = k.ssm_scan_chunks if takes is not None and takes(ctx, self.D, self.P) else k.ssm_scan
-        o = scan(qkv, dd, self.no_skip, ctx, cache.state, self.H, self.H, self.D, self.P)
+        args = (qkv, dd, self.no_skip, ctx, cache.state, self.H, self.H, self.D, self.P)
+        least = rows_in_runs("plain", self.rt, ctx, qkv.shape[0], self.H, self.D, self.P)
+        o = k.ssm_scan_chunks(*args, least) if least else k.ssm_scan(*args)
         gate = proj[:, 2 * self.H * self.D + self.inner:self.proj_features]
         return k.retention_gate_norm(o, gate, self.eps, self.H, self.P, self.rt.dtype)

@@ -3,7 +3,7 @@ from __future__ import annotations
 
 import torch
 
-from .base import Mixer, Runtime, StateSpec, WeightSpec, to_f32_vector
+from .base import Mixer, Runtime, StateSpec, WeightSpec, rows_in_runs, to_f32_vector
 from .linear import Linear
 
 
@@ -78,8 +78,8 @@ class StateSpaceMixer(Mixer):
         # convolution, SiLU, step sizes and decays: x | B | C in 32-bit, (dt | decay) per head
         xbc, dd = k.ssm_prepare(proj, self.conv_w, self.conv_b, self.a_log, self.dt_bias, ctx, cache.state, self.s_floats,
                                 self.H, self.G, self.N, self.P, self.taps)
-        takes = getattr(k, "chunk_scan_takes", None) if self.rt.dtype == torch.bfloat16 else None
-        scan = k.ssm_scan_chunks if takes is not None and takes(ctx, self.N, self.P) else k.ssm_scan
-        y = scan(xbc, dd, self.d_skip, ctx, cache.state, self.H, self.G, self.N, self.P)
+        args = (xbc, dd, self.d_skip, ctx, cache.state, self.H, self.G, self.N, self.P)
+        least = rows_in_runs("plain", self.rt, ctx, xbc.shape[0], self.H, self.N, self.P)
+        y = k.ssm_scan_chunks(*args, least) if least else k.ssm_scan(*args)
         y = k.gated_group_rmsnorm(y, proj[:, :self.inner], self.norm_w, self.eps, self.norm_groups, self.rt.dtype)
         return self.o.forward(y)

@@ -859,6 +859,39 @@ def test_portions_in_runs_of_tokens(rule, lens, H, G, D, P):
             assert torch.equal(o1[starts[r]:starts[r + 1]], o2[starts[r]:starts[r + 1]])
 
 
+@pytest.mark.parametrize("rule,D", [("delta", 64), ("delta", 128), ("plain", 64), ("plain", 128), ("channel delta", 64), ("channel delta", 128),
+                                    ("channel plain", 64)])
+def test_short_rows_join_the_runs_of_a_long_one(rule, D):
+    """In a step that goes in runs its rows of 16 tokens and more do, beside shorter ones that are walked; single tokens and short
+    steps are walked whole."""
+    torch.manual_seed(D)
+    lens, H, G, P = (16, 300, 1, 15, 31, 33, 17), 4, 4 if rule.endswith("plain") else 2, 32
+    starts, R = [0] + list(torch.tensor(lens).cumsum(0).tolist()), len(lens)
+    T, channel, delta = starts[-1], rule.startswith("channel"), rule.endswith("delta")
+    ctx = SimpleNamespace(R=R, row_start=torch.tensor(starts, dtype=torch.int32, device=DEV), max_q_len=max(lens), min_q_len=1,
+                          row_slot=torch.arange(R, dtype=torch.int32, device=DEV))
+    least = k().rows_in_runs(rule, ctx, T, 64, D, P)
+    assert least == 16 and k().rows_in_runs(rule, ctx, T, 1, D, P) == 0 and k().rows_in_runs(rule, ctx, T, 64, D, P + 8) == 0
+    assert k().rows_in_runs(rule, SimpleNamespace(max_q_len=1), T, 64, D, P) == 0 and k().rows_in_runs(rule, ctx, T, 64, 32, P) == 0
+    unit = lambda *s: torch.nn.functional.normalize(torch.randn(*s), dim=-1)
+    q, kk, v, w = unit(T, G, D), unit(T, G, D), torch.randn(T, H, P), torch.rand(T, H)
+    decay = torch.rand(T, H, D if channel else 1) * 0.2 + 0.8
+    x, state = torch.cat([t.flatten(1) for t in ([q, kk, v] if delta or channel else [v, kk, q])], 1).to(DEV), torch.randn(R, H * P * D).to(DEV)
+    if channel:
+        more, fns = (decay.flatten(1).to(DEV), w.to(DEV) if delta else None), (k().channel_scan, k().channel_scan_chunks)
+    elif delta:
+        more, fns = (torch.cat([decay.flatten(1), w], 1).to(DEV),), (k().delta_rule, k().delta_rule_chunks)
+    else:
+        more, fns = (torch.cat([w, decay.flatten(1)], 1).to(DEV), torch.randn(H).to(DEV)), (k().ssm_scan, k().ssm_scan_chunks)
+    s1, s2 = state.clone(), state.clone()
+    want, got = fns[0](x, *more, ctx, s1, H, G, D, P), fns[1](x, *more, ctx, s2, H, G, D, P, least)
+    for r in range(R):
+        at = slice(starts[r], starts[r + 1])
+        for a, b in ((want[at], got[at]), (s1[r], s2[r])):
+            # as in the tests above, with the walk's own roundings
+            assert torch.equal(a, b) if lens[r] < least else (a - b).abs().max() < 80 * 2.0 ** -24 * a.abs().max()
+
+
 @pytest.mark.parametrize("what", ["value", "key", "query", "decay", "weight"])
 @pytest.mark.parametrize("form,D,P", [("delta", 64, 48), ("delta", 128, 32), ("plain", 64, 32), ("plain", 128, 48), ("channel delta", 64, 32),
                                       ("channel delta", 128, 48), ("channel plain", 64, 48)])
