@@ -796,7 +796,8 @@ def test_greedy_head_chooses_the_largest_logit(M, V, K):
 
 @pytest.mark.parametrize("rule", ["delta", "plain"])
 @pytest.mark.parametrize("lens,H,G,D,P", [((64,), 4, 2, 64, 64), ((65, 1, 97, 31, 128), 4, 2, 64, 48), ((63, 200), 3, 3, 64, 16),
-                                          ((32, 33, 7), 4, 1, 128, 128), ((31, 64), 2, 2, 128, 16), ((1, 2, 40, 96), 64, 8, 128, 32)])
+                                          ((32, 33, 7), 4, 1, 128, 128), ((31, 64), 2, 2, 128, 16), ((1, 2, 40, 96), 64, 8, 128, 32),
+                                          ((64, 70, 96, 33), 32, 8, 64, 64)])      # (more blocks than two an SM: 32 columns each)
 def test_portions_in_runs_of_tokens(rule, lens, H, G, D, P):
     """The kernels that walk runs of 32 tokens as matrix products, against 64-bit arithmetic and beside the walk token by token:
     portions of whole runs and a token more or less, rows too short for them, decays that are zero or nearly one, slots with state
@@ -1065,13 +1066,14 @@ def test_infinite_scores_saturate_mixed_heads(where, cap):
 
 
 @pytest.mark.parametrize("form", ["delta", "ssm", "channel"])
+@pytest.mark.parametrize("D", [32, 64, 128])
 @pytest.mark.parametrize("lens", [(1,), (1, 1, 1, 1, 1), (2, 1, 3), (5, 40, 1, 17), (700, 4, 3)])
-def test_convolutions_by_strips_of_tokens(form, lens):
+def test_convolutions_by_strips_of_tokens(form, lens, D):
     """The kernels that walk strips of tokens with the last inputs in registers (four taps, channels in fours) beside those token by
     token, which rows of an odd stride take: the same sums in the same order, unit vectors to their sums' rounding, the same slots;
     a row of a captured step that is not there, rows shorter than the taps, strips that hold several rows."""
     torch.manual_seed(len(lens))
-    H, G, D, P, taps = 12, 4, 64, 64, 4
+    H, G, P, taps = 12, 4, 64, 4
     starts = [0] + list(torch.tensor(lens).cumsum(0).tolist())
     T, R = starts[-1] + 1, len(lens) + 1                               # the last row's slot is -1
     starts.append(T)
@@ -1159,7 +1161,8 @@ def test_queries_and_keys_in_fours(tin, tkv, hd, vd, rot, inter, form):
         assert (kv1 != kv2).float().mean() < 2e-3
 @pytest.mark.parametrize("delta,lens,H,G,D,P", [
     (True, (128,), 4, 2, 64, 64), (True, (129, 1, 161, 127, 192), 4, 2, 64, 48), (True, (64, 65, 63), 4, 1, 128, 128), (True, (31, 128), 2, 2, 128, 16),
-    (True, (3, 72, 96), 32, 8, 128, 96), (False, (256,), 3, 3, 64, 64), (False, (257, 5, 255, 300), 4, 4, 64, 48), (False, (1, 288), 32, 32, 64, 32)])
+    (True, (3, 72, 96), 32, 8, 128, 96), (False, (256,), 3, 3, 64, 64), (False, (257, 5, 255, 300), 4, 4, 64, 48), (False, (1, 288), 32, 32, 64, 32),
+    (True, (128, 130, 160, 129), 32, 8, 64, 64), (False, (256, 257, 288, 256), 32, 32, 64, 64)])          # (more than three: 32 columns each)
 def test_channel_decays_in_runs_of_tokens(delta, lens, H, G, D, P):
     """The kernels that walk runs of 32 tokens whose state decays by key channel, against 64-bit arithmetic and beside the walk token
     by token: decays that are zero, that vanish within a run and that are nearly one, portions of whole runs and a token more or
