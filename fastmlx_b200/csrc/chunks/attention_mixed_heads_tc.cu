@@ -13,6 +13,7 @@
 //            terms lie in shared memory as right fragments.  Cap and sigmoid; the weights go to shared memory as terms, rows of (key, token) per head.
 //   mix      a warp per two keys: W = M P over all heads, terms back to where the keys' weights were.
 //   values   two warps per key/value head again: O^T = V^T W^T, added to the registers' 32-bit sums tile by tile.
+// The order of a sum over keys follows the number of blocks that share them out, and so the step's tokens and rows (fmx_mixattn_tc_plan).
 // A row of 8 tokens is 16 bytes, so that every transposition is an ldmatrix.  Tokens are the products' 8 columns and keys,
 // heads and value dimensions their 16 rows: with 16 tokens Q's terms and the weights
 // would not fit shared memory.
@@ -27,7 +28,9 @@
 #include "tanh_small.cuh"
 
 namespace {
-constexpr int TQ = 8, TK = 32, KVH = 8, PER = 4, HEADS = KVH * PER;      // at most KVH key heads of PER query heads
+// At most KVH key heads of PER query heads of MAXD values: their 224 KB are what an SM has (Q's terms 96, keys and values 72, weights 50, the
+// mix 6).  Larger sizes stay with 32-bit multiply-adds.
+constexpr int TQ = 8, TK = 32, KVH = 8, PER = 4, HEADS = KVH * PER;
 constexpr int WARPS = 16, HW = 2, THREADS = WARPS * 32;        // two warps to a key head, two query heads to a warp
 constexpr int MAXD = 64, KLD = MAXD + 8;          // a key or value row in shared memory: eight rows' pieces meet no bank twice
 constexpr int PROW = TK * TQ + 8;                 // a head's weights: 32 keys x 8 tokens, likewise

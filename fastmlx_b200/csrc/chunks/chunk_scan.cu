@@ -10,12 +10,12 @@
 //     S  <- A_32 S + sum_s (A_32 / A_s) k_s u_s^T
 //
 // Ratios A_t / A_s are running products of decays (at most one, no logarithm, no division).  Every product that meets the
-// state runs on the tensor cores with three bfloat16 terms an operand (split_mma.cuh), so that it is as exact as the walk
-// token by token in 32-bit multiply-adds (the kernels of delta_rule.cu and ssm.cu; 2,048 tokens against 64-bit, decays near one:
-// 1.8e-7 of the result's norm here, 2.4e-7 there; decays of 0.8: 1.2e-7 and 1.1e-7).  That walk is one chain of dependent
-// steps of some 250 ns a token; a run of 32 tokens here takes 1.4 us at 64 rows of state, 3.3 us at 128.  One request of 2,048
-// tokens, 32 heads on 8 key heads, both kernels: delta rule 64 x 64 521 -> 115 us, 128 x 128 (two requests) 1,010 -> 234 us;
-// plain write 346 -> 98 and 660 -> 198 us; 1,777 tokens of five requests, 64 heads of 64 values over 128 rows 561 -> 188 us.
+// state runs on the tensor cores with three bfloat16 terms an operand (split_mma.cuh), so that its errors are those of the walk
+// token by token in 32-bit multiply-adds (the kernels of delta_rule.cu and ssm.cu; 2,048 tokens of the delta rule against 64-bit, of
+// the result's norm: decays of 0.9 to 1 1.3e-7 either way, of 0.8 to 1 1.2e-7 here and 1.1e-7 there; plain write 1.1e-7 and 1.3e-7).
+// That walk is one chain of dependent steps of some 250 ns a token; a run of 32 tokens here takes 1.4 us at 64 rows of state, 3.3 us at 128.  One request of 2,048
+// tokens, 32 heads on 8 key heads, both kernels: delta rule 64 x 64 525 -> 120 us, 128 x 128 (two requests) 1,052 -> 232 us;
+// plain write 349 -> 104 and 665 -> 190 us; 1,777 tokens of five requests, 64 heads of 64 values over 128 rows 579 -> 184 us.
 //
 //   chunk_prepare  per (run, key group): k and q as three terms; k . k^T and q . k^T in 32-bit, and per head of the group
 //                  the decayed q . k^T and T, as three terms.  All runs at once.
@@ -411,7 +411,9 @@ template <int D, bool DELTA> int launch(const Args& a, int wave, cudaStream_t st
   bf16* pt = qk + (long long)wave * a.G * QK_SIZE<D>;
   constexpr int prep = (2 * RUN * (D + 4) + (2 + PREP_WARPS<D>) * RUN * GRAM_LD) * 4;
   if (prep > 48 * 1024) raise_shared<chunk_prepare_kernel<D, DELTA>>(prep);
-  // 32 columns a block where blocks of 16 would be more than two for each SM: half the operands' traffic
+  // 32 columns a block halve the operands' traffic, at half as many blocks: with 128 rows of state, whose blocks of 16 fill an SM alone,
+  // above one for each SM (512 tokens of each request, 32 heads of 64 values: 128 blocks 49 us and 66 with 32 columns, 256 82 and 68, 512 177
+  // and 137), with 64 rows above two, where it costs up to a tenth at these sizes (384 87 and 90, 512 91 and 98, 1,024 177 and 196)
   const bool pair = a.P % 32 == 0 && (long long)a.R * a.H * (a.P / 16) > (long long)(D > 64 ? 1 : 2) * fmx_num_sms();
   const long long places = runs_of(a.T, a.R);
   for (long long at = 0; at < places; at += wave) {

@@ -17,9 +17,9 @@
 //
 // The operands of a run and head are 57 KB (64 rows of state) or 94 KB (128), so a step's runs go in waves whose workspace is
 // bounded.  An infinity or a NaN reaches what it reaches in chunk_scan.cu.
-// Two requests of 2,048 tokens together, 32 heads of 128 x 128 on 8 key heads: 657 us token by token (545 alone in a step), 374 here:
-// 150 to prepare, 227 for the runs, 3.5 us each.  64 x 64, one request: 384 and 237.  Against 64-bit: 1.3e-7 of the result's
-// norm, 1.4e-7 token by token.  Without the delta rule 64 x 64 262 and 198; 128 x 128, 308 either way, stays with the walk.
+// 32 heads on 8 key heads of 128 x 128, 2,048 tokens: one request 754 us token by token and 379 here, two of 768 and 1,280 637 and 380
+// (of which 150 to prepare and 227 for the runs).  64 x 64, one request: 387 and 249; without the delta rule 265 and 204, while 128 x 128
+// takes 308 either way and stays with the walk.  Against 64-bit: 1.3e-7 of the result's norm, 1.4e-7 token by token.
 #include <math.h>
 #include "runs.cuh"
 
@@ -396,6 +396,9 @@ channel_chunks_kernel(ChannelArgs a) {
 template <int D, bool DELTA> int launch(ChannelArgs a, int places, int per_wave, cudaStream_t stream) {
   constexpr int prep = PREP_SMEM<D>;
   raise_shared<channel_prepare_kernel<D, DELTA>>(prep);
+  // 32 columns a block as in chunk_scan.cu, above one (128 rows) and three (64 rows) blocks of 16 for each SM.  At 512 tokens of each
+  // request, 32 heads of 64 values, that is no gain: 128 rows 384 blocks 238 us and 244, 1,024 573 and 594; 64 rows 512 181 and 192, 1,024 319
+  // and 380 (without the delta rule 512 137 and 144).
   const bool pair = a.P % 32 == 0 && (long long)a.R * a.H * (a.P / 16) > (long long)(D > 64 ? 1 : 3) * fmx_num_sms();
   for (a.lo = 0; a.lo < places; a.lo += per_wave) {
     a.hi = a.lo + per_wave < places ? a.lo + per_wave : places;

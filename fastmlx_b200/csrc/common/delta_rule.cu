@@ -19,8 +19,9 @@
 //   gated_rmsnorm     o of each head divided by its root mean square, times a weight, times SiLU(gate): in head_norm.cu.
 //
 // A slot's state is one run of 32-bit floats: S^T of every head, [H, Dv, D], and then the convolution inputs,
-// [taps-1, C].  Everything is 32-bit but the projections that come in and the activations that go out.  No sum's
-// order depends on how a request's tokens were cut into steps or on what else is in the batch.
+// [taps-1, C].  Everything is 32-bit but the projections that come in and the activations that go out.  In these
+// kernels no sum's order depends on how a request's tokens were cut into steps or on what else is in the batch; portions
+// of the bfloat16 path may take ../chunks/chunk_scan.cu, whose sums follow a portion's runs of 32 tokens.
 #include <math.h>
 #include "common.cuh"
 

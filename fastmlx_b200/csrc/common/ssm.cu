@@ -19,7 +19,8 @@
 //
 // A slot's state is one run of 32-bit floats: S^T of every head, [H, P, N], and then the convolution inputs,
 // [taps-1, C], C = H*P + 2*G*N.  Everything is 32-bit but the projection that comes in and the activations that go
-// out.  No sum's order depends on how a request's tokens were cut into steps or on what else is in the batch.
+// out.  In these kernels no sum's order depends on how a request's tokens were cut into steps or on what else is in
+// the batch; portions of the bfloat16 path may take ../chunks/chunk_scan.cu, whose sums follow a portion's runs of 32 tokens.
 #include <math.h>
 #include "common.cuh"
 #include "conv_strip.cuh"

@@ -593,7 +593,8 @@ def delta_rule(qkv, gb, ctx, state, H, G, D, Dv, lanes: int = 0) -> torch.Tensor
 
 
 def chunk_min_tokens(D: int) -> int:
-    """Rows of at least so many tokens are walked in runs of 32 as matrix products, shorter ones token by token.  Alone, 64 tokens
+    """From so many tokens on the device gains by walking a row in runs of 32 as matrix products (`rows_in_runs` says which rows of a step
+    do).  Alone, 64 tokens
     of 64 rows of state take as long either way (the delta rule 19 and 18 us, the plain write 14 and 18), 128 tokens 36 and 18;
     32 tokens of 128 rows 24 and 19 (18 and 19), 64 tokens 43 and 22.  Decoding rows beside a portion stay on the walk: 63 of
     them and 128 tokens took 62 us all walked, 131 all in runs."""
@@ -602,8 +603,8 @@ def chunk_min_tokens(D: int) -> int:
 
 def chunk_scan_takes(ctx, D: int, Dv: int) -> bool:
     """Do the kernels that walk runs of 32 tokens as matrix products take this step's portions (`delta_rule_chunks`,
-    `ssm_scan_chunks`)?  64 or 128 rows of state, values in steps of 16, and a portion long enough to gain by it.  They are as exact
-    as the walk token by token, but a sum's order follows the runs of a portion: a caller that needs the same bits however a
+    `ssm_scan_chunks`)?  64 or 128 rows of state, values in steps of 16, and a portion long enough to gain by it.  Their errors
+    are those of the walk token by token, but a sum's order follows the runs of a portion: a caller that needs the same bits however a
     prompt is cut (the 32-bit path) takes that walk."""
     return D in (64, 128) and Dv % 16 == 0 and ctx.max_q_len >= chunk_min_tokens(D)
 
@@ -635,7 +636,7 @@ RUNS_LEAST_ROW = 16
 
 def rows_in_runs(rule: str, ctx, T: int, H: int, D: int, Dv: int) -> int:
     """Rows of how many tokens go in runs of 32 in this step of T tokens (`least` of `delta_rule_chunks` and its like), or 0: all rows
-    are walked token by token."""
+    are walked token by token.  So the order of a portion's sums follows from what else is in the step too."""
     longest, delta = ctx.max_q_len, rule != "channel plain"
     if longest < RUNS_LEAST_ROW or H * (T + longest) < RUNS_FROM.get((rule, D), WALK_ANY):
         return 0
@@ -858,7 +859,8 @@ def mixed_heads_library(nh: int, nkv: int, hd: int, vd: int, q=None, kv=None) ->
 
 
 # A tile on the tensor cores takes as long for one token as for its eight.  32 rows behind 500 tokens: 2 tokens each 155 us on
-# 32-bit multiply-adds, 4 each 195 us, on the tensor cores 48.
+# 32-bit multiply-adds, 4 each 195 us, on the tensor cores 48.  Nor do short rows without context lose by it (a layer of the pair of mixers
+# on the device: 20 tokens 78 -> 56 us, 33 of four rows 83 -> 59, 48 of six rows 85 -> 62).
 MIXED_TC_MIN_TOKENS = 4
 
 
@@ -970,7 +972,7 @@ def channel_scan(qkv, g, beta, ctx, state, H, G, D, Dv, lanes: int = 0, cpt: int
 
 
 def channel_chunks_least(D: int, delta: bool) -> int:
-    """Rows of at least so many tokens go in runs of 32 as matrix products, shorter ones token by token.  With the delta rule, alone:
+    """`chunk_min_tokens` for decays by key channel.  With the delta rule, alone:
     64 rows of state 64 tokens 16 us walked and 18 in runs, 128 tokens 28 and 23; 128 rows of state 32 tokens 17 and 25, 64 tokens 29
     and 28.  Without it the walk has half the steps: 64 rows of state 128 tokens 20 and 19 us, 256 tokens 36 and 25."""
     return 8192 // D if delta else 256
