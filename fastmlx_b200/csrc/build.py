@@ -3,7 +3,7 @@
 The kernels are plain `extern "C"` entry points that take device pointers and a stream;
 they include no PyTorch header, so a library compiles in seconds and is loaded with
 ctypes.  Each group of sources becomes one shared library, and only the groups a run
-needs are built: the 32-bit path compiles none of the bfloat16 tensor-core kernels.
+needs are built: the 32-bit path compiles none of the bfloat16 kernels but the products over matrices stored so.
 """
 from __future__ import annotations
 

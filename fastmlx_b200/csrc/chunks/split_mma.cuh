@@ -2,6 +2,7 @@
 // six of the nine products of terms, summed in 32-bit.  What is left out lies 2^-24 below a product.
 #pragma once
 #include "packed.cuh"
+#include "three_terms.cuh"
 
 namespace {
 // Lets a kernel have `bytes` (always the same for one kernel) of dynamic shared memory: asked for once per thread and device.
@@ -13,19 +14,6 @@ template <auto KERNEL> inline cudaError_t raise_shared(size_t bytes) {
   e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e == cudaSuccess) raised = device;
   return e;
-}
-
-// (x, y) -> three pairs of bfloat16 whose sums are x and y (to 2^-27 of them)
-__device__ __forceinline__ void three_terms(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-  const float2 hf = __bfloat1622float2(h);
-  const float rx = x - hf.x, ry = y - hf.y;
-  const __nv_bfloat162 m = __floats2bfloat162_rn(rx, ry);
-  const float2 mf = __bfloat1622float2(m);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(rx - mf.x, ry - mf.y);
-  hi = *reinterpret_cast<const unsigned*>(&h);
-  mid = *reinterpret_cast<const unsigned*>(&m);
-  lo = *reinterpret_cast<const unsigned*>(&l);
 }
 
 __device__ __forceinline__ void mma16816(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {

@@ -321,15 +321,36 @@ __global__ void act_mul_bf16_vec_kernel(const bf16* gu, bf16* out, int I, int bl
   }
 }
 
+// 32-bit with I a multiple of 4: four elements per thread, 16-byte loads and stores (333 rows of 8,192: a step's pass 145 us with one at a time, 139 here).
+template <int KIND>
+__global__ void act_mul_f32_vec_kernel(const float* gu, float* out, int I, int blk) {
+  pdl_wait();
+  pdl_trigger();
+  const long long t = blockIdx.y;
+  const int nvec = I / 4, bvec = blk / 4;
+  const float4* gp = reinterpret_cast<const float4*>(gu + t * 2 * I);
+  float4* op = reinterpret_cast<float4*>(out + t * I);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += gridDim.x * blockDim.x) {
+    const int b = i / bvec, j = i - b * bvec;
+    const float4 g = gp[b * 2 * bvec + j], u = gp[b * 2 * bvec + bvec + j];
+    op[i] = make_float4(gate_act<KIND>(g.x) * u.x, gate_act<KIND>(g.y) * u.y, gate_act<KIND>(g.z) * u.z, gate_act<KIND>(g.w) * u.w);
+  }
+}
+
 template <int KIND>
 static int act_mul_launch(const void* gu, void* out, int rows, int I, int blk, int dtype, cudaStream_t stream) {
   const long long n = (long long)rows * I;
   const int block = 256;
   const long long cap = (long long)fmx_num_sms() * 16;
   const int grid = (int)((n + block - 1) / block < cap ? (n + block - 1) / block : cap);
-  if (dtype == FMX_F32)
-    act_mul_kernel<float, KIND><<<grid, block, 0, stream>>>((const float*)gu, (float*)out, rows, I, blk);
-  else if (dtype == FMX_BF16) {
+  if (dtype == FMX_F32) {
+    if (I % 4 == 0 && blk % 4 == 0 && aligned16(gu) && aligned16(out) && rows <= 65535) {
+      const int bx = (I / 4 + block - 1) / block;
+      fmx_launch(act_mul_f32_vec_kernel<KIND>, dim3(bx < 64 ? bx : 64, rows), dim3(block), 0, stream, (const float*)gu, (float*)out, I, blk);
+    } else {
+      act_mul_kernel<float, KIND><<<grid, block, 0, stream>>>((const float*)gu, (float*)out, rows, I, blk);
+    }
+  } else if (dtype == FMX_BF16) {
     if (I % 8 == 0 && blk % 8 == 0 && aligned16(gu) && aligned16(out) && rows <= 65535) {
       const int bx = (I / 8 + block - 1) / block;
       fmx_launch(act_mul_bf16_vec_kernel<KIND>, dim3(bx < 64 ? bx : 64, rows), dim3(block), 0, stream, (const bf16*)gu,

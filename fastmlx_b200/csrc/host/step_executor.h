@@ -56,6 +56,7 @@ struct FmxOp {
   void* fn_attn_prefill_tc;
   void* fn_attn_plan;
   void* fn_attn_prefill_tc_plan;   // how many CTAs share the keys of a pair of query tiles
+  int terms;               // a 32-bit product over a bfloat16 matrix: the register of its input's three terms [rows, 3 k], bfloat16; -1: none
   int tc_attention_ok;     // sizes the tensor-memory attention kernel takes (head size, heads per kv head, page size, no window)
 };
 
@@ -73,6 +74,7 @@ struct FmxKernelTable {
   void* gemm_tcgen05;
   void* gemm_tcgen05_plan_fills;
   void* gemv_argmax;
+  void* gemm_three;
 };
 
 // One laid-out step: device pointers into the packed buffer, and the step's workspaces.

@@ -45,13 +45,13 @@ class FmxOp(Structure):
                 ("store", c_int), ("group", c_int), ("share_kv", c_int), ("kv", c_void_p), ("page_size", c_int),
                 ("num_pages", c_longlong), ("fn_attn_decode", c_void_p), ("fn_attn_prefill", c_void_p),
                 ("fn_attn_prefill_tc", c_void_p), ("fn_attn_plan", c_void_p), ("fn_attn_prefill_tc_plan", c_void_p),
-                ("tc_attention_ok", c_int)]
+                ("terms", c_int), ("tc_attention_ok", c_int)]
 
 
 class FmxKernelTable(Structure):
     _fields_ = [(n, c_void_p) for n in ("gather_rows", "gather_rows_f32_to_bf16", "add_rmsnorm", "silu_mul", "gemm_simple",
                                         "rope_kv_write", "paged_attention_simple", "fill_rows", "gemv", "gemm_tcgen05",
-                                        "gemm_tcgen05_plan_fills", "gemv_argmax")]
+                                        "gemm_tcgen05_plan_fills", "gemv_argmax", "gemm_three")]
 
 
 class FmxStepDesc(Structure):
@@ -158,11 +158,19 @@ class ProgramBuilder:
         self.keep.append(t)
         return t.data_ptr()
 
+    def terms(self, x: int, w) -> int:
+        """A register for the terms of a 32-bit product's input, where its matrix is held in bfloat16; else -1.  Released right after."""
+        if self.dtype_of(x) != F32 or w.dtype != torch.bfloat16:
+            return -1
+        r = self.reg(3 * w.shape[1], BF16)
+        self.release(r)
+        return r
+
     def op(self, kind: int, **fields) -> FmxOp:
         o = FmxOp()
         o.kind, o.in0, o.in1, o.out0, o.out1 = kind, -1, -1, -1, -1
         o.wanted_rows = 1 if self.wanted else 0
-        o.group = -1
+        o.group = o.terms = -1
         for name, value in fields.items():
             setattr(o, name, value)
         self.ops.append(o)
@@ -230,6 +238,8 @@ class NativeProgram:
             tc = _klib.load("tc")
             table.gemm_tcgen05 = _fn(tc, "fmx_gemm_tcgen05")
             table.gemm_tcgen05_plan_fills = _fn(tc, "fmx_gemm_tcgen05_plan_fills")
+        elif any(op.terms >= 0 for op in b.ops):       # matrices that the 32-bit path holds as they were stored
+            table.gemm_three = _fn(_klib.load("tc"), "fmx_gemm_three")
         self._ops = (FmxOp * len(b.ops))(*b.ops)
         self._regs = (FmxReg * len(b.regs))(*[FmxReg(c, d) for c, d in b.regs])
         self._blas_ws = torch.empty(self.CUBLAS_WORKSPACE, dtype=torch.uint8, device=rt.device)

@@ -179,7 +179,8 @@ def _status_word(device):
 #   M <= 16                    whole-K weight-streaming kernel (`gemv`), except the vocabulary-sized head
 #   M >= 128, full rounds      tcgen05 kernel (`gemm_tcgen05`)
 #   everything else in bf16    the library (cuBLAS through torch.mm), as tamnd/fastmlx calls its library's matmul
-#   32-bit or mixed types      fixed-order FMA kernel (`gemm_simple`)
+#   32-bit x, bfloat16 w       three-term tcgen05 kernel (`gemm_three`), whatever M: its sums do not depend on M
+#   other types                fixed-order FMA kernel (`gemm_simple`)
 GEMV_MAX_ROWS = 16
 LIBRARY_MIN_FEATURES = 65536     # from this many output features on (the vocabulary) the library's product streams best
 TC_MIN_ROWS = 128
@@ -314,11 +315,36 @@ def gemm_tcgen05(x, w, status=None, epilogue: int = EPI_PLAIN, residual=None, bn
     return out
 
 
+def holds_exactly(ws) -> bool:
+    """May the 32-bit path keep these matrices as the bfloat16 values they were stored as (`gemm_three` multiplies them exactly) instead
+    of widening them?  Rows of 16-byte pieces; finite, since an infinity would meet the zeros among an activation's terms."""
+    if not all(w.dtype == torch.bfloat16 and w.dim() == 2 and w.numel() > 0 and w.shape[1] % 8 == 0 for w in ws):
+        return False
+    ends = torch.stack([e for w in ws for e in torch.aminmax(w)])          # a NaN shows in both
+    return bool(torch.isfinite(ends).all())
+
+
+def gemm_three(x, w, bias=None, status=None) -> torch.Tensor:
+    """x[M, K] in 32-bit @ w[N, K]^T in bfloat16 (+ bias) -> 32-bit [M, N], to 32-bit accuracy on the tensor cores; a row's result
+    does not depend on the other rows."""
+    M, K = x.shape
+    N = w.shape[0]
+    out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    need = load("tc").fmx_gemm_three_bytes(M, K)
+    ws = torch.empty(need, dtype=torch.uint8, device=x.device)
+    call("tc", "fmx_gemm_three", x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), _ptr(bias), out.data_ptr(), out.stride(0),
+         M, N, K, ws.data_ptr(), num_sms(x.device), _ptr(status if status is not None else _status_word(x.device)), _stream())
+    return out
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, bias, out_dtype) -> torch.Tensor:
     """x[M, K] @ w[N, K]^T (+ bias) -> [M, N] in `out_dtype`, accumulated in 32-bit."""
     _need_cuda(x, w, bias)
     assert x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1], (x.shape, w.shape)
     assert x.stride(1) == 1 and w.stride(1) == 1
+    if (x.dtype == torch.float32 and w.dtype == torch.bfloat16 and out_dtype == torch.float32 and x.shape[1] % 8 == 0
+            and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0):
+        return gemm_three(x, w, bias)
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or x.shape[0] == 0:
         return gemm_simple(x, w, bias, out_dtype)
     if can_gemv(x, w) and (w.shape[0] < LIBRARY_MIN_FEATURES or bias is not None):

@@ -87,6 +87,7 @@ _SIGNATURES = {
         "fmx_moe_combine": [_P, _P, _P, _L, _I, _P, _L, _I, _I, _I, _I, _P],
     },
     "tc": {
+        "fmx_gemm_three": [_P, _L, _P, _L, _P, _P, _L, _I, _I, _I, _P, _I, _P, _P],
         "fmx_gemm_tcgen05": [_P, _L, _P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _P, _P],
         "fmx_grouped_act_tcgen05": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _P, _P],
         "fmx_grouped_down_tcgen05": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _P, _P, _P, _I, _P, _P],
@@ -163,6 +164,9 @@ def load(group: str) -> ctypes.CDLL:
     if group in ("tc", "tc_expiry"):
         lib.fmx_gemm_tcgen05_plan_width.argtypes = [_I, _I, _I]
         lib.fmx_gemm_tcgen05_plan_fills.argtypes = [_I, _I, _I]
+        lib.fmx_gemm_three_splits.argtypes = [_I, _I]
+        lib.fmx_gemm_three_bytes.argtypes = [_I, _I]
+        lib.fmx_gemm_three_bytes.restype = c_longlong
     if group == "chunks":
         lib.fmx_chunk_scan_bytes.argtypes = [_I, _I, _I, _I, _I, _I]
         lib.fmx_chunk_scan_bytes.restype = c_longlong

@@ -6,6 +6,17 @@ import torch
 from .base import FreeDim, Part, Runtime, WeightSpec, to_compute, to_f32_vector
 
 
+def exact_matrices(ws, rt: Runtime) -> list[torch.Tensor]:
+    """Matrices for a product: `to_compute`, but the 32-bit path keeps those that are all stored in bfloat16 as they are where its
+    product multiplies them exactly (`kernels.gemm_three`): half the bytes, and the tensor cores instead of 32-bit multiply-adds."""
+    ask = getattr(rt.k, "holds_exactly", None) if rt.is_fp32 else None
+    if ask is not None and all(w.dtype == torch.bfloat16 for w in ws):
+        held = [w.to(rt.device).contiguous() for w in ws]
+        if ask(held):
+            return held
+    return [to_compute(w, rt) for w in ws]
+
+
 class Linear(Part):
     """One or several checkpoint matrices applied as a single product: `names` lists
     (tensor name prefix, out features); their rows are stacked at bind time, so q/k/v or
@@ -37,7 +48,7 @@ class Linear(Part):
         return specs
 
     def bind_own(self, tensors, rt: Runtime):
-        ws = [to_compute(tensors[n + self.wsfx], rt) for n, _ in self.names]
+        ws = exact_matrices([tensors[n + self.wsfx] for n, _ in self.names], rt)
         if len({w.dtype for w in ws}) > 1:
             ws = [w.float() for w in ws]
         bs = [to_f32_vector(tensors[n + self.bsfx], rt) for n, _ in self.names] if self.has_bias else None
@@ -47,6 +58,8 @@ class Linear(Part):
             if bs is not None:
                 bs = [torch.stack([v.view(-1, b) for v in bs], dim=1).reshape(-1)]
         self.weight = ws[0].contiguous() if len(ws) == 1 else torch.cat(ws, dim=0).contiguous()
+        if self.weight.data_ptr() % 16:                # a view into a larger buffer: the products want rows on 16 bytes
+            self.weight = self.weight.clone()
         self.out_features = self.weight.shape[0]
         if bs is not None:
             self.bias = torch.cat(bs).contiguous()
@@ -64,7 +77,7 @@ class Linear(Part):
         if out is None:
             out = b.reg(self.out_features, dt)
         b.op(OP_LINEAR, in0=x, out0=out, w=b.ptr(self.weight), bias=b.ptr(self.bias), w_dtype=_dt(self.weight.dtype),
-             ldw=self.weight.stride(0), n=self.out_features, k=self.in_features, out_dtype=dt)
+             ldw=self.weight.stride(0), n=self.out_features, k=self.in_features, out_dtype=dt, terms=b.terms(x, self.weight))
         return out
 
 

@@ -86,7 +86,7 @@ class SwiGLU(FeedForward):
         both = b.reg(2 * self.intermediate)              # gate and up side by side, where no kernel fuses SiLU-mul in
         w = self.gate_up.weight
         b.op(OP_GATE_UP, in0=x, out0=act, out1=both, w=b.ptr(w), bias=b.ptr(self.gate_up.bias), w_dtype=_dt(w.dtype),
-             ldw=w.stride(0), n=2 * self.intermediate, k=self.width, block=self.block, out_dtype=b.act)
+             ldw=w.stride(0), n=2 * self.intermediate, k=self.width, block=self.block, out_dtype=b.act, terms=b.terms(x, w))
         b.release(both)
         out = self.down.emit(b, act)
         b.release(act)

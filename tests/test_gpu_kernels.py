@@ -1,5 +1,6 @@
 """Each CUDA kernel alone against its plain statement (tests/plain_ops.py), at sizes other
 than the engine's, in 32-bit and in bfloat16."""
+import math
 from types import SimpleNamespace
 
 import pytest
@@ -243,6 +244,41 @@ def test_gemm_simple_32bit_kernels_sum_in_one_order(M, N, K, bias):
     got = k().gemm_simple(x.to(DEV), w.to(DEV), b, torch.float32)
     assert torch.equal(got, k().gemm_simple(odd(x), odd(w), b, torch.float32))
     close(got, plain_ops.linear(x, w, None if b is None else b.cpu(), torch.float64), torch.float32, "gemm_simple", scale=None)
+
+
+@pytest.mark.parametrize("N,K,bias", [(1, 8, True), (127, 72, False), (129, 64, True), (200, 520, False), (130, 2056, True), (2048, 8192, False),
+                                      (16384, 256, False), (24000, 512, True)])
+def test_gemm_three_does_not_depend_on_the_batch(N, K, bias):
+    """32-bit rows against a bfloat16 matrix on the tensor cores: a row's result is the same bits whatever the number of rows (tiles of 16
+    to 128 tokens, K walked whole or in a cluster's shares), and as far from 64-bit as 32-bit sums are: up to 16 sums of the tensor cores
+    that are cut off, 2^-23 of what was summed each, and half of that for each rounded sum of the blocks of 64."""
+    x, w = torch.randn(300, K), rnd(N, K, dtype=torch.bfloat16, seed=11)
+    b = torch.randn(N).to(DEV) if bias else None
+    xd, wd = x.to(DEV), w.to(DEV)
+    full = k().linear(xd, wd, b, torch.float32)
+    ref = plain_ops.linear(x, w.float(), None if b is None else b.cpu(), torch.float64)
+    room = (x.abs().double() @ w.abs().double().t() + (0 if b is None else b.cpu().abs().double())) * 2.0 ** -23 * (16 + K / 128)
+    assert ((full.cpu().double() - ref).abs() <= room).all()
+    for a, m in ((0, 1), (0, 16), (5, 17), (100, 64), (7, 128), (40, 129), (3, 257)):
+        assert torch.equal(k().linear(xd[a:a + m], wd, b, torch.float32), full[a:a + m]), m
+    odd = torch.cat([x, x[:, :1]], 1).to(DEV)[:, :K]                       # rows that do not start on 16 bytes
+    assert torch.equal(k().linear(odd, wd, b, torch.float32), full)
+    assert int(k()._status_word(DEV)[0]) == 0
+
+
+def test_gemm_three_infinite_and_huge_activations():
+    """An infinity or a NaN stays in its row; values that would round to an infinity in bfloat16 do not."""
+    x, w = torch.randn(40, 192), rnd(70, 192, dtype=torch.bfloat16, seed=12)
+    x[3, 5], x[9, 0], x[17, 100] = math.inf, -math.inf, math.nan
+    x[21] *= 1e-3
+    x[21, 7] = 3.4e38
+    w[:, 7] = w[:, 7].abs().clamp(0.25, 0.5)
+    got = k().linear(x.to(DEV), w.to(DEV), None, torch.float32).cpu()
+    ref = x.double() @ w.double().t()
+    assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(torch.isinf(got), torch.isinf(ref))
+    assert torch.equal(got[[3, 9]].sign(), ref[[3, 9]].float().sign())
+    fin = torch.isfinite(ref)
+    assert ((got.double() - ref).abs()[fin] <= 2.0 ** -19 * (x.double().abs().nan_to_num(posinf=0) @ w.double().abs().t())[fin]).all()
 
 
 @pytest.mark.parametrize("ta,tw,tc", [(torch.bfloat16, torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32, torch.float32),
