@@ -39,11 +39,6 @@ constexpr size_t MIX_BYTES = 3 * 2 * 2 * 32 * 16; // M as left fragments: term, 
 constexpr size_t Q_BYTES = (size_t)HEADS * (MAXD / 16) * 3 * 32 * 8;            // Q as right fragments: head, 16 dimensions, term
 constexpr size_t SMEM = (size_t)3 * PTERM * 2 + Q_BYTES + (size_t)2 * KVH * TK * KLD * 2 + MIX_BYTES + HEADS * 4;
 
-__device__ __forceinline__ void ldmatrix4_trans(unsigned (&r)[4], const bf16* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
-}
-
 __device__ __forceinline__ float ex2_approx(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 
 // Places for the rows' tiles of 8 tokens: row r's first is row_start / 8 + r; rows do not overlap, whatever their lengths.

@@ -15,11 +15,11 @@
 // the result's norm: decays of 0.9 to 1 1.3e-7 either way, of 0.8 to 1 1.2e-7 here and 1.1e-7 there; plain write 1.1e-7 and 1.3e-7).
 // That walk is one chain of dependent steps of some 250 ns a token; a run of 32 tokens here takes 1.4 us at 64 rows of state, 3.3 us at 128.  One request of 2,048
 // tokens, 32 heads on 8 key heads, both kernels: delta rule 64 x 64 525 -> 120 us, 128 x 128 (two requests) 1,052 -> 232 us;
-// plain write 349 -> 104 and 665 -> 190 us; 1,777 tokens of five requests, 64 heads of 64 values over 128 rows 579 -> 184 us.
+// plain write 349 -> 112 (32 heads of keys of their own) and 665 -> 176 us (64 heads of 64 values over 128 rows); 1,777 tokens of five requests, 64 heads of 64 values over 128 rows 579 -> 172 us.
 //
 //   chunk_prepare  per (run, key group): k and q as three terms; k . k^T and q . k^T in 32-bit, and per head of the group
 //                  the decayed q . k^T and T, as three terms.  All runs at once.
-//   chunk_scan     per (request, head, 16 or 32 columns of S): the runs in order.
+//   chunk_delta, chunk_plain   per (request, head, 16 or 32 columns of S): the runs in order.
 //
 // An infinity or a NaN reaches what the walk lets it reach, its own token and the ones behind it (in its own column where a value holds
 // it), as a NaN: its second term is inf - inf.  A run that holds one sums over earlier tokens without the zeros of later ones (lower_sums).
@@ -53,7 +53,7 @@ chunk_prepare_kernel(const float* x, long long C, int qoff, int koff, const floa
   const int c = blockIdx.x, g = blockIdx.y, r = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float* mine = kkm + RUN * GRAM_LD + warp * RUN * GRAM_LD;      // a warp's matrix
-  pdl_wait();      // no early trigger: blocks of chunk_scan would sit on the shared memory that this kernel's blocks want
+  pdl_wait();      // no early trigger: blocks of the walk would sit on the shared memory that this kernel's blocks want
   const int first = row_start[r], n = row_start[r + 1] - first;
   if (c * RUN >= n || n < min_tokens) return;
   const int t0 = first + c * RUN, cnt = min(RUN, n - c * RUN);
@@ -159,13 +159,13 @@ chunk_prepare_kernel(const float* x, long long C, int qoff, int koff, const floa
   }
 }
 
-// Shared memory of chunk_scan: two stages of a run's operands, and what the four warps of 16 columns hand one another.
-template <int D, int MT, bool DELTA> struct ScanSmem {
+// Shared memory of chunk_delta: two stages of a run's operands, and what the four warps of 16 columns hand one another.
+template <int D, int MT> struct DeltaSmem {
   static constexpr int V_LD = 16 * MT + 4;                                // floats
-  static constexpr size_t STAGE = (size_t)(QK_SIZE<D> + PT_SIZE<DELTA>) * 2 + (size_t)RUN * V_LD * 4;
+  static constexpr size_t STAGE = (size_t)(QK_SIZE<D> + PT_SIZE<true>) * 2 + (size_t)RUN * V_LD * 4;
   static constexpr int S_WORDS = 3 * (D / 16) * 32 * 4;                   // 32-bit words of S^T's fragments, per 16 columns
   static constexpr int U_WORDS = 3 * (RUN / 16) * 32 * 4;                 // of R's, U's and E's
-  static constexpr size_t BYTES = 2 * STAGE + (size_t)MT * (S_WORDS + (DELTA ? 3 : 2) * U_WORDS) * 4;
+  static constexpr size_t BYTES = 2 * STAGE + (size_t)MT * (S_WORDS + 3 * U_WORDS) * 4;
 };
 
 // grid (columns / (16 MT), H, R), 128 MT + 32 threads: four warps per 16 columns, and one that copies.  S^T is kept as
@@ -175,12 +175,12 @@ template <int D, int MT, bool DELTA> struct ScanSmem {
 // memory as finished fragments.  Bound by the latency of that chain (four exchanges a run), not by a unit: hence 32 tokens
 // a run (64 take 1.2 times the products and 1.3 times the operands' bytes per token), four warps to share a link's
 // products, and copies that no link waits for.
-template <int D, int MT, bool DELTA>
+template <int D, int MT>
 __global__ void __launch_bounds__(128 * MT + 32)
-chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, int voff, const float* skip, const int* row_start,
+chunk_delta_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, int voff, const int* row_start,
                   const int* row_slot, float* state, long long slot_stride, float* out, int min_tokens, int H, int G, int P, int max_slots,
                   int lo, int hi) {
-  using Z = ScanSmem<D, MT, DELTA>;
+  using Z = DeltaSmem<D, MT>;
   constexpr int KT = D / 16, NS = D / 32;        // k-tiles of S; 8-row tiles of S^T per warp
   extern __shared__ __align__(16) unsigned char csm[];
   const int r = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * 16 * MT;
@@ -205,10 +205,10 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
 #pragma unroll 8
       for (int e = lane * 16; e < QK_SIZE<D> * 2; e += 512) cp16(dst + e, src + e, true);
       dst += QK_SIZE<D> * 2;
-      src = reinterpret_cast<const unsigned char*>(pt + ((run0 + c) * H + h) * PT_SIZE<DELTA>);
+      src = reinterpret_cast<const unsigned char*>(pt + ((run0 + c) * H + h) * PT_SIZE<true>);
 #pragma unroll 8
-      for (int e = lane * 16; e < PT_SIZE<DELTA> * 2; e += 512) cp16(dst + e, src + e, true);
-      float* dv = reinterpret_cast<float*>(dst + PT_SIZE<DELTA> * 2);
+      for (int e = lane * 16; e < PT_SIZE<true> * 2; e += 512) cp16(dst + e, src + e, true);
+      float* dv = reinterpret_cast<float*>(dst + PT_SIZE<true> * 2);
 #pragma unroll
       for (int e = lane; e < RUN * 4 * MT; e += 32) {
         const int t = e / (4 * MT), q = e % (4 * MT) * 4;
@@ -222,10 +222,9 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
     return;
   }
   unsigned* sfr = reinterpret_cast<unsigned*>(csm + 2 * Z::STAGE) + mt * Z::S_WORDS;
-  unsigned* ufr = reinterpret_cast<unsigned*>(csm + 2 * Z::STAGE) + MT * Z::S_WORDS + mt * (DELTA ? 3 : 2) * Z::U_WORDS;
+  unsigned* ufr = reinterpret_cast<unsigned*>(csm + 2 * Z::STAGE) + MT * Z::S_WORDS + mt * 3 * Z::U_WORDS;
   unsigned* efr = ufr + Z::U_WORDS;
   unsigned* rfr = efr + Z::U_WORDS;
-  const float sk = DELTA ? 0.f : skip[h];
   const int row = lane >> 2, two = (lane & 3) * 2;            // a thread's columns of S: row, row + 8; within a tile of 8: two, two + 1
   float* sp = state + (long long)slot * slot_stride + ((long long)h * P + c0 + mt * 16) * D + w * (D / 4);
   float S[NS][4];
@@ -273,36 +272,34 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
     const bf16* dq = reinterpret_cast<const bf16*>(csm + (c & 1) * Z::STAGE);
     const bf16* dk = dq + 3 * RUN * QK_LD<D>;
     const bf16* dp = dq + QK_SIZE<D>;
-    const float* ds = reinterpret_cast<const float*>(dp + (DELTA ? 2 : 1) * PLANE);
+    const float* ds = reinterpret_cast<const float*>(dp + 2 * PLANE);
     const float* dv = ds + 2 * RUN + mt * 16;
     const float A0 = ds[t0], A1 = ds[t0 + 1], E0 = ds[RUN + t0], E1 = ds[RUN + t0 + 1], last = ds[RUN - 1];
     float v[4] = {dv[t0 * Z::V_LD + row], dv[(t0 + 1) * Z::V_LD + row], dv[t0 * Z::V_LD + row + 8], dv[(t0 + 1) * Z::V_LD + row + 8]};
-    const float x0 = v[0], x1 = v[1], x2 = v[2], x3 = v[3];
     // what the state in front of the run gives these 8 tokens: S^T q, and S^T k for the delta rule; side by side, so that one's
     // chains of products fill the other's waits
     Sums o, kS;
     o.zero();
     kS.zero();
-    auto read_out = [&]() {
+    {
 #pragma unroll
       for (int k2 = 0; k2 < KT / 2; ++k2) {
         unsigned bq[3][4], bk[3][4];
 #pragma unroll
         for (int t = 0; t < 3; ++t) {
-          if (DELTA) ldmatrix4(bk[t], dk + (t * RUN + rows8) * QK_LD<D> + k2 * 32 + quarter);
+          ldmatrix4(bk[t], dk + (t * RUN + rows8) * QK_LD<D> + k2 * 32 + quarter);
           ldmatrix4(bq[t], dq + (t * RUN + rows8) * QK_LD<D> + k2 * 32 + quarter);
         }
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk) {
           unsigned a[3][4];
           fragment(a, sfr, KT, k2 * 2 + kk);
-          if (DELTA) kS.add(a, bk, kk * 2);
+          kS.add(a, bk, kk * 2);
           o.add(a, bq, kk * 2);
         }
       }
-    };
-    if (DELTA) read_out();
-    if (DELTA) {                                  // u = T diag(beta) (v - A (S^T k))
+    }
+    {                                             // u = T diag(beta) (v - A (S^T k))
       unsigned bt[3][4];
 #pragma unroll
       for (int t = 0; t < 3; ++t) ldmatrix4(bt[t], dp + PLANE + (t * RUN + rows8) * PT_LD + quarter);
@@ -327,7 +324,6 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
     share_tile(ufr, v);
     v[0] *= E0; v[1] *= E1; v[2] *= E0; v[3] *= E1;
     share_tile(efr, v);
-    if (!DELTA) read_out();                       // behind the tiles that the others wait for
     const bool odd = meet_any(1 + mt, mine);
     // S <- A_32 S + sum_s (E_s u_s) k_s^T for this warp's rows of state, and what the run's own tokens give: the decayed
     // q . k^T times u
@@ -365,10 +361,6 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
     if (odd) lower_sums(res, dp, ufr, t0, row);
 #pragma unroll
     for (int i = 0; i < 4; ++i) res[i] = fmaf(i & 1 ? A1 : A0, o.at(i), res[i]);
-    if (!DELTA) {
-      res[0] = fmaf(sk, x0, res[0]); res[1] = fmaf(sk, x1, res[1]);
-      res[2] = fmaf(sk, x2, res[2]); res[3] = fmaf(sk, x3, res[3]);
-    }
     if (t < n) {
       op[(long long)t * ostride + row] = res[0];
       op[(long long)t * ostride + row + 8] = res[2];
@@ -383,6 +375,124 @@ chunk_scan_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, i
     *reinterpret_cast<float2*>(sp + (long long)row * D + j * 8 + two) = make_float2(S[j][0], S[j][1]);
     *reinterpret_cast<float2*>(sp + (long long)(row + 8) * D + j * 8 + two) = make_float2(S[j][2], S[j][3]);
   }
+}
+
+// Shared memory of chunk_plain: stages of a run's operands, and what the four warps of 16 columns hand one another: their shares of S^T q,
+// and U and E as fragments.
+template <int D, int MT> struct PlainSmem {
+  static constexpr int V_LD = 16 * MT + 4;                                // floats
+  static constexpr size_t STAGE = (size_t)(QK_SIZE<D> + PT_SIZE<false>) * 2 + (size_t)RUN * V_LD * 4;
+  static constexpr int MEET = 4 * RED * 4 + 2 * LEFT_WORDS;               // 32-bit words per 16 columns
+  static constexpr size_t bytes(int stages) { return stages * STAGE + (size_t)MT * MEET * 4; }
+};
+
+// The same without the delta rule, whose u is at hand before the run: nothing on the state's own chain crosses warps, so each warp keeps its
+// quarter of the state's rows to itself (RunWarp).  Four warps copy, two stages of operands or three.  Bound by `mma.sync`, of which a
+// scheduler takes one in some 15 clocks here (105 a warp and run of 128 rows).  With the state shared as fragments and one copying
+// warp, which everything waited for: 1,777 tokens of five requests, 64 heads of 64 values over 128 rows 153 us, 138 here; 1,531 tokens of a
+// retention with 32 heads of 64 x 64 77 and 51.  For the delta rule the meeting of the quarters stands on the chain: 92 us that way, 95 this.
+template <int D, int MT>
+__global__ void __launch_bounds__(128 * MT + COPY_THREADS<D>)
+chunk_plain_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, int voff, const float* skip, const int* row_start,
+                  const int* row_slot, float* state, long long slot_stride, float* out, int min_tokens, int H, int G, int P, int max_slots,
+                  int lo, int hi, int stages) {
+  using Z = PlainSmem<D, MT>;
+  constexpr int KT = D / 16, NS = D / 32;        // k-tiles of S; 8-row tiles of S^T per warp
+  extern __shared__ __align__(16) unsigned char csm[];
+  const int r = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * 16 * MT;
+  const int tid = threadIdx.x, lane = tid & 31, mt = tid >> 7, w = tid >> 5 & 3;
+  pdl_wait();
+  pdl_trigger();
+  const int slot = row_slot[r];
+  if (slot < 0 || slot >= max_slots) return;
+  const int first = row_start[r], n = row_start[r + 1] - first;
+  if (n < min_tokens) return;                    // walked token by token in a launch of its own
+  const int place = first_run(first, r), g = h / (H / G);
+  const int c_lo = max(0, lo - place), c_hi = min((n + RUN - 1) / RUN, hi - place);        // the row's runs of this wave
+  if (c_lo >= c_hi) return;
+  const long long run0 = place - lo;             // (of the row's first run, which may lie in front of the workspace)
+  if (tid >= 128 * MT) {                       // the copying warps: a run's operands land while the runs before it are walked
+    const int at = tid - 128 * MT;
+    auto copy = [&](int c) {
+      if (c < c_hi) {
+        unsigned char* dst = csm + (c - c_lo) % stages * Z::STAGE;
+        copy_bytes<QK_SIZE<D> * 2, COPY_THREADS<D>>(dst, reinterpret_cast<const unsigned char*>(qk + ((run0 + c) * G + g) * QK_SIZE<D>), at);
+        dst += QK_SIZE<D> * 2;
+        copy_bytes<PT_SIZE<false> * 2, COPY_THREADS<D>>(dst, reinterpret_cast<const unsigned char*>(pt + ((run0 + c) * H + h) * PT_SIZE<false>), at);
+        float* dv = reinterpret_cast<float*>(dst + PT_SIZE<false> * 2);
+#pragma unroll
+        for (int e = at; e < RUN * 4 * MT; e += COPY_THREADS<D>) {
+          const int t = e / (4 * MT), q = e % (4 * MT) * 4;
+          const bool there = c * RUN + t < n;
+          copy16(dv + t * Z::V_LD + q, x + (long long)(first + (there ? c * RUN + t : 0)) * C + voff + (long long)h * P + c0 + q, there);
+        }
+      }
+      asm volatile("cp.async.commit_group;\n" ::);
+    };
+    for (int i = 0; i < stages - 1; ++i) copy(c_lo + i);
+    for (int c = c_lo; c < c_hi; ++c) {
+      if (stages == 3) asm volatile("cp.async.wait_group 1;\n" ::);
+      else asm volatile("cp.async.wait_group 0;\n" ::);
+      __syncthreads();                           // run c is there; run c - 1 has been walked, and its stage is free
+      copy(c + stages - 1);
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    return;
+  }
+  float4* red_q = reinterpret_cast<float4*>(csm + stages * Z::STAGE) + mt * (Z::MEET / 4);
+  unsigned* ufr = reinterpret_cast<unsigned*>(red_q + 4 * RED);
+  unsigned* efr = ufr + LEFT_WORDS;
+  RunWarp<D> me;
+  me.lane = lane; me.w = w; me.row = lane >> 2; me.two = (lane & 3) * 2;
+  float* sp = state + (long long)slot * slot_stride + ((long long)h * P + c0 + mt * 16) * D + w * (D / 4);
+  me.load(sp);
+  me.terms();
+  const float sk = skip[h];
+  const long long ostride = (long long)H * P;
+  float* op = out + (long long)first * ostride + (long long)h * P + c0 + mt * 16;
+  const int row = me.row, t0 = w * 8 + me.two;   // this thread's tokens of a run: t0, t0 + 1
+  for (int c = c_lo; c < c_hi; ++c) {
+    __syncthreads();                             // the run's operands are there; what the last run put down has been read
+    const bf16* dq = reinterpret_cast<const bf16*>(csm + (c - c_lo) % stages * Z::STAGE);
+    const bf16* dk = dq + 3 * RUN * QK_LD<D>;
+    const bf16* dp = dq + QK_SIZE<D>;
+    const float* ds = reinterpret_cast<const float*>(dp + PLANE);
+    const float* dv = ds + 2 * RUN + mt * 16;
+    const float A0 = ds[t0], A1 = ds[t0 + 1], E0 = ds[RUN + t0], E1 = ds[RUN + t0 + 1], last = ds[RUN - 1];
+    float v[4], e[4], o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = dv[(t0 + (i & 1)) * Z::V_LD + row + 8 * (i >> 1)];
+    const bool mine = not_finite(v);
+    me.share(ufr, v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) e[i] = v[i] * (i & 1 ? E1 : E0);
+    me.share(efr, e);
+    me.against(dq, red_q);
+    const bool odd = meet_any(1 + mt, mine);
+    // S <- A_32 S + sum_s (E_s u_s) k_s^T for this warp's rows of state
+    me.add(dk, efr, [&](int) { return make_float2(last, last); });
+    me.terms();
+    me.gather(o, red_q);
+    // and what the run's own tokens give: the decayed q . k^T times u
+    const int t = c * RUN + t0;
+    float res[4];
+    me.lower(res, dp, ufr);
+    if (odd) lower_sums(res, dp, ufr, t0, row);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      res[i] = fmaf(i & 1 ? A1 : A0, o[i], res[i]);
+      res[i] = fmaf(sk, v[i], res[i]);
+    }
+    if (t < n) {
+      op[(long long)t * ostride + row] = res[0];
+      op[(long long)t * ostride + row + 8] = res[2];
+    }
+    if (t + 1 < n) {
+      op[(long long)(t + 1) * ostride + row] = res[1];
+      op[(long long)(t + 1) * ostride + row + 8] = res[3];
+    }
+  }
+  me.store(sp);
 }
 
 struct Args {
@@ -405,6 +515,24 @@ long long place_bytes(int H, int G, int D, bool delta) {
                  : (delta ? bytes_of<128, true>(H, G) : bytes_of<128, false>(H, G));
 }
 
+template <int D, int MT, bool DELTA> void walk(const Args& a, const bf16* qk, const bf16* pt, int lo, int hi, cudaStream_t stream) {
+  const dim3 grid(a.P / (16 * MT), a.H, a.R);
+  if constexpr (DELTA) {
+    constexpr size_t smem = DeltaSmem<D, MT>::BYTES;
+    raise_shared<chunk_delta_kernel<D, MT>>(smem);
+    fmx_launch(chunk_delta_kernel<D, MT>, grid, dim3(128 * MT + 32), smem, stream, qk, pt, a.x, a.C, a.voff, a.row_start, a.row_slot, a.state,
+               a.slot_stride, a.out, a.min_tokens, a.H, a.G, a.P, a.max_slots, lo, hi);
+  } else {
+    // three stages where a block has an SM to itself anyway
+    using Z = PlainSmem<D, MT>;
+    constexpr size_t most = Z::bytes(3) <= 227 * 1024 ? Z::bytes(3) : Z::bytes(2);
+    const int stages = most > Z::bytes(2) && (long long)grid.x * a.H * a.R <= fmx_num_sms() ? 3 : 2;
+    raise_shared<chunk_plain_kernel<D, MT>>(most);
+    fmx_launch(chunk_plain_kernel<D, MT>, grid, dim3(128 * MT + COPY_THREADS<D>), Z::bytes(stages), stream, qk, pt, a.x, a.C, a.voff, a.skip, a.row_start,
+               a.row_slot, a.state, a.slot_stride, a.out, a.min_tokens, a.H, a.G, a.P, a.max_slots, lo, hi, stages);
+  }
+}
+
 // The step's runs in waves of `wave` places, whose operands the workspace holds; a state passes from wave to wave in its slot.
 template <int D, bool DELTA> int launch(const Args& a, int wave, cudaStream_t stream) {
   bf16* qk = reinterpret_cast<bf16*>(a.ws);
@@ -420,17 +548,8 @@ template <int D, bool DELTA> int launch(const Args& a, int wave, cudaStream_t st
     const int lo = (int)at, hi = (int)(at + wave < places ? at + wave : places);
     fmx_launch(chunk_prepare_kernel<D, DELTA>, dim3((a.max_q + RUN - 1) / RUN, a.G, a.R), dim3(32 * PREP_WARPS<D>), prep, stream, a.x, a.C, a.qoff,
                a.koff, a.decay, a.weight, 2 * a.H, a.row_start, a.min_tokens, a.H, a.G, qk, pt, lo, hi);
-#define FMX_SCAN(MT)                                                                                                         \
-  do {                                                                                                                       \
-    constexpr size_t smem = ScanSmem<D, MT, DELTA>::BYTES;                                                                   \
-    raise_shared<chunk_scan_kernel<D, MT, DELTA>>(smem);                                                                     \
-    fmx_launch(chunk_scan_kernel<D, MT, DELTA>, dim3(a.P / (16 * MT), a.H, a.R), dim3(128 * MT + 32), smem, stream, (const bf16*)qk, \
-               (const bf16*)pt, a.x, a.C, a.voff, a.skip, a.row_start, a.row_slot, a.state, a.slot_stride, a.out, a.min_tokens, a.H, a.G, \
-               a.P, a.max_slots, lo, hi);                                                                                    \
-  } while (0)
-    if (pair) FMX_SCAN(2);
-    else FMX_SCAN(1);
-#undef FMX_SCAN
+    if (pair) walk<D, 2, DELTA>(a, qk, pt, lo, hi, stream);
+    else walk<D, 1, DELTA>(a, qk, pt, lo, hi, stream);
   }
   FMX_LAUNCH_CHECK();
   return 0;

@@ -17,8 +17,8 @@
 //
 // The operands of a run and head are 57 KB (64 rows of state) or 94 KB (128), so a step's runs go in waves whose workspace is
 // bounded.  An infinity or a NaN reaches what it reaches in chunk_scan.cu.
-// 32 heads on 8 key heads of 128 x 128, 2,048 tokens: one request 754 us token by token and 379 here, two of 768 and 1,280 637 and 380
-// (of which 150 to prepare and 227 for the runs).  64 x 64, one request: 387 and 249; without the delta rule 265 and 204, while 128 x 128
+// 32 heads on 8 key heads of 128 x 128, 2,048 tokens: one request 754 us token by token and 342 here, two of 768 and 1,280 637 and 352
+// (of which 150 to prepare and 199 for the runs).  64 x 64, one request: 387 and 249; without the delta rule 265 and 204, while 128 x 128
 // takes 308 either way and stays with the walk.  Against 64-bit: 1.3e-7 of the result's norm, 1.4e-7 token by token.
 #include <math.h>
 #include "runs.cuh"
@@ -193,10 +193,15 @@ template <int D, int MT, bool DELTA> struct ChannelSmem {
   static constexpr size_t BYTES = FRONT_BYTES + BACK_BYTES + (size_t)MT * (S_WORDS + (DELTA ? 2 : 1) * U_WORDS) * 4;
 };
 
-// As chunk_scan_kernel (four warps per 16 columns, one that copies), but a run's operands are twice as many bytes: one buffer for what
+// Threads that copy: with 128 rows of state, whose block fills an SM, four warps, since everything waits for the copies (two prompts of 768 and
+// 1,280 tokens, 32 heads: 227 us with one, 199 with four); with 64 rows the registers of a second warp cost more than it brings (three requests of
+// 512 tokens 114 and 140 us).
+template <int D> constexpr int CHANNEL_COPY = D > 64 ? 128 : 32;
+
+// As chunk_delta_kernel (four warps per 16 columns, others that copy), but a run's operands are twice as many bytes: one buffer for what
 // the state is multiplied with in front and one for what comes after, each filled while the other one is in use.
 template <int D, int MT, bool DELTA>
-__global__ void __launch_bounds__(128 * MT + 32)
+__global__ void __launch_bounds__(128 * MT + CHANNEL_COPY<D>)
 channel_chunks_kernel(ChannelArgs a) {
   using Z = ChannelSmem<D, MT, DELTA>;
   constexpr int KT = D / 16, NS = D / 32, QK_LD = K_LD<D>;
@@ -216,10 +221,8 @@ channel_chunks_kernel(ChannelArgs a) {
   bf16* fr = reinterpret_cast<bf16*>(csm);
   float* dv = reinterpret_cast<float*>(fr + FRONT<D, DELTA>);
   bf16* bk = reinterpret_cast<bf16*>(csm + Z::FRONT_BYTES);
-  if (tid >= 128 * MT) {                       // the copying warp
-    auto cp16 = [](void* dst, const void* src, bool there) {
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0));
-    };
+  if (tid >= 128 * MT) {                       // the copying warps
+    const int at = CHANNEL_COPY<D> == 32 ? lane : tid - 128 * MT;
     auto landed = []() {
       asm volatile("cp.async.commit_group;\n" ::);
       asm volatile("cp.async.wait_group 0;\n" ::);
@@ -227,19 +230,16 @@ channel_chunks_kernel(ChannelArgs a) {
     const float* vp = a.qkv + 2LL * a.G * D + (long long)h * a.P + c0;
     for (int c = lo; c < hi; ++c) {
       const unsigned char* src = reinterpret_cast<const unsigned char*>(a.ws + ((long long)(base + c - a.lo) * a.H + h) * (FRONT<D, DELTA> + BACK<D, DELTA>));
-#pragma unroll 8
-      for (int e = lane * 16; e < FRONT<D, DELTA> * 2; e += 512) cp16(csm + e, src + e, true);
+      copy_bytes<FRONT<D, DELTA> * 2, CHANNEL_COPY<D>>(csm, src, at);
 #pragma unroll
-      for (int e = lane; e < RUN * 4 * MT; e += 32) {
+      for (int e = at; e < RUN * 4 * MT; e += CHANNEL_COPY<D>) {
         const int t = e / (4 * MT), q = e % (4 * MT) * 4;
         const bool there = c * RUN + t < n;
-        cp16(dv + t * Z::V_LD + q, vp + (long long)(first + (there ? c * RUN + t : 0)) * C + q, there);
+        copy16(dv + t * Z::V_LD + q, vp + (long long)(first + (there ? c * RUN + t : 0)) * C + q, there);
       }
       landed();
       __syncthreads();                         // (1) run c's front is there, the back of run c - 1 has been read
-      src += FRONT<D, DELTA> * 2;
-#pragma unroll 8
-      for (int e = lane * 16; e < BACK<D, DELTA> * 2; e += 512) cp16(csm + Z::FRONT_BYTES + e, src + e, true);
+      copy_bytes<BACK<D, DELTA> * 2, CHANNEL_COPY<D>>(csm + Z::FRONT_BYTES, src + FRONT<D, DELTA> * 2, at);
       landed();
       __syncthreads_or(0);                     // (2) its back is there, its front has been read
     }
@@ -406,11 +406,11 @@ template <int D, bool DELTA> int launch(ChannelArgs a, int places, int per_wave,
     if (pair) {
       constexpr size_t smem = ChannelSmem<D, 2, DELTA>::BYTES;
       raise_shared<channel_chunks_kernel<D, 2, DELTA>>(smem);
-      fmx_launch(channel_chunks_kernel<D, 2, DELTA>, dim3(a.P / 32, a.H, a.R), dim3(288), smem, stream, a);
+      fmx_launch(channel_chunks_kernel<D, 2, DELTA>, dim3(a.P / 32, a.H, a.R), dim3(256 + CHANNEL_COPY<D>), smem, stream, a);
     } else {
       constexpr size_t smem = ChannelSmem<D, 1, DELTA>::BYTES;
       raise_shared<channel_chunks_kernel<D, 1, DELTA>>(smem);
-      fmx_launch(channel_chunks_kernel<D, 1, DELTA>, dim3(a.P / 16, a.H, a.R), dim3(160), smem, stream, a);
+      fmx_launch(channel_chunks_kernel<D, 1, DELTA>, dim3(a.P / 16, a.H, a.R), dim3(128 + CHANNEL_COPY<D>), smem, stream, a);
     }
   }
   FMX_LAUNCH_CHECK();

@@ -30,6 +30,10 @@ __device__ __forceinline__ void ldmatrix2_trans(unsigned (&r)[2], const bf16* p)
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
                : "=r"(r[0]), "=r"(r[1]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
 }
+__device__ __forceinline__ void ldmatrix4_trans(unsigned (&r)[4], const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+}
 
 // A 16 x 8 tile of sums, kept apart by size of the terms: chains of dependent products that do not wait for one another.
 // Products of the leading terms are added up in rounded 32-bit sums: the tensor cores' own sums cut off, and of
@@ -54,4 +58,46 @@ struct Sums {
   }
   __device__ __forceinline__ float at(int i) const { return big[i] + (middle[i] + small[i]); }
 };
+
+// The six products of terms of `tiles` tiles of 16 of the contraction, for N right operands side by side: c[n] = a . b[n], both in three
+// terms (tile k's registers of b: b[n][term][2 k], b[n][term][2 k + 1]).  The tensor cores cut their sums off instead of rounding them,
+// and of the leading terms' products that would be seen: those of each tile are a sum of their own, added up rounded; the small terms'
+// products are CHAINS sums.  A product that waits for the one before it takes 30 clocks, one that does not 15: hence the sums side
+// by side, and the steps over all N at a time.
+template <int KT, int CHAINS, int N, int NB>
+__device__ __forceinline__ void products(float (&c)[N][4], const unsigned (&a)[KT][3][4], const unsigned (&b)[N][3][NB], int tiles = KT) {
+  constexpr int TA[5] = {2, 0, 1, 1, 0}, TB[5] = {0, 2, 1, 0, 1};
+  float big[KT][N][4], low[CHAINS][N][4];
+#pragma unroll
+  for (int n = 0; n < N; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int k = 0; k < KT; ++k) big[k][n][i] = 0.f;
+#pragma unroll
+      for (int x = 0; x < CHAINS; ++x) low[x][n][i] = 0.f;
+    }
+#pragma unroll
+  for (int s = 0; s < 5; ++s) {
+#pragma unroll
+    for (int k = 0; k < KT; ++k)
+      if (k < tiles)
+#pragma unroll
+        for (int n = 0; n < N; ++n) mma16816(low[k % CHAINS][n], a[k][TA[s]], b[n][TB[s]][2 * k], b[n][TB[s]][2 * k + 1]);
+    if (s < KT && s < tiles)
+#pragma unroll
+      for (int n = 0; n < N; ++n) mma16816(big[s % KT][n], a[s % KT][0], b[n][0][2 * (s % KT)], b[n][0][2 * (s % KT) + 1]);
+  }
+#pragma unroll
+  for (int n = 0; n < N; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float l = low[0][n][i], h = big[0][n][i];
+#pragma unroll
+      for (int x = 1; x < CHAINS; ++x) l += low[x][n][i];
+#pragma unroll
+      for (int k = 1; k < KT; ++k) h += big[k][n][i];
+      c[n][i] = h + l;
+    }
+}
 }  // namespace
