@@ -514,10 +514,32 @@ def wide_library(hd: int, vd: int) -> str:
     return f"attn_hd{hd}" if hd == vd else f"attn_hd{hd}_vd{vd}"
 
 
+def wide_tc_ok(kv, nh: int, nkv: int, hd: int, vd: int, scale: float, keep_first: int = 0, chunk: int = 0, sinks=None) -> bool:
+    """Layers that the kernel with two-term products on tensor memory takes: pages of keys and values of 64 or 128, at most 16 query
+    heads per kv head, a page size of at least 8 that divides its tile of 64 keys, a positive scale; a window or none."""
+    return (hd == vd and hd in (64, 128) and kv.dim() == 5 and kv.shape[1] == 2 and kv.is_contiguous() and kv.data_ptr() % 16 == 0 and nh // nkv <= 16
+            and kv.shape[3] >= 8 and 64 % kv.shape[3] == 0 and kv.shape[0] * 2 * nkv * kv.shape[3] < 2 ** 31 - 1
+            and scale > 0.0 and not keep_first and not chunk and sinks is None)
+
+
+# Keys from which on the tensor-memory kernel with two-term products is ahead of the `mma.sync` one, by the longest context after the step:
+# its start costs more than a short row's tiles (32 heads on 8, us, `mma.sync` and here: head size 64, 64 keys 7.2 and 8.7, 256 13.8 and 11.8;
+# head size 128, 256 keys 16.9 and 19.5, 512 31 and 26).
+WIDE_TC_KEYS = {64: 192, 128: 384}
+
+
 def _wide_launch(q, kv, ctx, group, nh, nkv, hd, scale, softcap, window, out, first_token: int = 0, splits: int = 1,
-                 keep_first: int = 0, chunk: int = 0, sinks=None, vd: int = 0) -> None:
+                 keep_first: int = 0, chunk: int = 0, sinks=None, vd: int = 0, tc: bool | None = None) -> None:
     vd = vd or hd
     bt = group.block_tables
+    if tc is None:
+        tc = (splits == 1 and ctx.max_q_len > 1 and wide_tc_ok(kv, nh, nkv, hd, vd, scale, keep_first, chunk, sinks)
+              and getattr(ctx, "max_ctx_after", 0) >= WIDE_TC_KEYS[hd])
+    if tc:
+        call(f"attn_hd{hd}", "fmx_attn_wide_tc", q.data_ptr(), q.stride(0), kv.data_ptr(), bt.data_ptr(), bt.stride(0), ctx.row_start.data_ptr(),
+             ctx.row_ctx.data_ptr(), ctx.positions.data_ptr(), out.data_ptr(), out.stride(0), ctx.R, int(ctx.max_q_len), nh, nkv, kv.shape[3],
+             kv.shape[0], float(scale), float(softcap or 0.0), int(window), _ptr(ctx.status), _stream())
+        return
     page_size = kv.shape[3] if kv.dim() == 5 else kv.shape[1] // (nkv * (hd + vd))
     scratch = None
     n_tokens = ctx.R

@@ -974,6 +974,60 @@ def test_values_that_are_not_finite_in_runs_of_tokens(form, D, P, what):
     assert torch.isfinite(o[1][:37]).all() and not torch.isfinite(o[1]).all()
 
 
+@pytest.mark.parametrize("lens,ctxs,nh,nkv,hd,page,window,cap,loud", [
+    ((64,), (0,), 32, 8, 64, 16, 0, 0.0, 1), ((300, 77, 1, 129), (0, 700, 40, 1033), 32, 8, 64, 16, 100, 30.0, 1),
+    ((200, 130), (1500, 0), 12, 4, 64, 8, 200, 5.0, 5), ((33, 65), (7, 130), 6, 2, 64, 64, 17, 0.0, 1), ((70,), (500,), 16, 1, 128, 16, 64, 0.0, 1),
+    ((200, 64), (300, 0), 32, 4, 128, 32, 0, 50.0, 3), ((2, 31), (63, 64), 8, 8, 128, 64, 150, 30.0, 20)])
+def test_two_term_attention_on_tensor_memory(lens, ctxs, nh, nkv, hd, page, window, cap, loud):
+    """Portions with 32-bit queries on tensor memory against 64-bit and beside the `mma.sync` kernel: tiles of tokens and keys with remainders,
+    heads that do not fill a tile's rows, pages behind a window given back, unused places that hold NaN, caps that serve as the
+    weights' scale and one that does not, scores beyond the short tangent, output rows that do not start on 16 bytes."""
+    torch.manual_seed(nh + hd)
+    R, starts = len(lens), [0] + list(torch.tensor(lens).cumsum(0).tolist())
+    T, blocks = starts[-1], [-(-(c + n) // page) for c, n in zip(ctxs, lens)]
+    perm, bt = torch.randperm(sum(blocks) + 3).tolist(), torch.full((R, max(blocks) + 1), -1, dtype=torch.int32)
+    kv = torch.full((sum(blocks) + 3, 2, nkv, page, hd), float("nan")).bfloat16()
+    K, V = ([torch.randn(c + n, nkv, hd).bfloat16() for c, n in zip(ctxs, lens)] for _ in range(2))
+    for r in range(R):
+        for b in range(blocks[r]):
+            if window and (b + 1) * page <= ctxs[r] - window + 1:
+                continue                              # given back
+            p = bt[r, b] = perm.pop()
+            for i, x in enumerate((K[r], V[r])):
+                x = x[b * page:(b + 1) * page]
+                kv[p, i, :, :len(x)] = x.transpose(0, 1)
+    q = torch.randn(T, nh * hd) * loud
+    pos = torch.cat([torch.arange(c, c + n) for c, n in zip(ctxs, lens)])
+    ints = lambda x: torch.as_tensor(x, dtype=torch.int32, device=DEV)
+    ctx = SimpleNamespace(R=R, T=T, positions=ints(pos), row_start=ints(starts), row_ctx=ints(ctxs), max_q_len=max(lens), status=ints([0] * 4))
+    kvd, qd, grp = kv.to(DEV), q.to(DEV), SimpleNamespace(block_tables=bt.to(DEV))
+    assert k().wide_tc_ok(kvd, nh, nkv, hd, hd, hd ** -0.5)
+    outs = []
+    for tc in (False, True):
+        wide = torch.zeros(T, nh * hd + 2, dtype=torch.bfloat16, device=DEV)
+        k()._wide_launch(qd, kvd, ctx, grp, nh, nkv, hd, hd ** -0.5, cap, window, wide[:, 2:], tc=tc)
+        outs.append(wide[:, 2:].cpu().double())
+    assert ctx.status.tolist() == [0] * 4
+    errs = [0.0, 0.0]
+    for r in range(R):
+        at, p = slice(starts[r], starts[r + 1]), torch.arange(ctxs[r], ctxs[r] + lens[r])
+        k_, v_ = (x[r].double().repeat_interleave(nh // nkv, 1) for x in (K, V))
+        qq = q[at].double().view(-1, nh, hd)
+        s = torch.einsum("qhd,khd->hqk", qq, k_) * hd ** -0.5
+        back = p[:, None] - torch.arange(len(k_))[None]
+        hidden = (back < 0) | ((back >= window) if window else False)
+        w = torch.softmax((cap * torch.tanh(s / cap) if cap else s).masked_fill(hidden, -float("inf")), -1)
+        want = torch.einsum("hqk,khd->qhd", w, v_).flatten(1)
+        size = torch.einsum("hqk,khd->qhd", w, v_.abs())
+        # operands of two terms are off by 2^-17: a weight, and by the queries a score, by 2^-17 of its products' sizes, which moves a weight by
+        # twice that; and the rounding to bfloat16
+        products = (torch.einsum("qhd,khd->hqk", qq.abs(), k_.abs()) * hd ** -0.5).masked_fill(hidden, 0.0).amax(-1).T[:, :, None]
+        room = 2.0 ** -8 * want.abs() + (2.0 ** -17 * (2 + 2 * products) * size).flatten(1)
+        assert ((outs[1][at] - want).abs() <= room).all()
+        errs = [e + ((o[at] - want) ** 2).sum().item() for e, o in zip(errs, outs)]
+    assert errs[1] <= 1.02 * errs[0]
+
+
 @pytest.mark.parametrize("weights", ["softmax", "sigmoid"])
 @pytest.mark.parametrize("window", [0, 20])
 def test_capped_scores_do_not_depend_on_later_keys(weights, window):
