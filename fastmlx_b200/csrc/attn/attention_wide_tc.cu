@@ -93,9 +93,6 @@ __device__ __forceinline__ f32x2 tanh_short(f32x2 y) {
   p = fma2(q, p, both(-0.33333272f));
   return fma2(mul2(y, q), p, y);
 }
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { f32x2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ void halves(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 __device__ __forceinline__ float tanh_any(float y) { return fabsf(y) <= TANH_SMALL ? tanh_short(y) : tanhf(y); }
 // Caps up to this: a score lies within cap of the largest possible one, exp(-2 cap) is far inside the range of 32-bit numbers and of bfloat16,
 // and the weights need no maximum: their scale is that of the cap itself.

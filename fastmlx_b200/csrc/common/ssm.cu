@@ -279,6 +279,78 @@ ssm_scan_kernel(const float* xbc, const float* dd, const float* __restrict__ d_s
   }
 }
 
+// Steps of one token a row: the walk's arithmetic, sum for sum, but everything a lane needs (CPT columns' shares, B, C) is asked for at once,
+// from memory into registers, as in the gated delta rule's step.  Measured (64 rows, states from memory): 48 heads of 128 x 64 77.8 -> 40.9 us
+// (4.9 TB/s), 32 heads of 64 x 64 30.7 -> 18.4 us; one row: 8 us either way.
+template <int NPL, int L, int CPT>
+__global__ void __launch_bounds__(128)
+ssm_step_kernel(const float* xbc, const float* dd, const float* __restrict__ d_skip, const int* row_start, const int* row_slot, float* state,
+                long long slot_stride, float* out, int H, int G, int N, int P, int max_slots) {
+  constexpr int COLS = 128 / L;
+  const int r = blockIdx.z, h = blockIdx.y, sub = threadIdx.x % L, col0 = blockIdx.x * COLS * CPT + threadIdx.x / L;
+  const float skip = d_skip[h];
+  pdl_wait();
+  pdl_trigger();
+  const int slot = row_slot[r], first = row_start[r], n = row_start[r + 1] - first;
+  if (slot < 0 || slot >= max_slots || n != 1) return;
+  const int inner = H * P, C = inner + 2 * G * N, g = h / (H / G);
+  const float* row = xbc + (long long)first * C;
+  const float dt = dd[(long long)first * 2 * H + h], decay = dd[(long long)first * 2 * H + H + h];
+  const bool vec = (N & 3) == 0 && (slot_stride & 3) == 0 && (((uintptr_t)state) & 15) == 0;
+  const bool wide = (N & 3) == 0 && (C & 3) == 0 && (inner & 3) == 0 && (((uintptr_t)xbc) & 15) == 0;
+  auto fetch = [&](float (&x)[NPL], const float* p, bool fours) {
+#pragma unroll
+    for (int i = 0; i < NPL; i += 4) {
+      const int d = sub * NPL + i;
+      if (fours) {
+        const float4 u = d < N ? *reinterpret_cast<const float4*>(p + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+        x[i] = u.x; x[i + 1] = u.y; x[i + 2] = u.z; x[i + 3] = u.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[i + j] = d + j < N ? p[d + j] : 0.f;
+      }
+    }
+  };
+  float S[CPT][NPL], b[NPL], c_[NPL], x[CPT];
+  float* sp[CPT];
+#pragma unroll
+  for (int c = 0; c < CPT; ++c) {                // lanes beyond the last column follow it and write nothing
+    const int col = min(col0 + c * COLS, P - 1);
+    sp[c] = state + (long long)slot * slot_stride + ((long long)h * P + col) * N;
+    fetch(S[c], sp[c], vec);
+    x[c] = row[(long long)h * P + col];
+  }
+  fetch(b, row + inner + g * N, wide);
+  fetch(c_, row + inner + (G + g) * N, wide);
+#pragma unroll
+  for (int c = 0; c < CPT; ++c) {
+    const float u = dt * x[c];
+    float op[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < NPL; ++i) {
+      S[c][i] = fmaf(b[i], u, S[c][i] * decay);
+      op[i & 3] = fmaf(S[c][i], c_[i], op[i & 3]);
+    }
+    float o = (op[0] + op[1]) + (op[2] + op[3]);
+#pragma unroll
+    for (int k = L / 2; k >= 1; k >>= 1) o += __shfl_xor_sync(0xffffffffu, o, k);
+    const int col = col0 + c * COLS;
+    if (col >= P) continue;
+    if (sub == 0) out[(long long)first * inner + (long long)h * P + col] = fmaf(skip, x[c], o);
+#pragma unroll
+    for (int i = 0; i < NPL; i += 4) {
+      const int d = sub * NPL + i;
+      if (vec) {
+        if (d < N) *reinterpret_cast<float4*>(sp[c] + d) = make_float4(S[c][i], S[c][i + 1], S[c][i + 2], S[c][i + 3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (d + j < N) sp[c][d + j] = S[c][i + j];
+      }
+    }
+  }
+}
+
 // One block per (token, part): v = y * silu(z) over the part's n values, out = v / sqrt(mean(v^2) + eps) * w.
 template <typename T>
 __global__ void __launch_bounds__(128)
@@ -389,6 +461,12 @@ FMX_EXPORT int fmx_ssm_scan(const float* xbc, const float* dd, const float* d_sk
   if (H > 65535 || R > 65535) return fmx_fail("fmx_ssm_scan: batch too large");
 #define FMX_SSM_SCAN(NPL, L, TB)                                                                                       \
   do {                                                                                                                 \
+    if (max_tokens == 1) {                                                                                             \
+      constexpr int cpt = 2, all = 128 / (L) * cpt;                                                                    \
+      fmx_launch(ssm_step_kernel<NPL, L, cpt>, dim3((P + all - 1) / all, H, R), dim3(128), 0, stream, xbc, dd, d_skip, row_start, row_slot, \
+                 state, slot_stride, out, H, G, N, P, max_slots);                                                      \
+      break;                                                                                                           \
+    }                                                                                                                  \
     constexpr int cols = 128 / (L), rowf = (2 * (NPL) * (L) + cols + 2 + 3) / 4 * 4;                                   \
     const dim3 grid((P + cols - 1) / cols, H, R);                                                                      \
     constexpr size_t smem = (size_t)2 * (TB) * rowf * sizeof(float);                                                   \

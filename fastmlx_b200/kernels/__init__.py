@@ -21,7 +21,7 @@ def launch_count() -> int:
     return _lib.launches
 
 F32, BF16 = 0, 1
-WALK_ANY = 0x7fffffff            # a walk token by token that takes rows of any length
+WALK_ANY = 0x7fffffff            # a walk token by token that takes rows of any length (1: rows of one token, by a kernel of their own)
 BAD_TOKEN, BAD_SLOT, BAD_PAGE, BAD_ROW = 1, 2, 3, 4
 
 
@@ -636,7 +636,7 @@ def delta_rule(qkv, gb, ctx, state, H, G, D, Dv, lanes: int = 0) -> torch.Tensor
     T = qkv.shape[0]
     out = torch.empty((T, H * Dv), dtype=torch.float32, device=qkv.device)
     call("common", "fmx_delta_rule", qkv.data_ptr(), gb.data_ptr(), ctx.row_start.data_ptr(), ctx.row_slot.data_ptr(),
-         state.data_ptr(), state.stride(0), out.data_ptr(), ctx.R, H, G, D, Dv, state.shape[0], int(lanes), WALK_ANY, _stream())
+         state.data_ptr(), state.stride(0), out.data_ptr(), ctx.R, H, G, D, Dv, state.shape[0], int(lanes), 1 if ctx.max_q_len == 1 else WALK_ANY, _stream())
     return out
 
 
@@ -816,7 +816,7 @@ def ssm_scan(xbc, dd, d_skip, ctx, state, H, G, N, P, lanes: int = 0) -> torch.T
     out = torch.empty((T, H * P), dtype=torch.float32, device=xbc.device)
     call("common", "fmx_ssm_scan", xbc.data_ptr(), dd.data_ptr(), d_skip.data_ptr(), ctx.row_start.data_ptr(),
          ctx.row_slot.data_ptr(), state.data_ptr(), state.stride(0), out.data_ptr(), ctx.R, H, G, N, P, state.shape[0],
-         int(lanes), WALK_ANY, _stream())
+         int(lanes), 1 if ctx.max_q_len == 1 else WALK_ANY, _stream())
     return out
 
 

@@ -896,6 +896,30 @@ def test_portions_in_runs_of_tokens(rule, lens, H, G, D, P):
             assert torch.equal(o1[starts[r]:starts[r + 1]], o2[starts[r]:starts[r + 1]])
 
 
+@pytest.mark.parametrize("rule", ["delta", "plain"])
+@pytest.mark.parametrize("R,H,G,D,P,lanes,odd", [(3, 4, 2, 128, 128, 0, 0), (37, 2, 2, 64, 50, 0, 0), (5, 4, 1, 100, 33, 0, 0), (2, 2, 1, 30, 17, 0, 1),
+                                                 (4, 3, 1, 33, 1, 0, 3), (1, 1, 1, 1, 5, 0, 0), (9, 2, 1, 64, 64, 2, 1), (3, 2, 2, 128, 40, 32, 0)])
+def test_recurrence_over_single_tokens(rule, R, H, G, D, P, lanes, odd):
+    """Steps of one token a row go through a kernel of their own: the same bits as the walk over the tokens, outputs and states, for states that
+    begin on any boundary, sizes that end within a vector, padding rows (slot -1) and slots out of order."""
+    torch.manual_seed(R + D)
+    slots = torch.randperm(R + 2)[:R].to(torch.int32)
+    if R > 2:
+        slots[1] = -1
+    ctx = lambda longest: SimpleNamespace(R=R, row_start=torch.arange(R + 1, dtype=torch.int32, device=DEV), max_q_len=longest,
+                                          row_slot=slots.to(DEV))
+    x, gates, skip = torch.randn(R, 2 * G * D + H * P, device=DEV), torch.rand(R, 2 * H, device=DEV), torch.randn(H, device=DEV)
+    base = torch.randn(R + 2, H * P * D + 5 + odd, device=DEV)
+    got = []
+    for longest in (2, 1):
+        state = base.clone()
+        out = k().delta_rule(x, gates, ctx(longest), state, H, G, D, P, lanes) if rule == "delta" else \
+            k().ssm_scan(x, gates, skip, ctx(longest), state, H, G, D, P, lanes)
+        got.append((out[(slots >= 0).to(DEV)], state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert not torch.equal(got[1][1], base) and torch.isfinite(got[1][0]).all()
+
+
 @pytest.mark.parametrize("rule,D", [("delta", 64), ("delta", 128), ("plain", 64), ("plain", 128), ("channel delta", 64), ("channel delta", 128),
                                     ("channel plain", 64)])
 def test_short_rows_join_the_runs_of_a_long_one(rule, D):
