@@ -1147,6 +1147,27 @@ def test_mixed_heads_on_tensor_cores(lens, ctxs, nh, nkv, hd, vd, page, window, 
             assert torch.equal(got[starts[r]:starts[r + 1]], fma[starts[r]:starts[r + 1]])
 
 
+@pytest.mark.parametrize("nh,nkv", [(32, 8), (8, 4)])
+@pytest.mark.parametrize("dust", [2.0 ** -12, -(2.0 ** -20)])            # a second term of one entry, a third term
+def test_mix_without_smaller_terms(nh, nkv, dust):
+    """A mix that bfloat16 holds exactly goes without the products of its smaller terms: one entry that has them changes its own head only,
+    every other head's values are the same bits."""
+    hd, page, T = 64, 16, 45
+    q, kv, ctx, grp = _attention_case(torch.bfloat16, nh, nkv, hd, page, [(30, T)], seed=3)
+    d, g = _full_ctx([(30, T)], ctx, grp)
+    d.T, d.h_row_start = T, [0, T]
+    mix, bias = (torch.eye(nh) + 0.1 * torch.randn(nh, nh)).bfloat16().float(), torch.full((nh,), -2.0)
+    mix[5, 2] = 0.75
+    more = mix.clone()
+    more[5, 2] += dust
+    assert more[5, 2].bfloat16() != more[5, 2]
+    a, b = (k().sigmoid_attention(q.float().to(DEV), kv.to(DEV), d, g, nh, nkv, hd, hd, hd ** -0.5, 0.0, 0, page, bias.to(DEV), m.to(DEV),
+                                  tensor_cores=True).view(T, nh, hd) for m in (mix, more))
+    others = [h for h in range(nh) if h != 5]
+    assert torch.equal(a[:, others], b[:, others]) and torch.isfinite(a).all()
+    assert torch.allclose(a[:, 5].float(), b[:, 5].float(), rtol=2.0 ** -7, atol=abs(dust) * 100)
+
+
 @pytest.mark.parametrize("ctx", [2000, 60000])
 @pytest.mark.parametrize("window", [1, 26, 27, 90, 120, 121, 122, 500])
 def test_shares_of_a_window_are_no_fewer_than_four_tiles(ctx, window):
