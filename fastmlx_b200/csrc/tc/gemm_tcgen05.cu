@@ -27,6 +27,8 @@
 // something that never comes, with no copy in flight, and the expiry path runs.  Only the test
 // library `tc_expiry` is built that way; the product library never is.
 #include <cuda.h>
+#include <type_traits>
+#include <cstdlib>
 #include "activations.cuh"
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -34,7 +36,8 @@
 namespace {
 using namespace fmx_tc;
 constexpr int BM = 128, BK = 64, UMMA_K = 16;
-constexpr int THREADS = 192;
+constexpr int EPI_WARPS = 8, THREADS = (2 + EPI_WARPS) * 32;
+constexpr int TURN_LD = 20;                        // floats from row to row where 16 columns of 32-bit results change lanes
 
 // RELU2: max(x, 0)^2.  EXPERT: a routed expert's gated activation, w g' sigmoid(1.702 g') (u' + 1) with g' = min(g, limit),
 // u' = clamp(u, -limit, limit) and w the row's weight (limit < 0: w silu(g) u), over gate/up blocks like SILU_MUL.  F32: the product as 32-bit floats.
@@ -59,18 +62,24 @@ struct Grouped {
   int expert_cols;               // the experts' matrices side by side instead: expert e's K columns start e * expert_cols columns in
 };
 
-template <int BN> struct Cfg {
+template <int BN, bool TURN = false> struct Cfg {
   static constexpr int STAGES = BN == 256 ? 4 : (BN == 192 ? 5 : 6);
   static constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int TMEM_COLS = BN > 128 ? 512 : 256;   // two accumulators; a power of two >= 32
-  static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024 /* alignment */ + 256 /* barriers */;
+  static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024 /* alignment */ + 256 /* barriers */ +
+                                 (TURN ? (size_t)EPI_WARPS * 32 * TURN_LD * 4 : 0);
   static_assert((2 * STAGES + 5) * 8 + 4 <= 256, "the barriers outgrow their corner of shared memory");
 };
 
 __device__ __forceinline__ unsigned pack2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<unsigned*>(&v);
+}
+// 32 bytes, a whole sector, from one lane
+__device__ __forceinline__ void store32(float* p, const float* v) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
 }
 __device__ __forceinline__ float silu(float g) { return g / (1.0f + expf(-g)); }
 __device__ __forceinline__ float gelu_tanh(float g) {
@@ -81,7 +90,7 @@ template <int BN, int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, bf16* C,
                     long long ldc, const bf16* residual, long long ldr, int M_max, int N, int K, int* status, Grouped gr) {
-  using cfg = Cfg<BN>;
+  using cfg = Cfg<BN, EPI == EPI_F32>;
   extern __shared__ unsigned char smem_raw[];
   // 1024-byte alignment: the swizzle pattern repeats every eight 128-byte rows
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -104,7 +113,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&acc_full[a]), 1);
-      mbar_init(smem_u32(&acc_empty[a]), 128);
+      mbar_init(smem_u32(&acc_empty[a]), EPI_WARPS * 32);
     }
     mbar_init(smem_u32(drain_bar), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -217,29 +226,46 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint32_t acc_phase = 0;
     bool ok = true;
     constexpr bool GATED = EPI == EPI_SILU_MUL || EPI == EPI_GELU_MUL || EPI == EPI_EXPERT;
-    constexpr int OUT_COLS = GATED ? BN / 2 : BN;
+    constexpr int OUT_COLS = GATED ? BN / 2 : BN, MY_COLS = OUT_COLS / 2;
+    static_assert(MY_COLS % 16 == 0, "two warps to a quarter");
+    const int c_first = (warp - 2) / 4 * MY_COLS;  // two warps to a quarter, half of the columns each
+    const int n_out = GATED ? N / 2 : N;
+    // whole sectors to a lane: 16 columns of bfloat16 in one store.  32-bit columns pass through shared memory, four lanes to a row's 64 bytes.
+    const bool wide = EPI == EPI_F32 ? (((uintptr_t)C) & 15) == 0 && ldc % 4 == 0 : (((uintptr_t)C) & 31) == 0 && ldc % 16 == 0;
+    float* turn = reinterpret_cast<float*>(smem + (size_t)cfg::STAGES * cfg::STAGE_BYTES + 256) + (warp - 2) * 32 * TURN_LD;
+    const bool wide_r = EPI == EPI_RESIDUAL && (((uintptr_t)residual) & 15) == 0 && ldr % 8 == 0;
     for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
       const int m0 = (t % tiles_m) * BM, n_tile = t / tiles_m;
-      if (!mbar_wait(smem_u32(&acc_full[acc]), acc_phase)) { ok = false; break; }
-      tc_fence_after();
       const int row = m0 + quarter * 32 + lane;
-      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN);
       const int out_n0 = n_tile * OUT_COLS;
-      const int n_out = GATED ? N / 2 : N;
       const bool row_in_use = row < M && (gr.row_token == nullptr || gr.row_token[row] >= 0);
+      const unsigned rows_in_use = __ballot_sync(0xffffffffu, row_in_use);
       float row_w = ((EPI == EPI_EXPERT || EPI == EPI_ACT) && row_in_use) ? (gr.row_weight != nullptr ? gr.row_weight[row] : 1.0f) : 0.f;
       float in_w = 1.0f;                           // ACT: what multiplies the product in front of its activation, row_w what does behind
       if (EPI == EPI_ACT) {
         if (gr.pre) { in_w = row_w; row_w = 1.0f; }
         if (gr.row_gate != nullptr && row_in_use) row_w *= sigmoid_f(gr.row_gate[(long long)row * gr.row_gate_stride]);
       }
+      if (!mbar_wait(smem_u32(&acc_full[acc]), acc_phase)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN);
+      // FORM: which activation, chosen in front of the loop (inside, each element's branch would wait for the element before)
+      auto columns = [&](auto form) {
+        constexpr int FORM = decltype(form)::value;
 #pragma unroll 1
-      for (int c = 0; c < OUT_COLS; c += 16) {
-        uint32_t v[16], u[16];
-        tmem_ld16(taddr + c, v);
-        if (GATED) tmem_ld16(taddr + BN / 2 + c, u);
-        tmem_ld_wait();
-        if (row_in_use) {
+        for (int c = c_first; c < c_first + MY_COLS; c += 16) {
+          uint32_t v[16], u[16];
+          tmem_ld16(taddr + c, v);
+          if (GATED) tmem_ld16(taddr + BN / 2 + c, u);
+          const int col = out_n0 + c;
+          const bool whole = col + 16 <= n_out;
+          uint4 ra, rb;
+          if (EPI == EPI_RESIDUAL && wide_r && whole && row_in_use) {
+            const uint4* rp = reinterpret_cast<const uint4*>(residual + (long long)row * ldr + col);
+            ra = rp[0];
+            rb = rp[1];
+          }
+          tmem_ld_wait();
           float f[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
@@ -250,52 +276,81 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
               const float w = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[i])));
               f[i] = (EPI == EPI_SILU_MUL ? silu(g) : gelu_tanh(g)) * w;
             }
-            if (EPI == EPI_EXPERT) {
-              if (gr.limit < 0.f) {                  // silu(g) u, without clamps
-                f[i] = row_w * silu(f[i]) * __uint_as_float(u[i]);
-              } else {
-                f[i] = row_w * clamped_gate(f[i], __uint_as_float(u[i]), gr.limit);
-              }
+            if (EPI == EPI_EXPERT) {                 // FORM 0: silu(g) u, without clamps
+              if (FORM == 0) f[i] = row_w * silu(f[i]) * __uint_as_float(u[i]);
+              else f[i] = row_w * clamped_gate(f[i], __uint_as_float(u[i]), gr.limit);
             }
-            if (EPI == EPI_ACT) f[i] = row_w * act_f(gr.act, in_w * f[i]);
+            if (EPI == EPI_ACT) f[i] = row_w * act_f(FORM, in_w * f[i]);
             if (EPI == EPI_RELU2) {
               // as the unfused path rounds: the product to bfloat16 first, then the square of its positive part
               const float p = fmaxf(__bfloat162float(__float2bfloat16_rn(f[i])), 0.f);
               f[i] = p * p;
             }
           }
-          const int col = out_n0 + c;
+          if (EPI == EPI_F32 && whole && wide) {
+            __syncwarp();                            // the columns before are read
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              *reinterpret_cast<float4*>(turn + lane * TURN_LD + 4 * i) = make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int r = 8 * j + lane / 4;
+              const float4 x = *reinterpret_cast<const float4*>(turn + r * TURN_LD + lane % 4 * 4);
+              if (rows_in_use >> r & 1)
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(C) + (long long)(m0 + quarter * 32 + r) * ldc + col + lane % 4 * 4) = x;
+            }
+            continue;
+          }
+          if (!row_in_use) continue;
           if (EPI == EPI_F32) {
             float* dstf = reinterpret_cast<float*>(C) + (long long)row * ldc + col;
-            if (col + 16 <= n_out && (((uintptr_t)dstf) & 15) == 0) {
 #pragma unroll
-              for (int i = 0; i < 4; ++i) reinterpret_cast<float4*>(dstf)[i] = make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
-            } else {
-#pragma unroll
-              for (int i = 0; i < 16; ++i)
-                if (col + i < n_out) dstf[i] = f[i];
-            }
+            for (int i = 0; i < 16; ++i)
+              if (col + i < n_out) dstf[i] = f[i];
             continue;
           }
           bf16* dst = C + (long long)row * ldc + col;
           if (EPI == EPI_RESIDUAL) {
-            const bf16* rp = residual + (long long)row * ldr + col;
+            if (wide_r && whole) {
+              const unsigned rw[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (col + i < n_out) f[i] = __bfloat162float(__float2bfloat16_rn(f[i])) + __bfloat162float(rp[i]);
+              for (int i = 0; i < 16; ++i)
+                f[i] = __bfloat162float(__float2bfloat16_rn(f[i])) + __uint_as_float(i & 1 ? rw[i / 2] & 0xffff0000u : rw[i / 2] << 16);
+            } else {
+              const bf16* rp = residual + (long long)row * ldr + col;
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (col + i < n_out) f[i] = __bfloat162float(__float2bfloat16_rn(f[i])) + __bfloat162float(rp[i]);
+            }
           }
-          if (col + 16 <= n_out && (((uintptr_t)dst) & 15) == 0) {
-            uint4 a, b;
-            a.x = pack2(f[0], f[1]); a.y = pack2(f[2], f[3]); a.z = pack2(f[4], f[5]); a.w = pack2(f[6], f[7]);
-            b.x = pack2(f[8], f[9]); b.y = pack2(f[10], f[11]); b.z = pack2(f[12], f[13]); b.w = pack2(f[14], f[15]);
-            reinterpret_cast<uint4*>(dst)[0] = a;
-            reinterpret_cast<uint4*>(dst)[1] = b;
+          if (whole && (wide || (((uintptr_t)dst) & 15) == 0)) {
+            float p[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) p[i] = __uint_as_float(pack2(f[2 * i], f[2 * i + 1]));
+            if (wide) {
+              store32(reinterpret_cast<float*>(dst), p);
+            } else {
+              reinterpret_cast<float4*>(dst)[0] = make_float4(p[0], p[1], p[2], p[3]);
+              reinterpret_cast<float4*>(dst)[1] = make_float4(p[4], p[5], p[6], p[7]);
+            }
           } else {
 #pragma unroll
             for (int i = 0; i < 16; ++i)
               if (col + i < n_out) dst[i] = __float2bfloat16_rn(f[i]);
           }
         }
+      };
+      if constexpr (EPI == EPI_EXPERT) {
+        if (gr.limit < 0.f) columns(std::integral_constant<int, 0>{});
+        else columns(std::integral_constant<int, 1>{});
+      } else if constexpr (EPI == EPI_ACT) {
+        if (gr.act == 0) columns(std::integral_constant<int, 0>{});
+        else if (gr.act == 1) columns(std::integral_constant<int, 1>{});
+        else if (gr.act == 3) columns(std::integral_constant<int, 3>{});
+        else columns(std::integral_constant<int, 2>{});
+      } else {
+        columns(std::integral_constant<int, 0>{});
       }
       tc_fence_before();
       mbar_arrive(smem_u32(&acc_empty[acc]));
@@ -315,7 +370,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 template <int BN, int EPI>
 int run(const void* A, long long lda, const void* W, long long ldw, void* C, long long ldc, const void* residual,
         long long ldr, int M, int N, int K, int sms, int* status, cudaStream_t stream, Grouped gr = Grouped{}, long long w_rows = 0, int w_cols = 0) {
-  using cfg = Cfg<BN>;
+  using cfg = Cfg<BN, EPI == EPI_F32>;
   CUtensorMap map_a, map_w;
   if (make_map_k128(&map_a, A, M, K, lda, BM) || make_map_k128(&map_w, W, w_rows > 0 ? w_rows : N, w_cols > 0 ? w_cols : K, ldw, BN)) return 1;
   static bool configured = false;
@@ -368,6 +423,10 @@ FMX_EXPORT int fmx_grouped_tcgen05(const void* A, long long lda, const void* W, 
   const Grouped gr{used_rows, tile_expert, row_token, row_weight, N, limit, 0, 0, nullptr, 0, 0};
   if (gated)
     return run<256, EPI_EXPERT>(A, lda, W, ldw, C, ldc, nullptr, 0, max_rows, N, K, sms, status, stream, gr, (long long)experts * N);
+  if (getenv("FMX_BN") && atoi(getenv("FMX_BN")) == 192)
+    return run<192, EPI_F32>(A, lda, W, ldw, C, ldc, nullptr, 0, max_rows, N, K, sms, status, stream, gr, (long long)experts * N);
+  if (getenv("FMX_BN") && atoi(getenv("FMX_BN")) == 128)
+    return run<128, EPI_F32>(A, lda, W, ldw, C, ldc, nullptr, 0, max_rows, N, K, sms, status, stream, gr, (long long)experts * N);
   return run<256, EPI_F32>(A, lda, W, ldw, C, ldc, nullptr, 0, max_rows, N, K, sms, status, stream, gr, (long long)experts * N);
 }
 
