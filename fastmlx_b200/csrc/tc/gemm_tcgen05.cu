@@ -28,7 +28,6 @@
 // library `tc_expiry` is built that way; the product library never is.
 #include <cuda.h>
 #include <type_traits>
-#include <cstdlib>
 #include "activations.cuh"
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -423,10 +422,6 @@ FMX_EXPORT int fmx_grouped_tcgen05(const void* A, long long lda, const void* W, 
   const Grouped gr{used_rows, tile_expert, row_token, row_weight, N, limit, 0, 0, nullptr, 0, 0};
   if (gated)
     return run<256, EPI_EXPERT>(A, lda, W, ldw, C, ldc, nullptr, 0, max_rows, N, K, sms, status, stream, gr, (long long)experts * N);
-  if (getenv("FMX_BN") && atoi(getenv("FMX_BN")) == 192)
-    return run<192, EPI_F32>(A, lda, W, ldw, C, ldc, nullptr, 0, max_rows, N, K, sms, status, stream, gr, (long long)experts * N);
-  if (getenv("FMX_BN") && atoi(getenv("FMX_BN")) == 128)
-    return run<128, EPI_F32>(A, lda, W, ldw, C, ldc, nullptr, 0, max_rows, N, K, sms, status, stream, gr, (long long)experts * N);
   return run<256, EPI_F32>(A, lda, W, ldw, C, ldc, nullptr, 0, max_rows, N, K, sms, status, stream, gr, (long long)experts * N);
 }
 
