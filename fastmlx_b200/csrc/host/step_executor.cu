@@ -20,7 +20,7 @@ typedef int (*add_rmsnorm_fn)(const void*, void*, const float*, void*, int, int,
 typedef int (*silu_mul_fn)(const void*, void*, int, int, int, int, cudaStream_t);
 typedef int (*gemm_simple_fn)(const void*, const void*, const float*, void*, int, int, int, long long, long long,
                               long long, int, int, int, cudaStream_t);
-typedef int (*gemm_three_fn)(const float*, long long, const void*, long long, const float*, float*, long long, int, int, int, void*, int,
+typedef int (*gemm_three_fn)(const float*, long long, const void*, long long, const float*, float*, long long, int, int, int, int, void*, int,
                              int*, cudaStream_t);
 typedef int (*rope_kv_write_fn)(void*, const int*, const float*, const long long*, void*, int, int, int, int, int, int,
                                 int, long long, long long, int, int*, cudaStream_t);
@@ -175,7 +175,7 @@ struct Run {
     if (M == 0) return 0;
     if (x_dtype == FMX_F32 && op.w_dtype == FMX_BF16 && out_dtype == FMX_F32 && ex.k.gemm_three != nullptr && op.terms >= 0) {
       ++ex.launches;
-      return ((gemm_three_fn)ex.k.gemm_three)((const float*)x, ldx, op.w, op.ldw, op.bias, (float*)out, ldo, M, N, K, reg(op.terms), ex.sms,
+      return ((gemm_three_fn)ex.k.gemm_three)((const float*)x, ldx, op.w, op.ldw, op.bias, (float*)out, ldo, M, N, K, N, reg(op.terms), ex.sms,
                                               d.status, stream);
     }
     if (x_dtype != FMX_BF16 || op.w_dtype != FMX_BF16) {

@@ -5,8 +5,9 @@
 // One order of sums for every M.  The tensor cores cut their sums off instead of rounding them, so they add up 64 k only:
 // the small terms first, then the leading ones (four sums of the full size).  Such blocks of 64 k are added up in rounded
 // 32-bit sums in registers, k ascending, over `splits` shares of K, and the shares' sums one after the other.  The
-// shares follow from N and K alone (plan_splits) and a product's column does not depend on the other columns, so
-// a token's result is the same whichever other tokens share the step.
+// shares follow from the matrix's N and K alone (plan_splits; a product over some of a matrix's rows takes the whole matrix's)
+// and a product's column does not depend on the other columns, so a token's result is the same whichever other tokens share the
+// step, and whichever other features the product.
 //
 //   split       lays the activations' terms out in memory, three matrices one under the other.
 //   warp 0      brings blocks of W (128 features x 64 k) and of the terms (up to 128 tokens x 64 k each) by TMA.
@@ -339,12 +340,13 @@ FMX_EXPORT int fmx_gemm_three_splits(int N, int K) { return N > 0 && K > 0 ? pla
 // Bytes of workspace that a product of M tokens over K takes: the activations' three terms.
 FMX_EXPORT long long fmx_gemm_three_bytes(int M, int K) { return 6LL * M * K; }
 
-// A 32-bit [M, K], W bfloat16 [N, K] with K-contiguous rows that start on 16 bytes, C 32-bit [M, N].  ws: fmx_gemm_three_bytes on 16
+// A 32-bit [M, K], W bfloat16 [N, K] with K-contiguous rows that start on 16 bytes, C 32-bit [M, N].  whole_n: features of the matrix
+// that W's rows are a part of, whose shares of K the product takes; N where W is all of it.  ws: fmx_gemm_three_bytes on 16
 // bytes.  status: the engine's status word (a wait that expires leaves FMX_WAIT_EXPIRED there).
 FMX_EXPORT int fmx_gemm_three(const float* A, long long lda, const void* W, long long ldw, const float* bias, float* C, long long ldc,
-                              int M, int N, int K, void* ws, int sms, int* status, cudaStream_t stream) {
+                              int M, int N, int K, int whole_n, void* ws, int sms, int* status, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
-  if (M < 0 || N < 0 || K <= 0) return fmx_fail("fmx_gemm_three: bad sizes M=%d N=%d K=%d", M, N, K);
+  if (M < 0 || N < 0 || K <= 0 || whole_n < N) return fmx_fail("fmx_gemm_three: bad sizes M=%d N=%d of %d K=%d", M, N, whole_n, K);
   if (K % 8 || ldw % 8 || ((uintptr_t)W & 15)) return fmx_fail("fmx_gemm_three: W's rows must start on 16 bytes (K=%d ldw=%lld)", K, ldw);
   if (ws == nullptr || ((uintptr_t)ws & 15)) return fmx_fail("fmx_gemm_three: the workspace is missing or does not lie on 16 bytes");
   if (sms <= 0) sms = fmx_num_sms();
@@ -356,7 +358,7 @@ FMX_EXPORT int fmx_gemm_three(const float* A, long long lda, const void* W, long
   const long long tiles = (long long)a.tiles_t * ((N + TF - 1) / TF);
   if (tiles > 0x7fffffffLL / MAX_SPLITS || M > 0x7fffffff / 3) return fmx_fail("fmx_gemm_three: M=%d N=%d are too large", M, N);
   a.tiles = (int)tiles;
-  a.splits = plan_splits(N, K);
+  a.splits = plan_splits(whole_n, K);
   // A CTA's whole walk over K, or a cluster's shares of it: blocks of K that the busiest SM takes, with APART more for each CTA of a
   // cluster (its start, the ring's filling, the sum over the shares).
   const int blocks = (K + BK - 1) / BK;

@@ -324,16 +324,17 @@ def holds_exactly(ws) -> bool:
     return bool(torch.isfinite(ends).all())
 
 
-def gemm_three(x, w, bias=None, status=None) -> torch.Tensor:
+def gemm_three(x, w, bias=None, status=None, whole: int = 0) -> torch.Tensor:
     """x[M, K] in 32-bit @ w[N, K]^T in bfloat16 (+ bias) -> 32-bit [M, N], to 32-bit accuracy on the tensor cores; a row's result
-    does not depend on the other rows."""
+    does not depend on the other rows.  `whole`: features of the matrix that w is some rows of (0: w is all of it); the results are then the
+    bits that the product over the whole matrix gives these features."""
     M, K = x.shape
     N = w.shape[0]
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     need = load("tc").fmx_gemm_three_bytes(M, K)
     ws = torch.empty(need, dtype=torch.uint8, device=x.device)
     call("tc", "fmx_gemm_three", x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), _ptr(bias), out.data_ptr(), out.stride(0),
-         M, N, K, ws.data_ptr(), num_sms(x.device), _ptr(status if status is not None else _status_word(x.device)), _stream())
+         M, N, K, int(whole or N), ws.data_ptr(), num_sms(x.device), _ptr(status if status is not None else _status_word(x.device)), _stream())
     return out
 
 

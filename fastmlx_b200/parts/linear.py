@@ -70,6 +70,13 @@ class Linear(Part):
     def forward(self, x, out_dtype=None):
         return self.rt.k.linear(x, self.weight, self.bias, out_dtype or self.rt.dtype)
 
+    def forward_rows(self, x, first: int, last: int, out_dtype=None):
+        """Features [first, last) of `forward` alone: on the 32-bit path the same bits, whose sums over K follow the whole matrix."""
+        w, b = self.weight[first:last], None if self.bias is None else self.bias[first:last]
+        if x.dtype == torch.float32 and w.dtype == torch.bfloat16 and self.rt.is_fp32:      # held by `exact_matrices`
+            return self.rt.k.gemm_three(x, w, b, whole=self.out_features)
+        return self.rt.k.linear(x, w, b, out_dtype or self.rt.dtype)
+
     def emit(self, b, x: int, out_dtype=None, out: int | None = None) -> int:
         """Native program: out = x . W^T (+ b) into a new register (or into `out`)."""
         from ..engine.native import OP_LINEAR, _dt

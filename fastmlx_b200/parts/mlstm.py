@@ -66,14 +66,14 @@ class MatrixMemoryMixer(Mixer):
 
     def forward_inner(self, x, ctx, cache, out=None):
         """The normalised, gated read-outs of all heads side by side, [T, heads * vdim]."""
-        k, w = self.rt.k, self.proj.weight
+        k = self.rt.k
         n, m = 2 * self.H * self.D + self.inner_features, self.inner_features
         if x.shape[0] <= self.WIDE_MAX_TOKENS:
-            proj = k.linear(x, w, None, torch.float32)
+            proj = self.proj.forward(x, torch.float32)
             z = proj[:, n + m:]
-        else:
-            proj = k.linear(x, w[:n + m], None, self.rt.dtype)
-            z = k.linear(x, w[n + m:], None, torch.float32)
+        else:                                    # (in 32-bit both ways give the same bits)
+            proj = self.proj.forward_rows(x, 0, n + m)
+            z = self.proj.forward_rows(x, n + m, self.proj.out_features, torch.float32)
         if ctx.max_q_len == 1:
             return k.mlstm_step(proj, z, self.gate_bias, self.cap, ctx, cache.state, self.H, self.D, self.Dv, self.norm_w, self.eps,
                                 self.rt.dtype, out=out)

@@ -378,6 +378,27 @@ def test_a_value_stored_long_ago_is_read_back(tmp_path, dtype, cut):
     _close(rig.feed([h], cut)[0], want, 4e-5 if dtype == "float32" else 3e-2)
 
 
+def test_projections_do_not_depend_on_the_step(monkeypatch):
+    """In 32-bit a token's projections are the same bits in a portion of 16 tokens (one product) and of 17 (two over some of the
+    matrix's rows each), at a width whose sums over K are split."""
+    from fastmlx_b200 import kernels as k
+    from fastmlx_b200.engine.loading import make_runtime
+    from fastmlx_b200.parts import MatrixMemoryMixer
+    d, H, D, Dv = 2048, 8, 128, 256
+    mixer = MatrixMemoryMixer(d, H, D, Dv, 15.0, 1e-6, "m")
+    g = torch.Generator().manual_seed(5)
+    W = {s.name: (torch.randn(s.shape, generator=g) * 0.02).bfloat16() for s in mixer.weight_specs()}
+    mixer.bind(W, make_runtime("float32"))
+    seen, scan = [], k.mlstm_scan
+    monkeypatch.setattr(k, "mlstm_scan", lambda proj, gates, *more: seen.append((proj, gates)) or scan(proj, gates, *more))
+    x = torch.randn(17, d, generator=g).cuda()
+    for n in (17, 16):
+        _, dev = _ctx([n], [0])
+        mixer.forward(x[:n], dev, SimpleNamespace(state=torch.zeros((1,) + mixer.state_spec().shape, device="cuda")))
+    (wide, gates), (few, gates16) = seen
+    assert torch.equal(wide[:16], few[:, :wide.shape[1]]) and torch.equal(gates[:16], gates16)
+
+
 # ----------------------------------------------------------------------------- kernels alone
 def _ctx(lens, slots):
     starts = [0]

@@ -266,6 +266,17 @@ def test_gemm_three_does_not_depend_on_the_batch(N, K, bias):
     assert int(k()._status_word(DEV)[0]) == 0
 
 
+@pytest.mark.parametrize("M", [1, 17, 200])
+@pytest.mark.parametrize("N,K,cuts", [(6160, 2048, (0, 6144, 6160)), (1032, 8192, (0, 8, 700, 1032)), (300, 520, (0, 1, 299, 300))])
+def test_gemm_three_over_some_rows_of_a_matrix(N, K, cuts, M):
+    """The product over some of a matrix's rows takes the whole matrix's shares of K: the bits that the whole product gives those features
+    (6,160 x 2,048: 2 shares, its last 16 rows by themselves would take 4)."""
+    x, w = torch.randn(M, K, device=DEV), rnd(N, K, dtype=torch.bfloat16, seed=14).to(DEV)
+    whole = k().gemm_three(x, w)
+    for a, b in zip(cuts, cuts[1:]):
+        assert torch.equal(k().gemm_three(x, w[a:b], whole=N), whole[:, a:b]), (a, b)
+
+
 def test_gemm_three_infinite_and_huge_activations():
     """An infinity or a NaN stays in its row; values that would round to an infinity in bfloat16 do not."""
     x, w = torch.randn(40, 192), rnd(70, 192, dtype=torch.bfloat16, seed=12)

@@ -16,3 +16,15 @@ def test_no_kernel_is_chosen_by_the_environment():
     sources = [p for p in pathlib.Path(build.HERE).rglob("*") if p.suffix in (".cu", ".cuh", ".h")]
     assert len(sources) > 40
     assert [p.name for p in sources if "getenv" in p.read_text()] == []
+
+
+def test_shares_of_the_three_term_product():
+    """They follow the matrix, so its rows by themselves would be summed otherwise: at a width of 2,048, all projections of a matrix memory
+    (8 heads, 128 x 256) and their gates' alone.  No more than a cluster holds, and no more than there are blocks of K."""
+    from fastmlx_b200.kernels import load
+    shares = load("tc").fmx_gemm_three_splits
+    assert shares(2 * 8 * 128 + 2 * 8 * 256 + 16, 2048) == 2 and shares(16, 2048) == 4
+    for N in (1, 128, 129, 2048, 16384, 128256):
+        for K in (8, 64, 65, 512, 2048, 8192, 14336):
+            assert 1 <= shares(N, K) <= min(8, -(-K // 64))
+    assert shares(0, 64) == shares(64, 0) == 0
