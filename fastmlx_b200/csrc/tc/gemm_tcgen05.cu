@@ -3,7 +3,7 @@
 // (cp.async.bulk.tensor, 128-byte swizzle), accumulators in tensor memory and read back with
 // tcgen05.ld for the epilogue.  This is the matrix product of prefill steps.
 //
-// One persistent CTA per SM walks over 128 x BN output tiles.  Six warps, three roles:
+// One persistent CTA per SM walks over 128 x BN output tiles.  Ten warps, three roles:
 //   warp 0, one lane : producer.  Waits for a free stage, arms its "full" barrier with the
 //                      stage's byte count and issues two TMA loads (A tile 128 x 64, W tile
 //                      BN x 64).  Both operands are K-major, so one box is one 128-byte row
@@ -13,8 +13,8 @@
 //                      "empty" barrier; after the last k block commits to the accumulator's
 //                      "full" barrier.  Two accumulators in tensor memory let the next tile's
 //                      mainloop run under this tile's epilogue.
-//   warps 2-5        : epilogue.  Each warp owns the 32 lanes of tensor memory it may read
-//                      (warp index mod 4), loads 16 columns at a time, converts and stores.
+//   warps 2-9        : epilogue.  Each warp owns the 32 lanes of tensor memory it may read
+//                      (warp index mod 4) and half of the columns, loads 16 at a time, converts and stores.
 //                      Variants: plain; SiLU(gate) * up for a weight whose rows come in blocks
 //                      of BN/2 gate rows followed by their BN/2 up rows; residual add.
 //
@@ -299,45 +299,45 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
               if (rows_in_use >> r & 1)
                 *reinterpret_cast<float4*>(reinterpret_cast<float*>(C) + (long long)(m0 + quarter * 32 + r) * ldc + col + lane % 4 * 4) = x;
             }
-            continue;
-          }
-          if (!row_in_use) continue;
-          if (EPI == EPI_F32) {
-            float* dstf = reinterpret_cast<float*>(C) + (long long)row * ldc + col;
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (col + i < n_out) dstf[i] = f[i];
-            continue;
-          }
-          bf16* dst = C + (long long)row * ldc + col;
-          if (EPI == EPI_RESIDUAL) {
-            if (wide_r && whole) {
-              const unsigned rw[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+          } else if (row_in_use) {
+            if constexpr (EPI == EPI_F32) {
+              float* dstf = reinterpret_cast<float*>(C) + (long long)row * ldc + col;
 #pragma unroll
               for (int i = 0; i < 16; ++i)
-                f[i] = __bfloat162float(__float2bfloat16_rn(f[i])) + __uint_as_float(i & 1 ? rw[i / 2] & 0xffff0000u : rw[i / 2] << 16);
+                if (col + i < n_out) dstf[i] = f[i];
             } else {
-              const bf16* rp = residual + (long long)row * ldr + col;
+              bf16* dst = C + (long long)row * ldc + col;
+              if (EPI == EPI_RESIDUAL) {
+                if (wide_r && whole) {
+                  const unsigned rw[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
 #pragma unroll
-              for (int i = 0; i < 16; ++i)
-                if (col + i < n_out) f[i] = __bfloat162float(__float2bfloat16_rn(f[i])) + __bfloat162float(rp[i]);
+                  for (int i = 0; i < 16; ++i)
+                    f[i] = __bfloat162float(__float2bfloat16_rn(f[i])) + __uint_as_float(i & 1 ? rw[i / 2] & 0xffff0000u : rw[i / 2] << 16);
+                } else {
+                  const bf16* rp = residual + (long long)row * ldr + col;
+#pragma unroll
+                  for (int i = 0; i < 16; ++i)
+                    if (col + i < n_out) f[i] = __bfloat162float(__float2bfloat16_rn(f[i])) + __bfloat162float(rp[i]);
+                }
+              }
+              if (whole && (wide || (((uintptr_t)dst) & 15) == 0)) {
+                float p[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) p[i] = __uint_as_float(pack2(f[2 * i], f[2 * i + 1]));
+                if (wide) {
+                  store32(reinterpret_cast<float*>(dst), p);
+                } else {
+                  reinterpret_cast<float4*>(dst)[0] = make_float4(p[0], p[1], p[2], p[3]);
+                  reinterpret_cast<float4*>(dst)[1] = make_float4(p[4], p[5], p[6], p[7]);
+                }
+              } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                  if (col + i < n_out) dst[i] = __float2bfloat16_rn(f[i]);
+              }
             }
           }
-          if (whole && (wide || (((uintptr_t)dst) & 15) == 0)) {
-            float p[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) p[i] = __uint_as_float(pack2(f[2 * i], f[2 * i + 1]));
-            if (wide) {
-              store32(reinterpret_cast<float*>(dst), p);
-            } else {
-              reinterpret_cast<float4*>(dst)[0] = make_float4(p[0], p[1], p[2], p[3]);
-              reinterpret_cast<float4*>(dst)[1] = make_float4(p[4], p[5], p[6], p[7]);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (col + i < n_out) dst[i] = __float2bfloat16_rn(f[i]);
-          }
+          __syncwarp();                              // tensor memory is read by whole warps: the lanes meet again in front of the next columns
         }
       };
       if constexpr (EPI == EPI_EXPERT) {

@@ -188,6 +188,56 @@ def test_gemm_tcgen05_epilogues(M, I, K):
     close(got, ref, torch.bfloat16, "residual epilogue", extra=2.0 ** -8 * ref.abs().max().item())
 
 
+@pytest.mark.parametrize("M", [1, 31, 33, 128, 200, 257])
+@pytest.mark.parametrize("epilogue,bn,N", [("EPI_PLAIN", 128, 136), ("EPI_PLAIN", 192, 400), ("EPI_PLAIN", 256, 520), ("EPI_SILU_MUL", 256, 512),
+                                           ("EPI_SILU_MUL", 128, 256), ("EPI_GELU_MUL", 256, 256), ("EPI_RELU2", 256, 300), ("EPI_RESIDUAL", 256, 281)])
+def test_tcgen05_epilogues_store_the_same_wherever_the_output_lies(M, epilogue, bn, N):
+    """Tiles whose rows end inside a warp's, outputs that start on 32, 16 and 2 bytes, a residual that lies likewise or is the output itself:
+    the same bits, and nothing beside them is written."""
+    x, w = rnd(M, 136, dtype=torch.bfloat16, seed=41).to(DEV), rnd(N, 136, dtype=torch.bfloat16, seed=42, scale=0.1).to(DEV)
+    e, n_out, st = getattr(k(), epilogue), N // 2 if epilogue.endswith("_MUL") else N, status()
+    res = rnd(M, N, dtype=torch.bfloat16, seed=43).to(DEV) if epilogue == "EPI_RESIDUAL" else None
+    base = torch.zeros(M, -(-n_out // 16) * 16, dtype=torch.bfloat16, device=DEV)[:, :n_out]
+    k().gemm_tcgen05(x, w, st, epilogue=e, residual=res, bn=bn, out=base)
+    product = x.double() @ w.double().t()
+    if res is not None:
+        close(base, product + res.double(), torch.bfloat16, epilogue, extra=2.0 ** -8 * product.abs().max().item())
+    elif epilogue == "EPI_PLAIN":
+        close(base, product, torch.bfloat16, epilogue)
+    for off, pad in ((0, 16), (8, 8), (1, 3), (16, 16)):
+        wide = torch.full((M + 2, off + n_out + pad), 7.0, dtype=torch.bfloat16, device=DEV)
+        out = wide[1:M + 1, off:off + n_out]
+        if res is not None:
+            out.copy_(res)
+        k().gemm_tcgen05(x, w, st, epilogue=e, residual=out if res is not None else None, bn=bn, out=out)
+        assert torch.equal(out, base), (off, pad)
+        assert (wide[0] == 7).all() and (wide[-1] == 7).all() and (wide[:, :off] == 7).all() and (wide[:, off + n_out:] == 7).all()
+    assert st.tolist() == [0] * 4
+
+
+@pytest.mark.parametrize("N", [16, 200, 264])
+@pytest.mark.parametrize("used", [1, 130, 300, 384])
+def test_grouped_tcgen05_writes_rows_in_use_alone(N, used):
+    """32-bit outputs of the grouped product, rows of 16 bytes and not: padding rows between the pairs and rows behind those in use stay as
+    they were, columns end inside a group of 16."""
+    from fastmlx_b200.kernels import call
+    K, experts = 136, 3
+    x, w = rnd(384, K, dtype=torch.bfloat16, seed=51).to(DEV), rnd(experts * N, K, dtype=torch.bfloat16, seed=52).to(DEV)
+    tile_expert = torch.tensor([2, 0, 1], dtype=torch.int32, device=DEV)
+    token = torch.arange(384, dtype=torch.int32, device=DEV)
+    token[torch.randperm(384, generator=torch.Generator().manual_seed(used))[:90].to(DEV)] = -1
+    n_used, st = torch.tensor([used], dtype=torch.int32, device=DEV), status()
+    want = torch.cat([x[128 * t:128 * t + 128].double() @ w[N * e:N * e + N].double().t() for t, e in enumerate((2, 0, 1))])
+    rows = (token >= 0) & (torch.arange(384, device=DEV) < used)
+    for ldc in (-(-N // 4) * 4, N + 1, N + 12):
+        c = torch.full((384, ldc), 7.0, device=DEV)
+        call("tc", "fmx_grouped_tcgen05", x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), c.data_ptr(), ldc, 384, N, K, experts, n_used.data_ptr(),
+             tile_expert.data_ptr(), token.data_ptr(), None, 0.0, 0, 0, st.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert (c[~rows] == 7).all() and (c[:, N:] == 7).all()
+        close(c[rows][:, :N], want[rows], torch.float32, "grouped product", scale=8 * want.abs().max().item())
+    assert st.tolist() == [0] * 4
+
+
 @pytest.mark.parametrize("M", [1, 2, 7, 8, 9, 16])
 @pytest.mark.parametrize("N,K", [(16, 32), (64, 64), (131, 80), (3072, 2048), (2048, 8192), (50, 8), (320, 192), (17, 1000)])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
