@@ -317,17 +317,18 @@ def gemm_tcgen05(x, w, status=None, epilogue: int = EPI_PLAIN, residual=None, bn
 
 def holds_exactly(ws) -> bool:
     """May the 32-bit path keep these matrices as the bfloat16 values they were stored as (`gemm_three` multiplies them exactly) instead
-    of widening them?  Rows of 16-byte pieces; finite, since an infinity would meet the zeros among an activation's terms."""
+    of widening them?  Rows of 16-byte pieces; finite (`gemm_three`'s `finite`)."""
     if not all(w.dtype == torch.bfloat16 and w.dim() == 2 and w.numel() > 0 and w.shape[1] % 8 == 0 for w in ws):
         return False
     ends = torch.stack([e for w in ws for e in torch.aminmax(w)])          # a NaN shows in both
     return bool(torch.isfinite(ends).all())
 
 
-def gemm_three(x, w, bias=None, status=None, whole: int = 0) -> torch.Tensor:
+def gemm_three(x, w, bias=None, status=None, whole: int = 0, finite: bool = False) -> torch.Tensor:
     """x[M, K] in 32-bit @ w[N, K]^T in bfloat16 (+ bias) -> 32-bit [M, N], to 32-bit accuracy on the tensor cores; a row's result
     does not depend on the other rows.  `whole`: features of the matrix that w is some rows of (0: w is all of it); the results are then the
-    bits that the product over the whole matrix gives these features."""
+    bits that the product over the whole matrix gives these features.  `finite`: the caller knows that w holds no infinity, which would meet
+    the zeros among an activation's smaller terms; else results that are not finite are worked out again by themselves."""
     M, K = x.shape
     N = w.shape[0]
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
@@ -335,6 +336,9 @@ def gemm_three(x, w, bias=None, status=None, whole: int = 0) -> torch.Tensor:
     ws = torch.empty(need, dtype=torch.uint8, device=x.device)
     call("tc", "fmx_gemm_three", x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), _ptr(bias), out.data_ptr(), out.stride(0),
          M, N, K, int(whole or N), ws.data_ptr(), num_sms(x.device), _ptr(status if status is not None else _status_word(x.device)), _stream())
+    if not finite:
+        call("tc", "fmx_gemm_three_not_finite", x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), _ptr(bias), out.data_ptr(), out.stride(0),
+             M, N, K, _stream())
     return out
 
 

@@ -87,6 +87,7 @@ _SIGNATURES = {
         "fmx_moe_combine": [_P, _P, _P, _L, _I, _P, _L, _I, _I, _I, _I, _P],
     },
     "tc": {
+        "fmx_gemm_three_not_finite": [_P, _L, _P, _L, _P, _P, _L, _I, _I, _I, _P],
         "fmx_gemm_three": [_P, _L, _P, _L, _P, _P, _L, _I, _I, _I, _I, _P, _I, _P, _P],
         "fmx_gemm_tcgen05": [_P, _L, _P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _I, _I, _P, _P],
         "fmx_grouped_act_tcgen05": [_P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _P, _P, _P, _P, _I, _I, _I, _P, _P],

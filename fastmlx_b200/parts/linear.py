@@ -68,14 +68,17 @@ class Linear(Part):
         return self.weight.numel() * self.weight.element_size()
 
     def forward(self, x, out_dtype=None):
-        return self.rt.k.linear(x, self.weight, self.bias, out_dtype or self.rt.dtype)
+        return self._product(x, self.weight, self.bias, out_dtype)
 
     def forward_rows(self, x, first: int, last: int, out_dtype=None):
         """Features [first, last) of `forward` alone: on the 32-bit path the same bits, whose sums over K follow the whole matrix."""
-        w, b = self.weight[first:last], None if self.bias is None else self.bias[first:last]
-        if x.dtype == torch.float32 and w.dtype == torch.bfloat16 and self.rt.is_fp32:      # held by `exact_matrices`
-            return self.rt.k.gemm_three(x, w, b, whole=self.out_features)
-        return self.rt.k.linear(x, w, b, out_dtype or self.rt.dtype)
+        return self._product(x, self.weight[first:last], None if self.bias is None else self.bias[first:last], out_dtype)
+
+    def _product(self, x, w, b, out_dtype):
+        out_dtype = out_dtype or self.rt.dtype
+        if self.rt.is_fp32 and x.dtype == out_dtype == torch.float32 and w.dtype == torch.bfloat16:      # `exact_matrices` looked through it
+            return self.rt.k.gemm_three(x, w, b, whole=self.out_features, finite=True)
+        return self.rt.k.linear(x, w, b, out_dtype)
 
     def emit(self, b, x: int, out_dtype=None, out: int | None = None) -> int:
         """Native program: out = x . W^T (+ b) into a new register (or into `out`)."""

@@ -342,6 +342,27 @@ def test_gemm_three_infinite_and_huge_activations():
     assert ((got.double() - ref).abs()[fin] <= 2.0 ** -19 * (x.double().abs().nan_to_num(posinf=0) @ w.double().abs().t())[fin]).all()
 
 
+@pytest.mark.parametrize("M,N,K,bias", [(1, 70, 2048, False), (40, 300, 2048, True), (130, 16390, 1096, False), (300, 140, 2056, True)])
+def test_linear_with_weights_that_are_not_finite(M, N, K, bias):
+    """32-bit rows against a bfloat16 matrix that holds infinities and a NaN: what 64-bit arithmetic gives, an infinity of the right sign and no
+    NaN but where an infinity meets a zero, another infinity or a NaN; the other features are the same bits as without them."""
+    x, w = torch.randn(M, K), rnd(N, K, dtype=torch.bfloat16, seed=15)
+    x[:, 9] = x[:, 9].bfloat16().float()                                   # smaller terms that are zeros
+    x[0, 9] = 0.0
+    b = torch.randn(N) if bias else None
+    bad = w.clone()
+    bad[3, 5], bad[60, 9], bad[N - 1, K - 1] = math.inf, -math.inf, math.inf
+    bad[7, 100], bad[12, 0], bad[12, 1] = math.nan, math.inf, -math.inf
+    run = lambda m: k().linear(x.to(DEV), m.to(DEV), None if b is None else b.to(DEV), torch.float32).cpu()
+    got, clean, ref = run(bad), run(w), plain_ops.linear(x, bad.double(), b, torch.float64)
+    odd = torch.tensor([3, 7, 12, 60, N - 1])
+    assert torch.equal(torch.isnan(got), torch.isnan(ref)) and torch.equal(torch.isinf(got), torch.isinf(ref))
+    assert torch.equal(got[:, odd].nan_to_num().sign(), ref[:, odd].nan_to_num().float().sign())
+    rest = torch.ones(N, dtype=torch.bool)
+    rest[odd] = False
+    assert torch.equal(got[:, rest], clean[:, rest])
+
+
 @pytest.mark.parametrize("ta,tw,tc", [(torch.bfloat16, torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32, torch.float32),
                                       (torch.bfloat16, torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16, torch.bfloat16)])
 def test_gemm_simple_mixed_types(ta, tw, tc):
