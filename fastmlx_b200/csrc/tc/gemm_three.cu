@@ -406,8 +406,9 @@ FMX_EXPORT int fmx_gemm_three(const float* A, long long lda, const void* W, long
   }
   if (e != cudaSuccess) return fmx_fail("fmx_gemm_three: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
   const long long want = ((long long)M * (K / 8) + 255) / 256, most = 8LL * sms;
-  fmx_launch(split_kernel, dim3((unsigned)(want < most ? want : most)), dim3(256), 0, stream, A, lda, (bf16*)ws, M, K,
-             lda % 4 == 0 && ((uintptr_t)A & 15) == 0 ? 1 : 0);
+  e = fmx_launch(split_kernel, dim3((unsigned)(want < most ? want : most)), dim3(256), 0, stream, A, lda, (bf16*)ws, M, K,
+                 lda % 4 == 0 && ((uintptr_t)A & 15) == 0 ? 1 : 0);
+  if (e != cudaSuccess) return fmx_fail("fmx_gemm_three: launch of the split failed: %s", cudaGetErrorString(e));
   if (a.shares_apart)
     e = fmx_launch_cluster(gemm_three_kernel, dim3(a.tiles * a.splits), dim3(THREADS), smem, stream, dim3(a.splits), map_w, map_x, a);
   else

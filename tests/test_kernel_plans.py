@@ -1,5 +1,9 @@
 """Host-side arithmetic of the kernels' work division, checked without a GPU."""
+import os
 import pathlib
+import subprocess
+
+import pytest
 
 
 def test_short_prompts_go_to_the_library_product():
@@ -28,3 +32,17 @@ def test_shares_of_the_three_term_product():
         for K in (8, 64, 65, 512, 2048, 8192, 14336):
             assert 1 <= shares(N, K) <= min(8, -(-K // 64))
     assert shares(0, 64) == shares(64, 0) == 0
+
+
+def test_a_refused_launch_of_the_three_term_product_is_an_error(tmp_path):
+    """Either of its two kernels: a product over terms that were never written would leave wrong numbers and say nothing."""
+    from fastmlx_b200.csrc import build
+    try:
+        nvcc = build.find_nvcc()
+    except build.BuildError:
+        pytest.skip("nvcc is not installed")
+    here, exe = os.path.dirname(os.path.abspath(__file__)), str(tmp_path / "refused_launch")
+    subprocess.run([nvcc, *build.NVCC_FLAGS, "-I", os.path.join(build.HERE, "tc"), os.path.join(here, "refused_launch.cu"),
+                    os.path.join(build.HERE, "common", "error.cu"), "-o", exe], check=True)
+    lines = [tuple(map(int, l.split())) for l in subprocess.run([exe], check=True, capture_output=True, text=True).stdout.splitlines()]
+    assert lines == [(0, 2), (1, 1), (1, 2)]
