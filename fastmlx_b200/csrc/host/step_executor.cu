@@ -132,7 +132,8 @@ long long place_registers(const Executor& ex, int T, std::vector<long long>* off
   for (size_t r = 0; r < ex.regs.size(); ++r) {
     at = align_up(at, 256);
     if (offsets != nullptr) (*offsets)[r] = at;
-    at += (long long)T * ex.regs[r].cols * elem_size(ex.regs[r].dtype);
+    const int most = ex.regs[r].max_rows;
+    at += (long long)(most > 0 && most < T ? most : T) * ex.regs[r].cols * elem_size(ex.regs[r].dtype);
   }
   return align_up(at, 256);
 }

@@ -29,6 +29,7 @@ enum FmxOpKind {
 struct FmxReg {
   int cols;
   int dtype;               // FMX_F32 / FMX_BF16
+  int max_rows;            // 0: a row per token of the step, else at most so many
 };
 
 struct FmxOp {

@@ -364,26 +364,29 @@ FMX_EXPORT int fmx_gemm_three_not_finite(const float* A, long long lda, const vo
 // Into how many shares a product of N features over K is split, whatever its number of tokens.
 FMX_EXPORT int fmx_gemm_three_splits(int N, int K) { return N > 0 && K > 0 ? plan_splits(N, K) : 0; }
 
-// Bytes of workspace that a product of M tokens over K takes: the activations' three terms.
-FMX_EXPORT long long fmx_gemm_three_bytes(int M, int K) { return 6LL * M * K; }
+// Tokens whose terms the workspace holds at most, 256 MB of them (whole tiles, and one at least): a product of more goes in waves of so
+// many, whose results are the same bits.  Sizes with more than one wave (5,376 tokens over 8,192) fill the GPU many times over.
+FMX_EXPORT int fmx_gemm_three_rows(int K) {
+  const long long rows = K > 0 ? (256LL << 20) / (6LL * K) / MAX_TOKENS * MAX_TOKENS : 0;
+  return rows < MAX_TOKENS ? MAX_TOKENS : (int)rows;
+}
 
-// A 32-bit [M, K], W bfloat16 [N, K] with K-contiguous rows that start on 16 bytes, C 32-bit [M, N].  whole_n: features of the matrix
-// that W's rows are a part of, whose shares of K the product takes; N where W is all of it.  ws: fmx_gemm_three_bytes on 16
-// bytes.  status: the engine's status word (a wait that expires leaves FMX_WAIT_EXPIRED there).
-FMX_EXPORT int fmx_gemm_three(const float* A, long long lda, const void* W, long long ldw, const float* bias, float* C, long long ldc,
-                              int M, int N, int K, int whole_n, void* ws, int sms, int* status, cudaStream_t stream) {
-  if (M == 0 || N == 0) return 0;
-  if (M < 0 || N < 0 || K <= 0 || whole_n < N) return fmx_fail("fmx_gemm_three: bad sizes M=%d N=%d of %d K=%d", M, N, whole_n, K);
-  if (K % 8 || ldw % 8 || ((uintptr_t)W & 15)) return fmx_fail("fmx_gemm_three: W's rows must start on 16 bytes (K=%d ldw=%lld)", K, ldw);
-  if (ws == nullptr || ((uintptr_t)ws & 15)) return fmx_fail("fmx_gemm_three: the workspace is missing or does not lie on 16 bytes");
-  if (sms <= 0) sms = fmx_num_sms();
+// Bytes of workspace that a product of M tokens over K takes: the three terms of a wave's activations.
+FMX_EXPORT long long fmx_gemm_three_bytes(int M, int K) {
+  const int rows = fmx_gemm_three_rows(K);
+  return 6LL * (M < rows ? M : rows) * K;
+}
+
+namespace {
+int run_wave(const float* A, long long lda, const void* W, long long ldw, const float* bias, float* C, long long ldc, int M, int N, int K,
+             int whole_n, void* ws, int sms, int* status, cudaStream_t stream) {
   Three a = {};
   a.bias = bias; a.C = C; a.ldc = ldc; a.M = M; a.N = N; a.K = K; a.status = status;
   a.tiles_t = (M + MAX_TOKENS - 1) / MAX_TOKENS;
   a.tokens = ((M + a.tiles_t - 1) / a.tiles_t + 15) / 16 * 16;
   a.tiles_t = (M + a.tokens - 1) / a.tokens;
   const long long tiles = (long long)a.tiles_t * ((N + TF - 1) / TF);
-  if (tiles > 0x7fffffffLL / MAX_SPLITS || M > 0x7fffffff / 3) return fmx_fail("fmx_gemm_three: M=%d N=%d are too large", M, N);
+  if (tiles > 0x7fffffffLL / MAX_SPLITS) return fmx_fail("fmx_gemm_three: M=%d N=%d are too large", M, N);
   a.tiles = (int)tiles;
   a.splits = plan_splits(whole_n, K);
   // A CTA's whole walk over K, or a cluster's shares of it: blocks of K that the busiest SM takes, with APART more for each CTA of a
@@ -414,5 +417,25 @@ FMX_EXPORT int fmx_gemm_three(const float* A, long long lda, const void* W, long
   else
     e = fmx_launch(gemm_three_kernel, dim3(a.tiles < sms ? a.tiles : sms), dim3(THREADS), smem, stream, map_w, map_x, a);
   if (e != cudaSuccess) return fmx_fail("fmx_gemm_three: launch failed: %s", cudaGetErrorString(e));
+  return 0;
+}
+}  // namespace
+
+// A 32-bit [M, K], W bfloat16 [N, K] with K-contiguous rows that start on 16 bytes, C 32-bit [M, N].  whole_n: features of the matrix
+// that W's rows are a part of, whose shares of K the product takes; N where W is all of it.  ws: fmx_gemm_three_bytes on 16
+// bytes.  status: the engine's status word (a wait that expires leaves FMX_WAIT_EXPIRED there).
+FMX_EXPORT int fmx_gemm_three(const float* A, long long lda, const void* W, long long ldw, const float* bias, float* C, long long ldc,
+                              int M, int N, int K, int whole_n, void* ws, int sms, int* status, cudaStream_t stream) {
+  if (M == 0 || N == 0) return 0;
+  if (M < 0 || N < 0 || K <= 0 || whole_n < N) return fmx_fail("fmx_gemm_three: bad sizes M=%d N=%d of %d K=%d", M, N, whole_n, K);
+  if (K % 8 || ldw % 8 || ((uintptr_t)W & 15)) return fmx_fail("fmx_gemm_three: W's rows must start on 16 bytes (K=%d ldw=%lld)", K, ldw);
+  if (ws == nullptr || ((uintptr_t)ws & 15)) return fmx_fail("fmx_gemm_three: the workspace is missing or does not lie on 16 bytes");
+  if (sms <= 0) sms = fmx_num_sms();
+  const int rows = fmx_gemm_three_rows(K);
+  for (int m = 0; m < M; m += rows) {
+    const int rc = run_wave(A + m * lda, lda, W, ldw, bias, C + m * ldc, ldc, M - m < rows ? M - m : rows, N, K, whole_n, ws, sms, status, stream);
+    if (rc != 0) return rc;
+    if (M - m <= rows) break;
+  }
   return 0;
 }

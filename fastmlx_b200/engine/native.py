@@ -33,7 +33,7 @@ class NotNative(Exception):
 
 
 class FmxReg(Structure):
-    _fields_ = [("cols", c_int), ("dtype", c_int)]
+    _fields_ = [("cols", c_int), ("dtype", c_int), ("max_rows", c_int)]
 
 
 class FmxOp(Structure):
@@ -124,15 +124,15 @@ class ProgramBuilder:
     def __init__(self, rt, manager):
         self.rt, self.manager = rt, manager
         self.act = _dt(rt.dtype)
-        self.regs: list[tuple[int, int]] = []
+        self.regs: list[tuple[int, int, int]] = []
         self.ops: list[FmxOp] = []
         self.keep: list = []                       # tensors whose addresses the program holds
-        self._free: dict[tuple[int, int], list[int]] = {}
+        self._free: dict[tuple[int, int, int], list[int]] = {}
         self.wanted = False                        # operations from here on run over the wanted rows only
         self.greedy_head_ok = False                # the head may choose greedily inside its product
 
-    def reg(self, cols: int, dtype=None) -> int:
-        key = (int(cols), self.act if dtype is None else _dt(dtype) if not isinstance(dtype, int) else dtype)
+    def reg(self, cols: int, dtype=None, max_rows: int = 0) -> int:
+        key = (int(cols), self.act if dtype is None else _dt(dtype) if not isinstance(dtype, int) else dtype, int(max_rows))
         free = self._free.get(key)
         if free:
             return free.pop()
@@ -162,7 +162,7 @@ class ProgramBuilder:
         """A register for the terms of a 32-bit product's input, where its matrix is held in bfloat16; else -1.  Released right after."""
         if self.dtype_of(x) != F32 or w.dtype != torch.bfloat16:
             return -1
-        r = self.reg(3 * w.shape[1], BF16)
+        r = self.reg(3 * w.shape[1], BF16, _klib.load("tc").fmx_gemm_three_rows(w.shape[1]))
         self.release(r)
         return r
 
@@ -241,7 +241,7 @@ class NativeProgram:
         elif any(op.terms >= 0 for op in b.ops):       # matrices that the 32-bit path holds as they were stored
             table.gemm_three = _fn(_klib.load("tc"), "fmx_gemm_three")
         self._ops = (FmxOp * len(b.ops))(*b.ops)
-        self._regs = (FmxReg * len(b.regs))(*[FmxReg(c, d) for c, d in b.regs])
+        self._regs = (FmxReg * len(b.regs))(*[FmxReg(*r) for r in b.regs])
         self._blas_ws = torch.empty(self.CUBLAS_WORKSPACE, dtype=torch.uint8, device=rt.device)
         path = os.path.join(os.path.dirname(torch.__file__), "..", "nvidia", "cublas", "lib", "libcublas.so.12")
         self.handle = self.lib.fmx_exec_create(self._ops, len(b.ops), self._regs, len(b.regs), ctypes.byref(table),

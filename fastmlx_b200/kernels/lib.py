@@ -167,6 +167,7 @@ def load(group: str) -> ctypes.CDLL:
         lib.fmx_gemm_tcgen05_plan_width.argtypes = [_I, _I, _I]
         lib.fmx_gemm_tcgen05_plan_fills.argtypes = [_I, _I, _I]
         lib.fmx_gemm_three_splits.argtypes = [_I, _I]
+        lib.fmx_gemm_three_rows.argtypes = [_I]
         lib.fmx_gemm_three_bytes.argtypes = [_I, _I]
         lib.fmx_gemm_three_bytes.restype = c_longlong
     if group == "chunks":

@@ -327,6 +327,19 @@ def test_gemm_three_over_some_rows_of_a_matrix(N, K, cuts, M):
         assert torch.equal(k().gemm_three(x, w[a:b], whole=N), whole[:, a:b]), (a, b)
 
 
+@pytest.mark.parametrize("N,bias", [(130, True), (2048, False)])
+def test_gemm_three_in_waves(N, bias):
+    """More tokens than the workspace holds terms of: each the bits it has by itself, on both sides of a wave's end."""
+    from fastmlx_b200.kernels.lib import load
+    K = 14336
+    rows = load("tc").fmx_gemm_three_rows(K)
+    x, w = torch.randn(2 * rows + 77, K, device=DEV), rnd(N, K, dtype=torch.bfloat16, seed=16).to(DEV)
+    b = torch.randn(N, device=DEV) if bias else None
+    full = k().gemm_three(x, w, b)
+    for a, m in ((0, 130), (rows - 3, 7), (rows - 1, 1), (2 * rows - 20, 97)):
+        assert torch.equal(k().gemm_three(x[a:a + m], w, b), full[a:a + m]), a
+
+
 def test_gemm_three_infinite_and_huge_activations():
     """An infinity or a NaN stays in its row; values that would round to an infinity in bfloat16 do not."""
     x, w = torch.randn(40, 192), rnd(70, 192, dtype=torch.bfloat16, seed=12)

@@ -4,6 +4,7 @@ import pathlib
 import subprocess
 
 import pytest
+import torch
 
 
 def test_short_prompts_go_to_the_library_product():
@@ -32,6 +33,32 @@ def test_shares_of_the_three_term_product():
         for K in (8, 64, 65, 512, 2048, 8192, 14336):
             assert 1 <= shares(N, K) <= min(8, -(-K // 64))
     assert shares(0, 64) == shares(64, 0) == 0
+
+
+def test_workspace_of_the_three_term_product_is_bounded():
+    """At most 256 MB of terms: more tokens go in waves, as a call and in the native executor's arena."""
+    import ctypes
+    from fastmlx_b200.engine import native as nat
+    from fastmlx_b200.kernels import load
+    lib = load("tc")
+    for K in (8, 2048, 8192, 14336, 65536):
+        rows = lib.fmx_gemm_three_rows(K)
+        assert rows % 128 == 0 and rows >= 128
+        for M in (1, 333, 8192, 1 << 20):
+            assert lib.fmx_gemm_three_bytes(M, K) == 6 * min(M, rows) * K <= 256 << 20
+    rt = type("Runtime", (), dict(dtype=torch.float32))()
+    b = nat.ProgramBuilder(rt, None)
+    x, w = b.reg(14336), torch.zeros(64, 14336, dtype=torch.bfloat16)
+    b.op(nat.OP_LINEAR, in0=x, out0=b.reg(64), n=64, k=14336, terms=b.terms(x, w))
+    host, table = nat.host_library(), nat.FmxKernelTable()
+    for name, _ in table._fields_:
+        setattr(table, name, 1)
+    ops, regs = (nat.FmxOp * 1)(*b.ops), (nat.FmxReg * len(b.regs))(*[nat.FmxReg(*r) for r in b.regs])
+    ex = host.fmx_exec_create(ops, 1, regs, len(b.regs), ctypes.byref(table), 148, None, None, 0)
+    assert ex
+    for T in (16, 3000, 8192):
+        assert host.fmx_exec_arena_bytes(ex, T) <= T * (14336 + 64) * 4 + min(6 * T * 14336, 256 << 20) + 1024
+    host.fmx_exec_destroy(ex)
 
 
 def test_a_refused_launch_of_the_three_term_product_is_an_error(tmp_path):
