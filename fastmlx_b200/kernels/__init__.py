@@ -179,7 +179,8 @@ def _status_word(device):
 #   M <= 16                    whole-K weight-streaming kernel (`gemv`), except the vocabulary-sized head
 #   M >= 128, full rounds      tcgen05 kernel (`gemm_tcgen05`)
 #   everything else in bf16    the library (cuBLAS through torch.mm), as tamnd/fastmlx calls its library's matmul
-#   32-bit x, bfloat16 w       three-term tcgen05 kernel (`gemm_three`), whatever M: its sums do not depend on M
+#   32-bit x, bfloat16 w       three-term tcgen05 kernel (`gemm_three`), whatever M: its sums do not depend on M (which matrices the 32-bit
+#                              path leaves in bfloat16: `holds_exactly`, by their sizes)
 #   other types                fixed-order FMA kernel (`gemm_simple`)
 GEMV_MAX_ROWS = 16
 LIBRARY_MIN_FEATURES = 65536     # from this many output features on (the vocabulary) the library's product streams best
@@ -315,10 +316,21 @@ def gemm_tcgen05(x, w, status=None, epilogue: int = EPI_PLAIN, residual=None, bn
     return out
 
 
+def three_terms_pay(N: int, K: int) -> bool:
+    """Is the three-term product over an [N, K] matrix ahead of multiply-adds over the widened one for any number of tokens?  It begins with
+    a kernel of its own and a longer start, which short sums do not win back at few tokens.  Multiply-adds and three terms, us, 1 / 16 / 64 tokens:
+    64 x 256 4.1 / 4.2 / 7.8 and 5.5 / 5.9 / 7.0; 2,048 x 512 6.5 / 7.1 / 16.6 and 7.7 / 7.8 / 9.2; 4,096 x 1,024 10.6 / 14.7 / 31 and
+    11.1 / 11.0 / 13.2; but 8,192 x 1,024 12.3 / 20.9 / 48 and 11.5 / 11.8 / 13.8; 16,384 x 512 10.3 / 21 / 34 and 9.5 / 9.5 / 11; 16 x 1,088
+    10.0 / 12.0 / 27 and 7.1 / 7.6 / 8.7; 64 x 2,048 16.2 / 19.4 / 51 and 8.2 / 8.5 / 9.6."""
+    return K > 1024 or N * K >= 1 << 23
+
+
 def holds_exactly(ws) -> bool:
-    """May the 32-bit path keep these matrices as the bfloat16 values they were stored as (`gemm_three` multiplies them exactly) instead
-    of widening them?  Rows of 16-byte pieces; finite (`gemm_three`'s `finite`)."""
+    """May the 32-bit path keep these matrices, the rows of one product, as the bfloat16 values they were stored as (`gemm_three` multiplies
+    them exactly) instead of widening them?  Rows of 16-byte pieces; finite (`gemm_three`'s `finite`); sizes at which it pays."""
     if not all(w.dtype == torch.bfloat16 and w.dim() == 2 and w.numel() > 0 and w.shape[1] % 8 == 0 for w in ws):
+        return False
+    if not three_terms_pay(sum(w.shape[0] for w in ws), ws[0].shape[1]):
         return False
     ends = torch.stack([e for w in ws for e in torch.aminmax(w)])          # a NaN shows in both
     return bool(torch.isfinite(ends).all())

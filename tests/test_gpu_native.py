@@ -45,6 +45,27 @@ def test_native_and_python_paths_agree_to_the_bit_in_32_bit(dirs, name, cut):
             assert np.array_equal(x, y)
 
 
+def test_matrices_kept_as_stored_in_the_native_program(tmp_path):
+    """A model wide enough for the three-term products (with biases, beside an output projection that is not): the native program and the Python
+    path agree to the bit in 32-bit, and with the plain model to rounding."""
+    cfg = {**tiny.TINY_C, "hidden_size": 1088, "num_hidden_layers": 2, "intermediate_size": 1160}
+    d = tiny.make_model_dir(tmp_path, cfg, seed=17)
+    prompts = {f"r{i}": tiny.rand_tokens(n, cfg["vocab_size"], 60 + i) for i, n in enumerate([7, 33, 130])}
+    steps = traces.mixed(prompts)
+    a, rp = _replay(d, "float32", steps, True)
+    b, _ = _replay(d, "float32", steps, False)
+    kept = [op.terms >= 0 for op in rp.step_fn.native.builder.ops if op.kind in (2, 3)]          # linear, gate/up
+    assert any(kept) and not all(kept)
+    for x, y in zip(a, b):
+        assert (x is None) == (y is None) and (x is None or np.array_equal(x, y))
+    rows, W = traces.collect(steps, a), tiny.load_plain_weights(d)
+    for rid, toks in prompts.items():
+        ref = plain_llama.forward(cfg, W, toks, None)
+        scale = ref.abs().max().item()
+        for pos in range(len(toks)):
+            assert np.abs(rows[rid][pos] - ref[pos].numpy()).max() / scale < 1e-5, (rid, pos)
+
+
 @pytest.mark.parametrize("name", ["A", "B", "C"])
 def test_native_path_in_bfloat16_against_the_plain_model_and_the_python_path(dirs, name):
     cfg = tiny.CONFIGS[name]

@@ -35,6 +35,21 @@ def test_shares_of_the_three_term_product():
     assert shares(0, 64) == shares(64, 0) == 0
 
 
+def test_small_matrices_stay_with_multiply_adds():
+    """Where a product of a few tokens is shorter than the three-term product's two kernels the 32-bit path widens the matrix as it did, by the
+    whole product's sizes alone; matrices of real widths are kept as they were stored."""
+    from fastmlx_b200 import kernels as k
+    pays = lambda N, K: k.holds_exactly([torch.ones(N, K, dtype=torch.bfloat16)])
+    assert not any(pays(N, K) for N, K in ((16, 64), (320, 80), (2048, 512), (64, 1024), (4096, 1024), (8192, 256)))
+    assert all(pays(N, K) for N, K in ((16, 1032), (64, 2048), (2048, 2048), (8192, 1024), (16384, 512)))
+    assert not k.three_terms_pay(64, 0) and not k.three_terms_pay(0, 512)
+    half = torch.ones(4096, 1024, dtype=torch.bfloat16)
+    assert k.holds_exactly([half, half]) and not k.holds_exactly([half])          # rows of one product count together
+    big = torch.ones(64, 2048, dtype=torch.bfloat16)
+    big[5, 7] = float("inf")
+    assert not k.holds_exactly([big]) and not k.holds_exactly([big.float()]) and not k.holds_exactly([torch.ones(64, 2047).bfloat16()])
+
+
 def test_workspace_of_the_three_term_product_is_bounded():
     """At most 256 MB of terms: more tokens go in waves, as a call and in the native executor's arena."""
     import ctypes
