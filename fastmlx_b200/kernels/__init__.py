@@ -9,6 +9,7 @@ matrix mode.  Nothing here runs on the CPU.
 from __future__ import annotations
 
 import functools
+import math
 
 import torch
 
@@ -539,10 +540,35 @@ def wide_tc_ok(kv, nh: int, nkv: int, hd: int, vd: int, scale: float, keep_first
             and scale > 0.0 and not keep_first and not chunk and sinks is None)
 
 
-# Keys from which on the tensor-memory kernel with two-term products is ahead of the `mma.sync` one, by the longest context after the step:
-# its start costs more than a short row's tiles (32 heads on 8, us, `mma.sync` and here: head size 64, 64 keys 7.2 and 8.7, 256 13.8 and 11.8;
-# head size 128, 256 keys 16.9 and 19.5, 512 31 and 26).
+# Keys from which on the tensor-memory kernel with two-term products is ahead of the `mma.sync` one where each row sees all of its context, by
+# the longest context after the step: its start costs more than a short row's tiles (32 heads on 8, us, `mma.sync` and here: head size 64,
+# 64 keys 7.2 and 8.7, 256 13.8 and 11.8; head size 128, 256 keys 16.9 and 19.5, 512 31 and 26).
 WIDE_TC_KEYS = {64: 192, 128: 384}
+# us of a launch of either kernel, least squares over 956 launches (6 % off on average): a + (b + c if scores are capped) x tiles of 64 keys that a
+# block walks + (d + e with a window) x the share of its query rows that are in use + f with a window, times the larger of 1 and g + h x blocks
+# per SM.
+WIDE_COST = {64: ((4.15, 1.56, 0.38, 0.62, 0.05, -0.12, 0.49, 0.43), (5.88, 1.14, -0.04, 0.91, 1.35, -0.44, 0.40, 0.58)),
+             128: ((4.68, 2.39, 0.37, 1.58, 0.14, 0.0, 0.35, 0.56), (6.92, 1.54, 0.07, 5.61, 2.20, -0.53, -0.16, 1.19))}
+
+
+def wide_tc_pays(hd: int, rep: int, nkv: int, rows: int, tokens: int, max_q_len: int, longest: int, window: int, capped: bool, sms: int = 148) -> bool:
+    """Does this step go to the tensor-memory kernel?  Its tiles are twice (head size 64) or four times as many tokens as the `mma.sync` kernel's,
+    so behind a window, or with portions that leave most of a tile empty, a block walks more keys or works for rows that are not there:
+    16 heads of 64, 128 tokens behind a window of 64: 8.9 us by `mma.sync`, 12.0 here; of 128 values, 32 rows of 16 tokens behind a window of
+    128: 28.8 and 48.4.  Not where the estimates (WIDE_COST) have `mma.sync` ahead by 5 %."""
+    if longest < WIDE_TC_KEYS[hd]:
+        return False
+
+    def cost(c, tile, queries):            # tile: tokens of a block's queries
+        seen = -(-longest // 64) if not window else (min(longest, window + min(max_q_len, tile) - 1) - 1) / 64 + 1
+        blocks = rows * nkv * max(1, math.ceil(tokens / rows / tile))
+        in_use, a, b, per_cap, share, share_window, with_window, e, f = min(max_q_len * rep, queries) / queries, *c
+        t = a + (b + per_cap * bool(capped)) * seen + share * in_use
+        return (t + with_window + share_window * in_use if window else t) * max(1.0, e + f * blocks / sms)
+
+    old, new = WIDE_COST[hd]
+    queries = 128 if hd == 64 else 256
+    return cost(new, queries // rep, queries) < 1.05 * cost(old, -(-64 // rep), 64)
 
 
 def _wide_launch(q, kv, ctx, group, nh, nkv, hd, scale, softcap, window, out, first_token: int = 0, splits: int = 1,
@@ -551,7 +577,8 @@ def _wide_launch(q, kv, ctx, group, nh, nkv, hd, scale, softcap, window, out, fi
     bt = group.block_tables
     if tc is None:
         tc = (splits == 1 and ctx.max_q_len > 1 and wide_tc_ok(kv, nh, nkv, hd, vd, scale, keep_first, chunk, sinks)
-              and getattr(ctx, "max_ctx_after", 0) >= WIDE_TC_KEYS[hd])
+              and wide_tc_pays(hd, nh // nkv, nkv, ctx.R, getattr(ctx, "T", 0) or ctx.R * ctx.max_q_len, ctx.max_q_len,
+                               getattr(ctx, "max_ctx_after", 0), int(window), bool(softcap), num_sms(q.device)))
     if tc:
         call(f"attn_hd{hd}", "fmx_attn_wide_tc", q.data_ptr(), q.stride(0), kv.data_ptr(), bt.data_ptr(), bt.stride(0), ctx.row_start.data_ptr(),
              ctx.row_ctx.data_ptr(), ctx.positions.data_ptr(), out.data_ptr(), out.stride(0), ctx.R, int(ctx.max_q_len), nh, nkv, kv.shape[3],
@@ -1643,7 +1670,8 @@ def _rows_of(ctx, group, a: int, b: int, max_q_len: int, max_ctx_after: int):
     row start at row a, token indices and positions stay those of the whole step."""
     from types import SimpleNamespace
     sub = SimpleNamespace(positions=ctx.positions, status=ctx.status, row_start=ctx.row_start[a:], row_ctx=ctx.row_ctx[a:],
-                          R=b - a, max_q_len=max_q_len, max_ctx_after=max_ctx_after, all_decode=max_q_len == 1, n_splits=0)
+                          R=b - a, T=b - a if max_q_len == 1 else max(0, getattr(ctx, "T", 0) - a), max_q_len=max_q_len,
+                          max_ctx_after=max_ctx_after, all_decode=max_q_len == 1, n_splits=0)
     return sub, SimpleNamespace(block_tables=group.block_tables[a:b])
 
 

@@ -88,3 +88,20 @@ def test_a_refused_launch_of_the_three_term_product_is_an_error(tmp_path):
                     os.path.join(build.HERE, "common", "error.cu"), "-o", exe], check=True)
     lines = [tuple(map(int, l.split())) for l in subprocess.run([exe], check=True, capture_output=True, text=True).stdout.splitlines()]
     assert lines == [(0, 2), (1, 1), (1, 2)]
+
+
+@pytest.mark.parametrize("hd,nh,nkv,rows,q,ctx,window,capped,mma,tc", [
+    (64, 32, 8, 1, 128, 2000, 64, True, 8.9, 10.9), (64, 16, 16, 1, 128, 2000, 64, True, 8.9, 12.0),
+    (64, 16, 16, 1, 512, 2000, 128, True, 11.3, 13.2), (64, 32, 8, 1, 64, 2000, 256, True, 15.0, 14.3),
+    (64, 32, 8, 8, 128, 2000, 64, True, 18.9, 13.7), (64, 32, 8, 1, 2048, 2000, 64, True, 29.1, 25.0),
+    (64, 16, 1, 1, 512, 0, 0, True, 20.5, 15.3), (64, 32, 8, 1, 64, 0, 0, True, 6.6, 7.9), (64, 32, 8, 1, 64, 512, 0, True, 22.2, 15.8),
+    (128, 16, 16, 32, 16, 2000, 128, True, 28.8, 48.4), (128, 16, 16, 1, 512, 2000, 256, True, 20.9, 28.9),
+    (128, 32, 8, 1, 64, 2000, 64, True, 12.5, 17.1), (128, 16, 1, 1, 64, 2000, 128, True, 15.3, 18.8),
+    (128, 32, 8, 1, 2048, 2000, 128, True, 68.3, 39.5), (128, 32, 8, 1, 128, 2000, 1024, True, 54.2, 44.3),
+    (128, 12, 4, 1, 512, 2000, 128, True, 15.7, 23.2), (128, 32, 8, 1, 512, 512, 0, True, 62.5, 40.2),
+    (64, 32, 8, 1, 64, 2000, 128, False, 9.8, 12.7)])
+def test_two_term_attention_goes_where_it_is_faster(hd, nh, nkv, rows, q, ctx, window, capped, mma, tc):
+    """The choice between the two kernels of the two-term attention, at sizes that were timed on both (us): by the keys that a block walks and the
+    rows that fill its tile, not by the longest context alone."""
+    from fastmlx_b200 import kernels as k
+    assert k.wide_tc_pays(hd, nh // nkv, nkv, rows, rows * q, q, ctx + q, window, capped) == (tc < mma)
