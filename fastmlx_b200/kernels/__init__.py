@@ -342,8 +342,10 @@ def gemm_three(x, w, bias=None, status=None, whole: int = 0, finite: bool = Fals
     does not depend on the other rows.  `whole`: features of the matrix that w is some rows of (0: w is all of it); the results are then the
     bits that the product over the whole matrix gives these features.  `finite`: the caller knows that w holds no infinity, which would meet
     the zeros among an activation's smaller terms; else results that are not finite are worked out again by themselves."""
+    _need_cuda(x, w, bias)
     M, K = x.shape
     N = w.shape[0]
+    assert w.shape[1] == K and x.stride(1) == 1 and w.stride(1) == 1 and x.dtype == torch.float32 and w.dtype == torch.bfloat16
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     need = load("tc").fmx_gemm_three_bytes(M, K)
     ws = torch.empty(need, dtype=torch.uint8, device=x.device)
@@ -551,7 +553,8 @@ WIDE_COST = {64: ((4.15, 1.56, 0.38, 0.62, 0.05, -0.12, 0.49, 0.43), (5.88, 1.14
              128: ((4.68, 2.39, 0.37, 1.58, 0.14, 0.0, 0.35, 0.56), (6.92, 1.54, 0.07, 5.61, 2.20, -0.53, -0.16, 1.19))}
 
 
-def wide_tc_pays(hd: int, rep: int, nkv: int, rows: int, tokens: int, max_q_len: int, longest: int, window: int, capped: bool, sms: int = 148) -> bool:
+@functools.lru_cache(maxsize=1024)       # a step asks once for each of its layers
+def wide_tc_pays(hd: int, rep: int, nkv: int, rows: int, tokens: int, max_q_len: int, longest: int, window: int, capped: bool) -> bool:
     """Does this step go to the tensor-memory kernel?  Its tiles are twice (head size 64) or four times as many tokens as the `mma.sync` kernel's,
     so behind a window, or with portions that leave most of a tile empty, a block walks more keys or works for rows that are not there:
     16 heads of 64, 128 tokens behind a window of 64: 8.9 us by `mma.sync`, 12.0 here; of 128 values, 32 rows of 16 tokens behind a window of
@@ -567,7 +570,7 @@ def wide_tc_pays(hd: int, rep: int, nkv: int, rows: int, tokens: int, max_q_len:
         return (t + with_window + share_window * in_use if window else t) * max(1.0, e + f * blocks / sms)
 
     old, new = WIDE_COST[hd]
-    queries = 128 if hd == 64 else 256
+    sms, queries = num_sms(), 128 if hd == 64 else 256
     return cost(new, queries // rep, queries) < 1.05 * cost(old, -(-64 // rep), 64)
 
 
@@ -576,9 +579,10 @@ def _wide_launch(q, kv, ctx, group, nh, nkv, hd, scale, softcap, window, out, fi
     vd = vd or hd
     bt = group.block_tables
     if tc is None:
-        tc = (splits == 1 and ctx.max_q_len > 1 and wide_tc_ok(kv, nh, nkv, hd, vd, scale, keep_first, chunk, sinks)
-              and wide_tc_pays(hd, nh // nkv, nkv, ctx.R, getattr(ctx, "T", 0) or ctx.R * ctx.max_q_len, ctx.max_q_len,
-                               getattr(ctx, "max_ctx_after", 0), int(window), bool(softcap), num_sms(q.device)))
+        longest = getattr(ctx, "max_ctx_after", 0)
+        tc = (splits == 1 and ctx.max_q_len > 1 and longest >= WIDE_TC_KEYS.get(hd, longest + 1)
+              and wide_tc_ok(kv, nh, nkv, hd, vd, scale, keep_first, chunk, sinks) and wide_tc_pays(
+                  hd, nh // nkv, nkv, ctx.R, getattr(ctx, "T", 0) or ctx.R * ctx.max_q_len, ctx.max_q_len, longest, window, bool(softcap)))
     if tc:
         call(f"attn_hd{hd}", "fmx_attn_wide_tc", q.data_ptr(), q.stride(0), kv.data_ptr(), bt.data_ptr(), bt.stride(0), ctx.row_start.data_ptr(),
              ctx.row_ctx.data_ptr(), ctx.positions.data_ptr(), out.data_ptr(), out.stride(0), ctx.R, int(ctx.max_q_len), nh, nkv, kv.shape[3],

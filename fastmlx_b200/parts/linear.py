@@ -40,6 +40,7 @@ class Linear(Part):
             raise ValueError("interleaving takes two matrices of equal height, a multiple of the block")
         self.weight = None
         self.bias = None
+        self.kept = False
 
     def own_weight_specs(self):
         specs = [WeightSpec(n + self.wsfx, (o, self.in_features), "matrix") for n, o in self.names]
@@ -61,6 +62,7 @@ class Linear(Part):
         if self.weight.data_ptr() % 16:                # a view into a larger buffer: the products want rows on 16 bytes
             self.weight = self.weight.clone()
         self.out_features = self.weight.shape[0]
+        self.kept = rt.is_fp32 and self.weight.dtype == torch.bfloat16        # as stored, looked through by `exact_matrices`: 32-bit in and out
         if bs is not None:
             self.bias = torch.cat(bs).contiguous()
 
@@ -68,17 +70,16 @@ class Linear(Part):
         return self.weight.numel() * self.weight.element_size()
 
     def forward(self, x, out_dtype=None):
-        return self._product(x, self.weight, self.bias, out_dtype)
+        if self.kept:
+            return self.rt.k.gemm_three(x, self.weight, self.bias, finite=True)
+        return self.rt.k.linear(x, self.weight, self.bias, out_dtype or self.rt.dtype)
 
     def forward_rows(self, x, first: int, last: int, out_dtype=None):
         """Features [first, last) of `forward` alone: on the 32-bit path the same bits, whose sums over K follow the whole matrix."""
-        return self._product(x, self.weight[first:last], None if self.bias is None else self.bias[first:last], out_dtype)
-
-    def _product(self, x, w, b, out_dtype):
-        out_dtype = out_dtype or self.rt.dtype
-        if self.rt.is_fp32 and x.dtype == out_dtype == torch.float32 and w.dtype == torch.bfloat16:      # `exact_matrices` looked through it
+        w, b = self.weight[first:last], None if self.bias is None else self.bias[first:last]
+        if self.kept:
             return self.rt.k.gemm_three(x, w, b, whole=self.out_features, finite=True)
-        return self.rt.k.linear(x, w, b, out_dtype)
+        return self.rt.k.linear(x, w, b, out_dtype or self.rt.dtype)
 
     def emit(self, b, x: int, out_dtype=None, out: int | None = None) -> int:
         """Native program: out = x . W^T (+ b) into a new register (or into `out`)."""
