@@ -94,9 +94,10 @@ __device__ __forceinline__ f32x2 tanh_short(f32x2 y) {
   return fma2(mul2(y, q), p, y);
 }
 __device__ __forceinline__ float tanh_any(float y) { return fabsf(y) <= TANH_SMALL ? tanh_short(y) : tanhf(y); }
-// Caps up to this: a score lies within cap of the largest possible one, exp(-2 cap) is far inside the range of 32-bit numbers and of bfloat16,
-// and the weights need no maximum: their scale is that of the cap itself.
-constexpr float CAP_AS_SCALE = 38.f;
+// Caps up to this: two scores differ by 2 cap at most, exp(2 cap) is far inside the range of 32-bit numbers and of bfloat16, and the weights need no
+// maximum: their scale is that of a score of zero, or 2^-SCALE_ROOM of the cap's own where that is more, so that sums over many keys stay in
+// range.  (At the cap's own scale, far above most scores, an exponent's argument was rounded four times as coarsely.)
+constexpr float CAP_AS_SCALE = 38.f, SCALE_ROOM = 32.f;
 
 __global__ void __launch_bounds__(THREADS, HD == 64 ? 2 : 1)
 attn_wide_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ Wide a) {
@@ -282,7 +283,7 @@ attn_wide_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
     const int sure_lo = a.window > 0 ? ctx + my_tok0 + my_tok - a.window : 0, sure_hi = ctx + my_tok0;
     const bool whole = my_tok == per_tile;
     const bool fixed = capped && a.softcap <= CAP_AS_SCALE;
-    float m = fixed ? cap_l2 : -INFINITY;      // the scale in use (of the scores in base 2)
+    float m = fixed ? fmaxf(cap_l2 - SCALE_ROOM, 0.f) : -INFINITY;      // the scale in use (of the scores in base 2)
     float l = 0.f;                             // the row's sum at that scale
     bool ok = true;
     for (int j = 0; j < my_tiles; ++j) {
