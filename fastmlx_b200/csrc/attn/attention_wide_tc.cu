@@ -446,8 +446,6 @@ attn_wide_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const __grid_con
 }
 }  // namespace
 
-FMX_EXPORT int fmx_attn_wide_tc_available() { return 1; }
-
 // As fmx_attn_prefill_wide_masked without kept tokens, runs of positions, shares and terms without a value, over pages of keys and values,
 // for up to 16 query heads per kv head, a page size of at least 8 that divides the 64 keys of a tile
 // and a positive scale.
@@ -490,7 +488,6 @@ FMX_EXPORT int fmx_attn_wide_tc(const float* q, long long q_stride, const void* 
 }
 #else
 #include "common.cuh"
-FMX_EXPORT int fmx_attn_wide_tc_available() { return 0; }
 FMX_EXPORT int fmx_attn_wide_tc(const float*, long long, const void*, const int*, int, const int*, const int*, const int*, void*, long long, int, int, int,
                                 int, int, long long, float, float, int, int*, cudaStream_t) {
   return fmx_fail("fmx_attn_wide_tc: this head size has no tensor-memory attention kernel");

@@ -13,9 +13,9 @@
 // state runs on the tensor cores with three bfloat16 terms an operand (split_mma.cuh), so that its errors are those of the walk
 // token by token in 32-bit multiply-adds (the kernels of delta_rule.cu and ssm.cu; 2,048 tokens of the delta rule against 64-bit, of
 // the result's norm: decays of 0.9 to 1 1.3e-7 either way, of 0.8 to 1 1.2e-7 here and 1.1e-7 there; plain write 1.1e-7 and 1.3e-7).
-// That walk is one chain of dependent steps of some 250 ns a token; a run of 32 tokens here takes 1.4 us at 64 rows of state, 3.3 us at 128.  One request of 2,048
-// tokens, 32 heads on 8 key heads, both kernels: delta rule 64 x 64 525 -> 120 us, 128 x 128 (two requests) 1,052 -> 232 us;
-// plain write 349 -> 112 (32 heads of keys of their own) and 665 -> 176 us (64 heads of 64 values over 128 rows); 1,777 tokens of five requests, 64 heads of 64 values over 128 rows 579 -> 172 us.
+// That walk is one chain of dependent steps of some 250 ns a token; a run of 32 tokens here takes 1.4 us at 64 rows of state, 3.3 us at 128.  2,048
+// tokens, 32 heads on 8 key heads, both kernels, walk and runs in us: one request of 64 x 64 delta rule 522 and 116, plain write 346 and
+// 85; two of 128 x 128 937 and 227, 646 and 174; 64 heads of 64 values over 128 rows, one request 828 and 178, 1,777 tokens of five 560 and 171.
 //
 //   chunk_prepare  per (run, key group): k and q as three terms; k . k^T and q . k^T in 32-bit, and per head of the group
 //                  the decayed q . k^T and T, as three terms.  All runs at once.
@@ -387,8 +387,10 @@ template <int D, int MT> struct PlainSmem {
 };
 
 // The same without the delta rule, whose u is at hand before the run: nothing on the state's own chain crosses warps, so each warp keeps its
-// quarter of the state's rows to itself (RunWarp).  Four warps copy, two stages of operands or three.  Bound by `mma.sync`, of which a
-// scheduler takes one in some 15 clocks here (105 a warp and run of 128 rows).  With the state shared as fragments and one copying
+// quarter of the state's rows to itself (RunWarp).  Four warps copy (two for 64 rows), two stages of operands or three.  Bound by no unit: the tensor pipe is
+// busy for 35 % of the time (1,777 tokens of five requests, 64 heads of 64 values over 128 rows; 105 products a warp and run, one every 8.2
+// clocks of a scheduler where none waits for another, 21 where one does), and warps wait in turns for results of fixed latency, at the block's
+// barriers, for that pipe and for operands.  With the state shared as fragments and one copying
 // warp, which everything waited for: 1,777 tokens of five requests, 64 heads of 64 values over 128 rows 153 us, 138 here; 1,531 tokens of a
 // retention with 32 heads of 64 x 64 77 and 51.  For the delta rule the meeting of the quarters stands on the chain: 92 us that way, 95 this.
 template <int D, int MT>
@@ -397,7 +399,6 @@ chunk_plain_kernel(const bf16* qk, const bf16* pt, const float* x, long long C, 
                   const int* row_slot, float* state, long long slot_stride, float* out, int min_tokens, int H, int G, int P, int max_slots,
                   int lo, int hi, int stages) {
   using Z = PlainSmem<D, MT>;
-  constexpr int KT = D / 16, NS = D / 32;        // k-tiles of S; 8-row tiles of S^T per warp
   extern __shared__ __align__(16) unsigned char csm[];
   const int r = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * 16 * MT;
   const int tid = threadIdx.x, lane = tid & 31, mt = tid >> 7, w = tid >> 5 & 3;

@@ -62,7 +62,7 @@ struct Sums {
 // The six products of terms of `tiles` tiles of 16 of the contraction, for N right operands side by side: c[n] = a . b[n], both in three
 // terms (tile k's registers of b: b[n][term][2 k], b[n][term][2 k + 1]).  The tensor cores cut their sums off instead of rounding them,
 // and of the leading terms' products that would be seen: those of each tile are a sum of their own, added up rounded; the small terms'
-// products are CHAINS sums.  A product that waits for the one before it takes 30 clocks, one that does not 15: hence the sums side
+// products are CHAINS sums.  A product that waits for the one before it takes 21 clocks, one that does not 8.2: hence the sums side
 // by side, and the steps over all N at a time.
 template <int KT, int CHAINS, int N, int NB>
 __device__ __forceinline__ void products(float (&c)[N][4], const unsigned (&a)[KT][3][4], const unsigned (&b)[N][3][NB], int tiles = KT) {
