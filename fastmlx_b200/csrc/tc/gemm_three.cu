@@ -19,8 +19,8 @@
 //
 // Bound by the products and the clock that they leave under the power limit (2,048 tokens: 1.24 PFLOP/s of bfloat16, three products to a
 // 32-bit one), below some 64 tokens by twelve products of at least 44 clocks a block.  Against 32-bit multiply-adds over the widened
-// matrix (gemm_simple.cu), the split with it, us: 16,384 x 2,048, 1 token 31 -> 17, 333 597 -> 64, 2,048 2,619 -> 335; 2,048 x 8,192 58 -> 14,
-// 479 -> 59, 1,535 -> 203.  Error against 64-bit, of the result's norm: 1.2e-7 to 1.6e-7, multiply-adds 0.8e-6 to 2.1e-6.
+// matrix (gemm_simple.cu), the split with it, weights from memory, us: 16,384 x 2,048, 1 token 29 -> 19, 333 592 -> 65, 1,024 1,314 -> 168;
+// 2,048 x 8,192 55 -> 14, 474 -> 60, 841 -> 101.  Error against 64-bit, of the result's norm: 1.2e-7 to 1.6e-7, multiply-adds 0.8e-6 to 2.1e-6.
 #include "common.cuh"
 #include "tcgen05.cuh"
 #include "three_terms.cuh"
